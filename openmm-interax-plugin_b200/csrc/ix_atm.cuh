@@ -5,16 +5,14 @@
 //
 //   kSiteCentroids       site positions (unweighted centroids, double) and the site rebuild check
 //   kSiteNeighbors       (rebuild only) per site A the sites B > A of other molecules within cutoff + skin
-//   kTriplesFast         one warp per site A with at most kAtmFast listed neighbors: the neighbors within the cutoff
-//                        are staged in shared memory with their double-precision minimum-image displacements from A
-//                        (rounded to float); the pairs (B, C) of them are enumerated by a flat triangular index so
-//                        that all lanes are busy, in rounds of kAtmRound pairs; each triple is counted once (A
-//                        lowest) and evaluated in float; the forces on B and C of each pair are stored and gathered
-//                        per staged neighbor in a fixed order (no atomics)
-//   kTriplesWide         the same for the rare sites with longer lists (chunked beyond kAtmMaxStaged within the
-//                        cutoff, so any length), with the B and C forces accumulated by shared-memory atomics; a
-//                        site whose list overflowed its capacity scans every later site instead, so an overflow
-//                        never drops a triple
+//   kTriplesFast         one warp per site A with a short list: the neighbors within the cutoff are staged in shared
+//                        memory with their double-precision minimum-image displacements from A (rounded to float);
+//                        four lanes take one neighbor C and share the others B among them, so that each triple is
+//                        seen once from B and once from C and each visit adds only the force on its own C, in
+//                        registers (no stores per triple, no gather, no atomics)
+//   kTriplesWide         the same for sites with longer lists, 8 warps per site (chunked beyond kAtmMaxStaged within
+//                        the cutoff, so any length); a site whose list overflowed its capacity scans the sites
+//                        instead, so an overflow never drops a triple
 //   kSpreadSiteForces    the site forces, shared equally among each site's particles, into the particle forces
 #pragma once
 
@@ -38,7 +36,15 @@ struct AtmConfig {
     float invCentroidRadius;     // 0 = no centroid damping
     float maxMove2;
     int zeroSlots, zeroOffset;   // energy slots the fast kernel clears (those of a wide kernel that may not run)
+    int imageBC;                 // the displacement of C from B can need a minimum image of its own
 };
+
+// Whether two neighbors of a site can be nearest to each other through another image than the site's: not in a
+// rectangular box whose edges exceed three cutoffs, where such an image is farther than the cutoff.
+inline int tripleNeedsImages(const AtmConfig& C, double cutoff) {
+    return C.periodic && (C.box.triclinic || !(C.box.a[0] > 3.001 * cutoff && C.box.b[1] > 3.001 * cutoff &&
+                                               C.box.c[2] > 3.001 * cutoff));
+}
 
 // Cell grid of the site-list search in a rectangular periodic box whose edges hold at least three cells as wide as
 // the list cutoff: every site within the list cutoff of a site lies in its cell or the 26 around it.
@@ -50,7 +56,19 @@ struct SiteCells {
     int* siteCell;               // numSites
     float4* wrapped;             // numSites: each site's position wrapped into the box (float), w its molecule (int
                                  // bits), written by the cell sort for the list search
+    unsigned* order;             // numSites: the x coordinate as a 32-bit fraction of the box, at the last build
 };
+
+// The owner of a triple is the site that comes first; site `b` comes after site `a` (both within the list cutoff of
+// each other).  By index, the lists of the sites next to the periodic boundary hold all their neighbors where the
+// others hold half (in the 96,000-atom box with a 0.8 nm cutoff those long lists took the wide kernel 179 of the 421 us
+// of both).  Where the cell grid serves (edges of at least three list cutoffs) the order is that of the x displacement,
+// which gives every site half of its neighbors: the difference of the 32-bit box fractions wraps as the minimum image
+// does, and as no two of three mutual neighbors are a third of the box apart it orders them without a cycle.
+__device__ __forceinline__ bool siteAfter(const SiteCells& G, int byIndex, int a, int b) {
+    const int d = byIndex ? 0 : (int)(G.order[b] - G.order[a]);
+    return d > 0 || (d == 0 && b > a);
+}
 constexpr int kSiteCellMax = 8192;   // cells the one-block sort holds in shared memory
 // sites up to this count are scattered and ordered in dynamic shared memory by the one-block sort (160 KB)
 constexpr int kSiteSortSharedMax = 40000;
@@ -64,7 +82,8 @@ struct AtmBuffers {
     double* siteRef;             // numSites x 3, at the last list build
     float4* chunkBox;            // 2 per chunk of 32 consecutive sites: box center (w = 1: usable) and half extents,
                                  // of the positions wrapped into a rectangular box; null: the list search scans all
-    int* flag;                   // [0] rebuild, [1] neighbor overflow, [2] a list longer than kAtmFast
+    int* flag;                   // [0] rebuild, [1] neighbor overflow, [2] a list longer than the fast kernel takes,
+                                 // [3] the lists are ordered by index (set by their build, see siteAfter)
     int* nbrCount;               // numSites
     int* nbr;                    // numSites x cap
     int cap;
@@ -72,27 +91,19 @@ struct AtmBuffers {
     long long* particleForce;    // 3 x numParticles, SoA fixed point (original order)
     int numParticles;
     double* energyPartials;      // one per warp of the fast triple kernel's grid, then one per warp of the wide one
-    unsigned long long* tripleCount;
+    unsigned long long* tripleVisits;   // each interacting triple counts two (it is visited from two of its sites)
     SiteCells cells;
 };
 
-constexpr int kAtmFast = IX_TUNE_ATM_FAST;     // neighbor lists up to this length take the fast triple kernel
-constexpr int kAtmRound = IX_TUNE_ATM_ROUND;   // (B, C) pairs evaluated before their forces are gathered
-constexpr int kAtmAccum = IX_TUNE_ATM_ACCUM;   // 1: B and C forces as fixed-point shared-memory sums (no rounds)
+// Lists up to kAtmFast take the fast triple kernel, one warp per site: a longer one would hold its warp after the
+// others have finished (a cluster's first site has all the others listed).  The cell grid's lists are all of about
+// the same length, so there the fast kernel takes what its storage holds.
+constexpr int kAtmFast = IX_TUNE_ATM_FAST;
+constexpr int kAtmFastStaged = 2 * kAtmFast;
 constexpr int kAtmFastWarps = 4;
 
-// The flat triangular index p = c (c - 1) / 2 + b of the pairs b < c < kAtmFast, decoded: b | c << 8.
-struct TrianglePairs {
-    unsigned short bc[kAtmFast * (kAtmFast - 1) / 2];
-};
-constexpr TrianglePairs makeTrianglePairs() {
-    TrianglePairs t{};
-    int p = 0;
-    for (int c = 1; c < kAtmFast; c++)
-        for (int b = 0; b < c; b++) t.bc[p++] = (unsigned short)(b | (c << 8));
-    return t;
-}
-__device__ const TrianglePairs kTrianglePairs = makeTrianglePairs();
+// The longest list the fast kernel takes, by the order the lists were built in.
+__device__ __forceinline__ int fastListMax(const AtmBuffers& A) { return A.flag[3] ? kAtmFast : kAtmFastStaged; }
 
 // A site position as float, wrapped into a rectangular periodic box (unchanged otherwise): the frame of the chunk
 // boxes, in which the minimum-image distance between a point and a box bounds that to every point in the box.
@@ -207,6 +218,7 @@ __global__ void kSiteNeighbors(AtmBuffers A, AtmConfig C) {
         if (count > A.cap) atomicOr(A.flag + 1, 1);
         // flag[2]: some site needs the wide triple kernel (cleared before each build)
         if (count > kAtmFast || count > A.cap) atomicOr(A.flag + 2, 1);
+        if (a == 0) A.flag[3] = 1;
     }
     for (int d = 0; d < 3; d++)
         if (lane == 0) A.siteRef[3 * a + d] = A.sitePos[3 * a + d];
@@ -235,6 +247,8 @@ __global__ void __launch_bounds__(1024) kSiteCellSort(AtmBuffers A, AtmConfig C,
         const int cell = (cz * G.nc[1] + cy) * G.nc[0] + cx;
         G.siteCell[s] = cell;
         G.wrapped[s] = make_float4(p.x, p.y, p.z, __int_as_float(A.molecule[s]));
+        const double f = A.sitePos[3 * s] * C.box.inv[0];
+        G.order[s] = (unsigned)(unsigned long long)((f - floor(f)) * 4294967296.0);
         atomicAdd(&count[cell], 1);
     }
     __syncthreads();
@@ -293,8 +307,8 @@ __global__ void __launch_bounds__(1024) kSiteCellSort(AtmBuffers A, AtmConfig C,
     }
 }
 
-// The list search over the cell grid (rebuild only): one warp per site A takes the sites B > A of other molecules
-// within the list cutoff from the 27 cells around A's cell, in cell order.  The 27 cells' sites are taken as one
+// The list search over the cell grid (rebuild only): one warp per site A takes the sites B after A (siteAfter) of
+// other molecules within the list cutoff from the 27 cells around A's cell, in cell order.  The 27 cells' sites are taken as one
 // sequence (a prefix over the cell sizes), so the lanes stay busy across cell boundaries.  The distance test uses the
 // float wrapped positions of the cell sort with a margin of 1e-4 of the squared list cutoff, far above their rounding
 // (a few 1e-6): the list may hold a pair at the very edge of the list cutoff that the double-precision distance would
@@ -348,7 +362,7 @@ __global__ void __launch_bounds__(256) kSiteNeighborsCells(AtmBuffers A, AtmConf
             b = G.cellSites[cellFirst[w][lo] + (k - before)];
         }
         bool near = false;
-        if (b > a) {
+        if (b >= 0 && siteAfter(G, 0, a, b)) {
             const float4 pb = G.wrapped[b];
             float dx = pb.x - pa.x, dy = pb.y - pa.y, dz = pb.z - pa.z;
             dx -= C.boxf.a[0] * rintf(dx * C.boxf.inv[0]);
@@ -366,7 +380,8 @@ __global__ void __launch_bounds__(256) kSiteNeighborsCells(AtmBuffers A, AtmConf
     if (lane == 0) {
         A.nbrCount[a] = count;
         if (count > A.cap) atomicOr(A.flag + 1, 1);
-        if (count > kAtmFast || count > A.cap) atomicOr(A.flag + 2, 1);
+        if (count > kAtmFastStaged || count > A.cap) atomicOr(A.flag + 2, 1);
+        if (a == 0) A.flag[3] = 0;
         for (int d = 0; d < 3; d++) A.siteRef[3 * a + d] = A.sitePos[3 * a + d];
     }
 }
@@ -399,93 +414,158 @@ __device__ __forceinline__ void centroidDampingF(float r, float invR0, float& g,
     dg = 6.0f * x6 * e * rcpApprox(r);
 }
 
-// One triple (A, B, C) from the displacements AB = (ax, ay, az) and AC = (bx, by, bz) (minimum images) and the three
-// sites' parameters: the C9 coefficient (InteraxThreeBodyForceImpl.h:69-72) with the scale and alchemical factor
-// (ReferenceInteraxThreeBodyIxn.cpp:116-120), the ATM energy and its gradients (InteraxThreeBodyTerms.h:97-146),
-// optionally Tang-Toennies and centroid damping.  Returns false when BC is outside the cutoff or C9 vanishes.
-// fA, fB, fC: the forces on the three sites.
-__device__ __forceinline__ bool atmTriple(const AtmConfig& C, const float4& pa, const float4& pb, const float4& pc,
-                                          float ax, float ay, float az, float bx, float by, float bz, float& energy,
-                                          float3& fA, float3& fB, float3& fC) {
-    // a = AB, b = AC, c = BC (minimum image of C - B)
-    float cx = bx - ax, cy = by - ay, cz = bz - az;
-    if (C.periodic) minimumImageF(cx, cy, cz, C.boxf);
-    const float w = fmaf(cx, cx, fmaf(cy, cy, cz * cz));
-    if (!(w < C.cutoff2)) return false;
-    const float wa = pa.y, wb = pb.y, wc = pc.y;
-    float c9 = 1.5f * pa.x * pb.x * pc.x * wa * wb * wc * ((wa + wb) + wc) *
-               __fdividef(1.0f, (wa + wb) * (wb + wc) * (wc + wa)) * C.scale;
-    if (pa.w != 0.0f || pb.w != 0.0f || pc.w != 0.0f) c9 *= C.lambda;
-    if (c9 == 0.0f) return false;
-    const float u = fmaf(ax, ax, fmaf(ay, ay, az * az));
-    const float v = fmaf(bx, bx, fmaf(by, by, bz * bz));
-    const float pp = fmaf(ax, bx, fmaf(ay, by, az * bz));
-    const float qq = fmaf(ax, cx, fmaf(ay, cy, az * cz));
-    const float ss = fmaf(bx, cx, fmaf(by, cy, bz * cz));
-    const float P = u * v * w;
-    const float y = rsqrtApprox(P);
-    const float invP = y * y;
-    const float invP32 = invP * y;
-    const float invP52 = invP32 * invP;
-    const float pqs = pp * qq * ss;
-    energy = c9 * fmaf(-3.0f * pqs, invP52, invP32);
-    const float radial = c9 * fmaf(15.0f * pqs, invP52, -3.0f * invP32);
-    const float cross = -3.0f * c9 * invP52;
-    const float ru = radial * rcpApprox(u), rv = radial * rcpApprox(v), rw = radial * rcpApprox(w);
-    float gax = ax * ru + (bx * (qq * ss) + cx * (pp * ss)) * cross;
-    float gay = ay * ru + (by * (qq * ss) + cy * (pp * ss)) * cross;
-    float gaz = az * ru + (bz * (qq * ss) + cz * (pp * ss)) * cross;
-    float gbx = bx * rv + (ax * (qq * ss) + cx * (pp * qq)) * cross;
-    float gby = by * rv + (ay * (qq * ss) + cy * (pp * qq)) * cross;
-    float gbz = bz * rv + (az * (qq * ss) + cz * (pp * qq)) * cross;
-    float gcx = cx * rw + (ax * (pp * ss) + bx * (pp * qq)) * cross;
-    float gcy = cy * rw + (ay * (pp * ss) + by * (pp * qq)) * cross;
-    float gcz = cz * rw + (az * (pp * ss) + bz * (pp * qq)) * cross;
-    if (C.useTangToennies || C.invCentroidRadius > 0.0f) {
-        float len[3], invLen[3];
-        len[0] = sqrtRefined(u, invLen[0]);
-        len[1] = sqrtRefined(v, invLen[1]);
-        len[2] = sqrtRefined(w, invLen[2]);
-        const float widths[3] = {pa.z + pb.z, pa.z + pc.z, pb.z + pc.z};
-        float f[3], dfdr[3];
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            if (C.useTangToennies) {
-                const float rate = C.twoBeta * __fdividef(1.0f, widths[k]);
-                tangToennies3f(rate * len[k], f[k], dfdr[k]);
-                dfdr[k] *= rate;
-            }
-            else {
-                f[k] = 1.0f;
-                dfdr[k] = 0.0f;
-            }
-            if (C.invCentroidRadius > 0.0f) {
-                float g, dg;
-                centroidDampingF(len[k], C.invCentroidRadius, g, dg);
-                dfdr[k] = fmaf(dfdr[k], g, f[k] * dg);
-                f[k] *= g;
-            }
-        }
-        const float damping = f[0] * f[1] * f[2];
-        const float sa = energy * dfdr[0] * f[1] * f[2] * invLen[0];
-        const float sb = energy * f[0] * dfdr[1] * f[2] * invLen[1];
-        const float sc = energy * f[0] * f[1] * dfdr[2] * invLen[2];
-        gax = fmaf(gax, damping, ax * sa);
-        gay = fmaf(gay, damping, ay * sa);
-        gaz = fmaf(gaz, damping, az * sa);
-        gbx = fmaf(gbx, damping, bx * sb);
-        gby = fmaf(gby, damping, by * sb);
-        gbz = fmaf(gbz, damping, bz * sb);
-        gcx = fmaf(gcx, damping, cx * sc);
-        gcy = fmaf(gcy, damping, cy * sc);
-        gcz = fmaf(gcz, damping, cz * sc);
-        energy *= damping;
+// A staged neighbor k of site A.  pos: displacement from A and its squared length; par: frequency, the frequency and
+// polarizability part of C9 that A and k make, alchemical (0/1), molecule (int bits); damp (damping only): width, the
+// damping of the A-k distance, its r-derivative over the distance.
+struct SiteDamping {
+    float width, f, dfr;
+};
+
+// Damping of one distance: Tang-Toennies of the two widths' sum and the centroid damping (InteraxThreeBodyTerms.h:51-77),
+// and its r-derivative divided by r.
+__device__ __forceinline__ void siteDamping(const AtmConfig& C, float r2, float widths, float& f, float& dfr) {
+    float invR;
+    const float r = sqrtRefined(r2, invR);
+    float df = 0.0f;
+    f = 1.0f;
+    if (C.useTangToennies) {
+        const float rate = C.twoBeta * __fdividef(1.0f, widths);
+        tangToennies3f(rate * r, f, df);
+        df *= rate;
     }
-    // forceA += dEda + dEdb; forceB += dEdc - dEda; forceC -= dEdb + dEdc (InteraxThreeBodyTerms.h:142-144)
-    fA = make_float3(gax + gbx, gay + gby, gaz + gbz);
-    fB = make_float3(gcx - gax, gcy - gay, gcz - gaz);
-    fC = make_float3(-(gbx + gcx), -(gby + gcy), -(gbz + gcz));
-    return true;
+    if (C.invCentroidRadius > 0.0f) {
+        float g, dg;
+        centroidDampingF(r, C.invCentroidRadius, g, dg);
+        df = fmaf(df, g, f * dg);
+        f *= g;
+    }
+    dfr = df * invR;
+}
+
+// What one warp stages per neighbor.
+template <bool DAMP, int N>
+struct TripleStorage {
+    float4 pos[N];
+    float4 par[N];
+    int site[N];
+    SiteDamping damp[DAMP ? N : 1];
+};
+
+template <bool DAMP, int N>
+__device__ __forceinline__ void storeNeighbor(TripleStorage<DAMP, N>& S, const AtmBuffers& A, const AtmConfig& C,
+                                              const float4& pa, int slot, int b, float x, float y, float z) {
+    const float4 p = A.siteParams[b];
+    const float u = fmaf(x, x, fmaf(y, y, z * z));
+    S.pos[slot] = make_float4(x, y, z, u);
+    // C9 = 3/2 aA aB aC wA wB wC (wA + wB + wC)/((wA + wB)(wB + wC)(wC + wA)) (InteraxThreeBodyForceImpl.h:69-72)
+    //    = (3/2 aA wA) gB gC (1 + wA/(wB + wC)),  g = a w/(wA + w)
+    S.par[slot] = make_float4(p.y, __fdividef(p.x * p.y, pa.y + p.y), p.w, __int_as_float(A.molecule[b]));
+    S.site[slot] = b;
+    if (DAMP) {
+        SiteDamping d;
+        d.width = p.z;
+        siteDamping(C, u, pa.z + p.z, d.f, d.dfr);
+        S.damp[slot] = d;
+    }
+}
+
+// One warp's share of the triples of site A (parameters pa): the neighbors C of storage entries cFirst, cFirst +
+// cStep, ... (8 at a time, below cEnd), each against every neighbor B of entries [bBegin, bEnd).  Four lanes take one
+// C; lane s of them takes B = bBegin + s, + 4, ...  A triple is visited from both sides, and each visit adds the
+// force on its own C only: the same number of warp iterations as visiting it once with half of the lanes idle, and
+// a third of the arithmetic of all three forces.  The force on A is minus the sum of the others'.
+//   energy (InteraxThreeBodyTerms.h:97-146), with a = AB, b = AC, c = BC, p = a.b, q = a.c, s = b.c, P = (a b c)^2:
+//     E = C9 (P^-3/2 - 3 p q s P^-5/2)
+//     -force on C = b (R/b^2 + t) + c (R/c^2 + t) + a X s (p + q),
+//     R = C9 (15 p q s P^-5/2 - 3 P^-3/2), X = -3 C9 P^-5/2, t = X p q
+//   C9 with the scale and the alchemical factor (ReferenceInteraxThreeBodyIxn.cpp:116-120).
+// What bounds it: FP32 issue, about 75 instructions a visit, and for a few thousand sites the latency of the staging
+// (list, position, parameters, three dependent loads).  The earlier form gave each lane a pair (B, C) of a flat
+// triangular index, stored both forces in shared memory and gathered them per neighbor, 425 issue slots per 32 pairs.
+// Kernel times on one B200, both triple kernels, before and now: 96,000-atom box, 0.8 nm, 13.6 M triples: 421 and
+// 159 us; 24,000 atoms, 0.6 nm, 0.46 M triples: 24 and 19 us; 648 atoms: 15.7 and 10.9 us.
+template <bool DAMP, bool IMAGE, int N>
+__device__ __forceinline__ void siteTriples(const TripleStorage<DAMP, N>& S, const AtmBuffers& A, const AtmConfig& C,
+                                            const float4& pa, int cFirst, int cStep, int cEnd, int bBegin, int bEnd,
+                                            int lane, float (&fa)[3], float& energy,
+                                            unsigned long long& visits) {
+    unsigned seen = 0;
+    const int s = lane & 3;
+    const float kA = 1.5f * pa.x * pa.y * C.scale * (pa.w != 0.0f ? C.lambda : 1.0f);
+    const float lambdaBC = pa.w != 0.0f ? 1.0f : C.lambda;
+    for (int c0 = cFirst; c0 < cEnd; c0 += cStep) {
+        const int k = c0 + (lane >> 2);
+        const bool have = k < cEnd;
+        const float4 xc = S.pos[have ? k : cFirst], pc = S.par[have ? k : cFirst];
+        SiteDamping dc;
+        if (DAMP) dc = S.damp[have ? k : cFirst];
+        const float invV = rcpApprox(xc.w);
+        float gx = 0.0f, gy = 0.0f, gz = 0.0f;
+        for (int b = have ? bBegin + s : bEnd; b < bEnd; b += 4) {
+            const float4 xb = S.pos[b], pb = S.par[b];
+            if (__float_as_int(pb.w) == __float_as_int(pc.w)) continue;      // one molecule, B = C among them
+            float cx = xc.x - xb.x, cy = xc.y - xb.y, cz = xc.z - xb.z;
+            if (IMAGE) minimumImageF(cx, cy, cz, C.boxf);
+            const float w = fmaf(cx, cx, fmaf(cy, cy, cz * cz));
+            if (!(w < C.cutoff2)) continue;
+            float c9 = (pb.y * pc.y) * kA * fmaf(pa.y, rcpApprox(pb.x + pc.x), 1.0f);
+            if (pb.z != 0.0f || pc.z != 0.0f) c9 *= lambdaBC;
+            if (c9 == 0.0f) continue;
+            const float p = fmaf(xb.x, xc.x, fmaf(xb.y, xc.y, xb.z * xc.z));
+            const float q = fmaf(xb.x, cx, fmaf(xb.y, cy, xb.z * cz));
+            const float r = fmaf(xc.x, cx, fmaf(xc.y, cy, xc.z * cz));
+            const float y = rsqrtApprox(xb.w * xc.w * w);
+            const float invP = y * y;
+            const float invP32 = invP * y;
+            const float invP52 = invP32 * invP;
+            const float pq = p * q;
+            const float pqr = pq * r;
+            const float e = c9 * fmaf(-3.0f * pqr, invP52, invP32);
+            const float radial = c9 * fmaf(15.0f * pqr, invP52, -3.0f * invP32);
+            const float cross = -3.0f * c9 * invP52;
+            const float t = cross * pq;
+            float kb = fmaf(radial, invV, t), kc = fmaf(radial, rcpApprox(w), t), ka = cross * r * (p + q);
+            if (DAMP) {
+                const SiteDamping db = S.damp[b];
+                float f, dfr;
+                siteDamping(C, w, db.width + dc.width, f, dfr);
+                const float fbc = db.f * f, damping = dc.f * fbc;
+                kb = fmaf(kb, damping, e * fbc * dc.dfr);
+                kc = fmaf(kc, damping, e * db.f * dc.f * dfr);
+                ka *= damping;
+                energy = fmaf(e, damping, energy);
+            }
+            else energy += e;
+            gx = fmaf(xc.x, kb, fmaf(cx, kc, fmaf(xb.x, ka, gx)));
+            gy = fmaf(xc.y, kb, fmaf(cy, kc, fmaf(xb.y, ka, gy)));
+            gz = fmaf(xc.z, kb, fmaf(cz, kc, fmaf(xb.z, ka, gz)));
+            seen++;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int o = 1; o < 4; o <<= 1) {
+            gx += __shfl_xor_sync(0xffffffffu, gx, o);
+            gy += __shfl_xor_sync(0xffffffffu, gy, o);
+            gz += __shfl_xor_sync(0xffffffffu, gz, o);
+        }
+        fa[0] += gx;
+        fa[1] += gy;
+        fa[2] += gz;
+        // lane s of the four adds component s
+        const float g = s == 0 ? gx : (s == 1 ? gy : gz);
+        if (have && s < 3 && g != 0.0f) atomicAddFixed(A.siteForce + s * C.numSites + S.site[k], -toFixed(g));
+    }
+    visits += seen;
+}
+
+// The force on A of a warp's share (the four lanes of a C hold the same sums).
+__device__ __forceinline__ void addSiteForce(const AtmBuffers& A, const AtmConfig& C, int a, int lane,
+                                             const float (&fa)[3]) {
+    float f[3] = {fa[0], fa[1], fa[2]};
+    for (int o = 4; o < 32; o <<= 1)
+        for (int d = 0; d < 3; d++) f[d] += __shfl_xor_sync(0xffffffffu, f[d], o);
+    const float g = lane == 0 ? f[0] : (lane == 1 ? f[1] : f[2]);
+    if (lane < 3 && g != 0.0f) atomicAddFixed(A.siteForce + lane * C.numSites + a, toFixed(g));
 }
 
 // Stage the neighbors of site a that are within the cutoff (in list order) with their displacements from a and their
@@ -514,20 +594,20 @@ __device__ __forceinline__ int stageTripleNeighbors(const AtmBuffers& A, const A
     return m;
 }
 
-// The same for a site whose list overflowed its capacity: every later site of another molecule is tested against the
-// cutoff, which gives the same neighbors within the cutoff (in increasing order), so the same triples are evaluated.
+// The same for a site whose list overflowed its capacity: every site after it (in the order of the lists' build) of
+// another molecule is tested against the cutoff, which gives the same neighbors, so the same triples are evaluated.
 // The reference falls back the same way
 // (platforms/common/src/kernels/interaxThreeBody.cc:111-112, 437-438).
 template <class Store>
 __device__ __forceinline__ int stageTripleNeighborsScan(const AtmBuffers& A, const AtmConfig& C, int a, int lane,
                                                         int first, int capacity, Store store) {
-    const int molA = A.molecule[a];
+    const int molA = A.molecule[a], byIndex = A.flag[3];
     int m = 0;
-    for (int b0 = a + 1; b0 < C.numSites; b0 += 32) {
+    for (int b0 = byIndex ? a + 1 : 0; b0 < C.numSites; b0 += 32) {
         const int b = b0 + lane;
         bool in = false;
         double d[3];
-        if (b < C.numSites && A.molecule[b] != molA) {
+        if (b < C.numSites && A.molecule[b] != molA && siteAfter(A.cells, byIndex, a, b)) {
             siteDelta(A, C, a, b, d);
             in = (float)(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]) < C.cutoff2;
         }
@@ -541,289 +621,129 @@ __device__ __forceinline__ int stageTripleNeighborsScan(const AtmBuffers& A, con
     return m;
 }
 
-struct AtmFastStorage {
-    float4 pos[kAtmFast];        // displacement from A; w holds the molecule (int bits)
-    float4 params[kAtmFast];
-    int site[kAtmFast];
-    float4 fb[kAtmAccum ? 1 : kAtmRound];   // force on B of each pair of the current round
-    float4 fc[kAtmAccum ? 1 : kAtmRound];   // force on C
-    unsigned long long acc[kAtmAccum ? 3 : 1][kAtmAccum ? kAtmFast : 1];   // fixed-point force sums per neighbor
-};
-
+template <bool DAMP, bool IMAGE>
 __global__ void __launch_bounds__(32 * kAtmFastWarps, IX_TUNE_ATM_MIN_BLOCKS) kTriplesFast(AtmBuffers A, AtmConfig C) {
-    __shared__ AtmFastStorage storage[kAtmFastWarps];
+    __shared__ TripleStorage<DAMP, kAtmFastStaged> storage[kAtmFastWarps];
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < C.zeroSlots; k += gridDim.x * blockDim.x)
         A.energyPartials[C.zeroOffset + k] = 0.0;
-    AtmFastStorage& S = storage[threadIdx.x >> 5];
+    auto& S = storage[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const int warp = blockIdx.x * kAtmFastWarps + (threadIdx.x >> 5);
+    const int fastMax = fastListMax(A);
     double eAcc = 0.0;
-    unsigned long long triples = 0;
+    unsigned long long visits = 0;
     for (int a = warp; a < C.numSites; a += gridDim.x * kAtmFastWarps) {
         const int n = A.nbrCount[a];
-        if (n > kAtmFast || n > A.cap) continue;      // the wide kernel takes this site
+        if (n > fastMax || n > A.cap) continue;        // the wide kernel takes this site
         const float4 pa = A.siteParams[a];
         __syncwarp();
-        const int m = stageTripleNeighbors(A, C, a, n, lane, 0, kAtmFast,
+        const int m = stageTripleNeighbors(A, C, a, n, lane, 0, kAtmFastStaged,
                                            [&](int slot, int b, float x, float y, float z) {
-                                               S.pos[slot] = make_float4(x, y, z, __int_as_float(A.molecule[b]));
-                                               S.params[slot] = A.siteParams[b];
-                                               S.site[slot] = b;
+                                               storeNeighbor(S, A, C, pa, slot, b, x, y, z);
                                            });
         __syncwarp();
         float fa[3] = {0.0f, 0.0f, 0.0f};
-        float f0[3] = {0.0f, 0.0f, 0.0f}, f1[3] = {0.0f, 0.0f, 0.0f};   // staged neighbors lane, lane + 32
         float eSite = 0.0f;
-        int next0 = lane + 1, next1 = lane + 33;    // next C of the pairs (k, C) each lane gathers as B
-        const int numPairs = m * (m - 1) / 2;
-        if constexpr (kAtmAccum) {
-            // each triple's B and C forces go to the neighbors' fixed-point sums (integer adds: the order of the
-            // lanes does not change them), flushed once per site
-            for (int k = lane; k < m; k += 32) S.acc[0][k] = S.acc[1][k] = S.acc[2][k] = 0ull;
-            __syncwarp();
-            for (int q = lane; q < numPairs; q += 32) {
-                const unsigned bc = __ldg(kTrianglePairs.bc + q);
-                const int b = bc & 0xff, c = bc >> 8;
-                const float4 xb = S.pos[b], xc = S.pos[c];
-                if (__float_as_int(xb.w) == __float_as_int(xc.w)) continue;
-                float e;
-                float3 fA, fB, fC;
-                if (!atmTriple(C, pa, S.params[b], S.params[c], xb.x, xb.y, xb.z, xc.x, xc.y, xc.z, e, fA, fB, fC))
-                    continue;
-                fa[0] += fA.x;
-                fa[1] += fA.y;
-                fa[2] += fA.z;
-                eSite += e;
-                triples++;
-                atomicAdd(&S.acc[0][b], (unsigned long long)toFixed(fB.x));
-                atomicAdd(&S.acc[1][b], (unsigned long long)toFixed(fB.y));
-                atomicAdd(&S.acc[2][b], (unsigned long long)toFixed(fB.z));
-                atomicAdd(&S.acc[0][c], (unsigned long long)toFixed(fC.x));
-                atomicAdd(&S.acc[1][c], (unsigned long long)toFixed(fC.y));
-                atomicAdd(&S.acc[2][c], (unsigned long long)toFixed(fC.z));
-            }
-            __syncwarp();
-            for (int k = lane; k < m; k += 32) {
-                const int b = S.site[k];
-                for (int d = 0; d < 3; d++)
-                    if (S.acc[d][k]) atomicAddFixed(A.siteForce + d * C.numSites + b, (long long)S.acc[d][k]);
-            }
-        }
-        else
-        for (int base = 0; base < numPairs; base += kAtmRound) {
-            const int count = min(kAtmRound, numPairs - base);
-            for (int q = lane; q < count; q += 32) {
-                const unsigned bc = __ldg(kTrianglePairs.bc + base + q);
-                const int b = bc & 0xff, c = bc >> 8;
-                const float4 xb = S.pos[b], xc = S.pos[c];
-                float3 fB = make_float3(0.0f, 0.0f, 0.0f), fC = fB;
-                if (__float_as_int(xb.w) != __float_as_int(xc.w)) {
-                    float e;
-                    float3 fA;
-                    if (atmTriple(C, pa, S.params[b], S.params[c], xb.x, xb.y, xb.z, xc.x, xc.y, xc.z, e, fA, fB, fC)) {
-                        fa[0] += fA.x;
-                        fa[1] += fA.y;
-                        fa[2] += fA.z;
-                        eSite += e;
-                        triples++;
-                    }
-                    else fB = fC = make_float3(0.0f, 0.0f, 0.0f);
-                }
-                S.fb[q] = make_float4(fB.x, fB.y, fB.z, 0.0f);
-                S.fc[q] = make_float4(fC.x, fC.y, fC.z, 0.0f);
-            }
-            __syncwarp();
-            // gather, for the staged neighbors k = lane and lane + 32: the pairs (b, k) with b < k (contiguous) and
-            // the pairs (k, c) with c > k (increasing p as c grows)
-            auto gather = [&](int k, float f[3], int& next) {
-                if (k >= m) return;
-                const int first = k * (k - 1) / 2;
-                const int lo = max(first, base), hi = min(first + k, base + count);
-                for (int p = lo; p < hi; p++) {
-                    const float4 v = S.fc[p - base];
-                    f[0] += v.x;
-                    f[1] += v.y;
-                    f[2] += v.z;
-                }
-                for (; next < m; next++) {
-                    const int p = next * (next - 1) / 2 + k;
-                    if (p >= base + count) break;
-                    const float4 v = S.fb[p - base];
-                    f[0] += v.x;
-                    f[1] += v.y;
-                    f[2] += v.z;
-                }
-            };
-            gather(lane, f0, next0);
-            gather(lane + 32, f1, next1);
-            __syncwarp();
-        }
-        // the staged neighbors' forces, then A's (a fixed reduction tree over the lanes)
-        auto flush = [&](int k, const float f[3]) {
-            if (k >= m) return;
-            const int b = S.site[k];
-            if (f[0] != 0.0f) atomicAddFixed(A.siteForce + b, toFixed(f[0]));
-            if (f[1] != 0.0f) atomicAddFixed(A.siteForce + C.numSites + b, toFixed(f[1]));
-            if (f[2] != 0.0f) atomicAddFixed(A.siteForce + 2 * C.numSites + b, toFixed(f[2]));
-        };
-        if constexpr (!kAtmAccum) {
-            flush(lane, f0);
-            flush(lane + 32, f1);
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-            fa[0] += __shfl_xor_sync(0xffffffffu, fa[0], o);
-            fa[1] += __shfl_xor_sync(0xffffffffu, fa[1], o);
-            fa[2] += __shfl_xor_sync(0xffffffffu, fa[2], o);
-        }
-        if (lane == 0) {
-            if (fa[0] != 0.0f) atomicAddFixed(A.siteForce + a, toFixed(fa[0]));
-            if (fa[1] != 0.0f) atomicAddFixed(A.siteForce + C.numSites + a, toFixed(fa[1]));
-            if (fa[2] != 0.0f) atomicAddFixed(A.siteForce + 2 * C.numSites + a, toFixed(fa[2]));
-        }
+        siteTriples<DAMP, IMAGE>(S, A, C, pa, 0, 8, m, 0, m, lane, fa, eSite, visits);
+        addSiteForce(A, C, a, lane, fa);
         eAcc += (double)eSite;
     }
-    const double sum = warpSumD(eAcc);
+    const double sum = 0.5 * warpSumD(eAcc);           // each triple was visited twice
     if (lane == 0) A.energyPartials[warp] = sum;
-    for (int o = 16; o > 0; o >>= 1) triples += __shfl_xor_sync(0xffffffffu, triples, o);
-    if (lane == 0 && triples) atomicAdd(A.tripleCount, triples);
+    for (int o = 16; o > 0; o >>= 1) visits += __shfl_xor_sync(0xffffffffu, visits, o);
+    if (lane == 0 && visits) atomicAdd(A.tripleVisits, visits);
 }
-
-struct AtmWarpStorage {
-    float dx[256], dy[256], dz[256];
-    float4 params[256];
-    int mol[256];
-    int site[256];
-    float fx[256], fy[256], fz[256];
-};
 
 constexpr int kAtmWarps = 4;
 constexpr int kAtmMaxStaged = 256;
 constexpr int kAtmChunk = kAtmMaxStaged / 2;
-// Each long-list site is taken by this many warps, each evaluating every kAtmWideParts-th group of 32 of its pairs:
+// Each long-list site is taken by this many warps, each evaluating every kAtmWideParts-th group of 8 of its neighbors:
 // a site near the start of a large cluster has tens of thousands of (B, C) pairs, which one warp would take alone.
 constexpr int kAtmWideParts = 8;
 
-// Sites whose lists are longer than kAtmFast, in units (site, part) of kAtmWideParts parts per site.  A unit stages up
-// to kAtmMaxStaged neighbors within the cutoff at once and evaluates its part of their pairs, enumerated by a flat
-// triangular index; a longer list is taken in chunks of kAtmChunk, each pair of chunks (I <= J) staged side by side,
-// so any length is handled.  The forces on B and C accumulate in shared memory and are flushed to the fixed-point
-// site forces after each staging (integer sums: the split changes no result's dependence on the order).  Energies go
-// to energyPartials[partialsOffset + warp]: with a grid of one warp per unit, one slot per unit (unit = site x
-// kAtmWideParts + part).
-// `gate` (may be null): the kernel returns at once unless *gate is set (a list longer than kAtmFast exists).
+// Sites whose lists are longer than the fast kernel takes, in units (site, part) of kAtmWideParts parts per site.  A
+// unit stages up to kAtmMaxStaged neighbors within the cutoff at once and evaluates its part of them against all; a
+// longer list is taken in chunks of kAtmChunk, each pair of chunks staged side by side, so any length is handled.
+// Energies go to energyPartials[partialsOffset + warp]: with a grid of one warp per unit, one slot per unit (unit =
+// site x kAtmWideParts + part).
+// `gate` (may be null): the kernel returns at once unless *gate is set (a list longer than the fast kernel takes).
+template <bool DAMP, bool IMAGE>
 __global__ void __launch_bounds__(32 * kAtmWarps) kTriplesWide(AtmBuffers A, AtmConfig C, int partialsOffset,
                                                                const int* gate) {
     if (gate && *(volatile const int*)gate == 0) return;
-    extern __shared__ unsigned char atmShared[];
-    AtmWarpStorage& S = reinterpret_cast<AtmWarpStorage*>(atmShared)[threadIdx.x >> 5];
+    extern __shared__ float4 atmShared[];
+    auto& S = reinterpret_cast<TripleStorage<DAMP, kAtmMaxStaged>*>(atmShared)[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
+    const int fastMax = fastListMax(A);
     double eAcc = 0.0;
-    unsigned long long triples = 0;
+    unsigned long long visits = 0;
     const int units = C.numSites * kAtmWideParts;
     for (int u = blockIdx.x * kAtmWarps + (threadIdx.x >> 5); u < units; u += gridDim.x * kAtmWarps) {
         const int a = u / kAtmWideParts, part = u % kAtmWideParts;
         const int n = A.nbrCount[a];
-        if (n <= kAtmFast && n <= A.cap) continue;     // the fast kernel takes this site
+        if (n <= fastMax && n <= A.cap) continue;      // the fast kernel takes this site
         const float4 pa = A.siteParams[a];
-        const bool scan = n > A.cap;                   // the list overflowed: scan every later site
+        const bool scan = n > A.cap;                   // the list overflowed: scan the sites
         auto stage = [&](int first, int base, int capacity) {
             auto store = [&](int slot, int b, float x, float y, float z) {
-                const int k = base + slot;
-                S.dx[k] = x;
-                S.dy[k] = y;
-                S.dz[k] = z;
-                S.params[k] = A.siteParams[b];
-                S.mol[k] = A.molecule[b];
-                S.site[k] = b;
-                S.fx[k] = 0.0f;
-                S.fy[k] = 0.0f;
-                S.fz[k] = 0.0f;
+                storeNeighbor(S, A, C, pa, base + slot, b, x, y, z);
             };
             return scan ? stageTripleNeighborsScan(A, C, a, lane, first, capacity, store)
                         : stageTripleNeighbors(A, C, a, n, lane, first, capacity, store);
         };
-        float fax = 0.0f, fay = 0.0f, faz = 0.0f;
-        auto pair = [&](int b, int c) {
-            if (S.mol[b] == S.mol[c]) return;
-            float energy;
-            float3 fA, fB, fC;
-            if (!atmTriple(C, pa, S.params[b], S.params[c], S.dx[b], S.dy[b], S.dz[b], S.dx[c], S.dy[c], S.dz[c],
-                           energy, fA, fB, fC))
-                return;
-            fax += fA.x;
-            fay += fA.y;
-            faz += fA.z;
-            atomicAdd(&S.fx[b], fB.x);
-            atomicAdd(&S.fy[b], fB.y);
-            atomicAdd(&S.fz[b], fB.z);
-            atomicAdd(&S.fx[c], fC.x);
-            atomicAdd(&S.fy[c], fC.y);
-            atomicAdd(&S.fz[c], fC.z);
-            eAcc += energy;
-            triples++;
-        };
-        auto triangle = [&](int m) {
-            const int numPairs = m * (m - 1) / 2;
-            for (int p = lane + 32 * part; p < numPairs; p += 32 * kAtmWideParts) {
-                // p = c (c - 1)/2 + b with b < c
-                int c = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)p)) * 0.5f);
-                while (c * (c - 1) / 2 > p) c--;
-                while ((c + 1) * c / 2 <= p) c++;
-                pair(p - c * (c - 1) / 2, c);
-            }
-        };
-        auto flush = [&](int lo, int hi) {
-            for (int k = lo + lane; k < hi; k += 32) {
-                const int b = S.site[k];
-                if (S.fx[k] != 0.0f) atomicAddFixed(A.siteForce + b, toFixed(S.fx[k]));
-                if (S.fy[k] != 0.0f) atomicAddFixed(A.siteForce + C.numSites + b, toFixed(S.fy[k]));
-                if (S.fz[k] != 0.0f) atomicAddFixed(A.siteForce + 2 * C.numSites + b, toFixed(S.fz[k]));
-            }
-        };
+        float fa[3] = {0.0f, 0.0f, 0.0f};
+        float energy = 0.0f;
         __syncwarp();
         const int m = stage(0, 0, kAtmMaxStaged);
         __syncwarp();
         if (m <= kAtmMaxStaged) {
-            triangle(m);
-            __syncwarp();
-            flush(0, m);
+            siteTriples<DAMP, IMAGE>(S, A, C, pa, 8 * part, 8 * kAtmWideParts, m, 0, m, lane, fa, energy, visits);
+            eAcc += (double)energy;
         }
         else {
             const int chunks = (m + kAtmChunk - 1) / kAtmChunk;
             for (int I = 0; I < chunks; I++) {
                 const int cI = min(kAtmChunk, m - I * kAtmChunk);
-                for (int J = I; J < chunks; J++) {
+                for (int J = 0; J < chunks; J++) {
                     const int cJ = min(kAtmChunk, m - J * kAtmChunk);
                     __syncwarp();
                     stage(I * kAtmChunk, 0, kAtmChunk);
                     if (J != I) stage(J * kAtmChunk, kAtmChunk, kAtmChunk);
                     __syncwarp();
-                    if (J == I) triangle(cI);
-                    else
-                        for (int p = lane + 32 * part; p < cI * cJ; p += 32 * kAtmWideParts)
-                            pair(p / cJ, kAtmChunk + p % cJ);
-                    __syncwarp();
-                    flush(0, cI);
-                    if (J != I) flush(kAtmChunk, kAtmChunk + cJ);
+                    const int b0 = J == I ? 0 : kAtmChunk;
+                    energy = 0.0f;
+                    siteTriples<DAMP, IMAGE>(S, A, C, pa, 8 * part, 8 * kAtmWideParts, cI, b0, b0 + cJ, lane, fa,
+                                             energy, visits);
+                    eAcc += (double)energy;
                 }
             }
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            fax += __shfl_xor_sync(0xffffffffu, fax, o);
-            fay += __shfl_xor_sync(0xffffffffu, fay, o);
-            faz += __shfl_xor_sync(0xffffffffu, faz, o);
-        }
-        if (lane == 0) {
-            if (fax != 0.0f) atomicAddFixed(A.siteForce + a, toFixed(fax));
-            if (fay != 0.0f) atomicAddFixed(A.siteForce + C.numSites + a, toFixed(fay));
-            if (faz != 0.0f) atomicAddFixed(A.siteForce + 2 * C.numSites + a, toFixed(faz));
-        }
+        addSiteForce(A, C, a, lane, fa);
         __syncwarp();
     }
-    const double sum = warpSumD(eAcc);
+    const double sum = 0.5 * warpSumD(eAcc);
     if (lane == 0) A.energyPartials[partialsOffset + blockIdx.x * kAtmWarps + (threadIdx.x >> 5)] = sum;
-    for (int o = 16; o > 0; o >>= 1) triples += __shfl_xor_sync(0xffffffffu, triples, o);
-    if (lane == 0 && triples) atomicAdd(A.tripleCount, triples);
+    for (int o = 16; o > 0; o >>= 1) visits += __shfl_xor_sync(0xffffffffu, visits, o);
+    if (lane == 0 && visits) atomicAdd(A.tripleVisits, visits);
+}
+
+// The fast kernel, and the wide one where its grid is not empty.
+template <bool DAMP, bool IMAGE>
+static void launchTriplesAs(const AtmBuffers& A, const AtmConfig& C, int fastBlocks, int wideBlocks, const int* gate,
+                            cudaStream_t st) {
+    kTriplesFast<DAMP, IMAGE><<<fastBlocks, 32 * kAtmFastWarps, 0, st>>>(A, C);
+    if (wideBlocks > 0)
+        kTriplesWide<DAMP, IMAGE><<<wideBlocks, 32 * kAtmWarps,
+                                    kAtmWarps * sizeof(TripleStorage<DAMP, kAtmMaxStaged>), st>>>(
+            A, C, fastBlocks * kAtmFastWarps, gate);
+}
+static void launchTriples(const AtmBuffers& A, const AtmConfig& C, int fastBlocks, int wideBlocks, const int* gate,
+                          cudaStream_t st) {
+    const bool damp = C.useTangToennies || C.invCentroidRadius > 0.0f;
+    if (damp && C.imageBC) launchTriplesAs<true, true>(A, C, fastBlocks, wideBlocks, gate, st);
+    else if (damp) launchTriplesAs<true, false>(A, C, fastBlocks, wideBlocks, gate, st);
+    else if (C.imageBC) launchTriplesAs<false, true>(A, C, fastBlocks, wideBlocks, gate, st);
+    else launchTriplesAs<false, false>(A, C, fastBlocks, wideBlocks, gate, st);
 }
 
 // Each particle of a site receives the site force divided by the number of particles

@@ -41,7 +41,7 @@ __global__ void kBatchEnergies(int numSystems, const int* tileStart, const doubl
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s == 0) {
         counts[2] = counts[0];
-        counts[3] = counts[1];
+        counts[3] = counts[1] / 2;   // visits, two a triple
         counts[0] = 0;
         counts[1] = 0;
         *taskCounter = 0;
@@ -481,7 +481,7 @@ int buildBatchSites(ix_batch* b) {
     A.siteParams = dParams;
     IX_TRY(batchAlloc(b, "sitePos", 3 * (size_t)ns, &A.sitePos));
     IX_TRY(batchUpload(b, "siteRef", std::vector<double>(3 * (size_t)ns, 0.0), &A.siteRef));
-    IX_TRY(batchUpload(b, "atmFlag", std::vector<int>{0, 0, 0, 0}, &A.flag));
+    IX_TRY(batchUpload(b, "atmFlag", std::vector<int>{0, 0, 0, 1}, &A.flag));
     IX_TRY(batchUpload(b, "nbrCount", count, &A.nbrCount));
     IX_TRY(batchUpload(b, "nbr", nbr, &A.nbr));
     A.cap = cap;
@@ -497,7 +497,7 @@ int buildBatchSites(ix_batch* b) {
     const size_t slots = (size_t)b->atmFastBlocks * kAtmFastWarps + (size_t)wideBlocks * kAtmWarps;
     IX_TRY(batchUpload(b, "sitePartials", std::vector<double>(slots, 0.0), &b->sitePartials));
     A.energyPartials = b->sitePartials;
-    A.tripleCount = b->dCounts + 1;
+    A.tripleVisits = b->dCounts + 1;
     return IX_OK;
 }
 
@@ -529,10 +529,7 @@ int enqueueBatch(ix_batch* b) {
         const AtmConfig& C = b->atmC;
         const int gS = (b->numSites + tpb - 1) / tpb;
         kSiteCentroids<<<gS, tpb, 0, st>>>(A, C, b->dPos);
-        kTriplesFast<<<b->atmFastBlocks, 32 * kAtmFastWarps, 0, st>>>(A, C);
-        if (b->atmWideBlocks > 0)
-            kTriplesWide<<<b->atmWideBlocks, 32 * kAtmWarps, sizeof(AtmWarpStorage) * kAtmWarps, st>>>(
-                A, C, b->atmFastBlocks * kAtmFastWarps, nullptr);
+        launchTriples(A, C, b->atmFastBlocks, b->atmWideBlocks, nullptr, st);
         kSpreadSiteForces<<<gS, tpb, 0, st>>>(A, C);
     }
     kFinalize<<<(b->numParticles + tpb - 1) / tpb, tpb, 0, st>>>(b->numParticles, L.np, L.slotOf, b->P.forceFixed,

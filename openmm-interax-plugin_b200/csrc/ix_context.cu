@@ -969,6 +969,7 @@ static int allocateAtm(ix_ctx* ctx) {
         IX_TRY(deviceAlloc(ctx, "siteCellSites", ns, &A.cells.cellSites));
         IX_TRY(deviceAlloc(ctx, "siteCell", ns, &A.cells.siteCell));
         IX_TRY(deviceAlloc(ctx, "siteWrapped", ns, &A.cells.wrapped));
+        IX_TRY(deviceAlloc(ctx, "siteOrder", ns, &A.cells.order));
         // the one-block cell sort scatters up to kSiteSortSharedMax sites in dynamic shared memory (on this device)
         IX_CUDA(ctx, cudaFuncSetAttribute(kSiteCellSort, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           kSiteSortSharedMax * (int)sizeof(int)));
@@ -1011,7 +1012,7 @@ static int allocateAtm(ix_ctx* ctx) {
                                                               (long long)ctx->numSMs * 4));
     IX_TRY(deviceAlloc(ctx, "atmPartials", atmPartialCount(ctx), &ctx->dAtmPartials));
     A.energyPartials = ctx->dAtmPartials;
-    A.tripleCount = ctx->dCounts + 1;
+    A.tripleVisits = ctx->dCounts + 1;
     ctx->atmAllocated = true;
     ctx->atmDirty = true;
     bumpVersion(ctx);
@@ -1140,7 +1141,7 @@ __device__ void reduceEnergiesBlock(const EnergyReduction& R, int block, int num
         if (t == 0) {
             if (R.counts) {
                 R.counts[2] = R.counts[0];
-                R.counts[3] = R.counts[1];
+                R.counts[3] = R.counts[1] / 2;   // the triple kernels count visits, two a triple
                 R.counts[0] = 0;
                 R.counts[1] = 0;
             }
@@ -1414,6 +1415,7 @@ static int launchEvaluation(ix_ctx* ctx, unsigned terms, double* outForces, doub
         C.twoBeta = (float)(2.0 * ctx->atmDampingScale);
         C.invCentroidRadius = ctx->atmCentroidRadius > 0 ? (float)(1.0 / ctx->atmCentroidRadius) : 0.0f;
         C.maxMove2 = 0.25f * kSiteSkin * kSiteSkin;
+        C.imageBC = tripleNeedsImages(C, ctx->atmCutoff);
         const int tpb = 256;
         const int gS = (C.numSites + 63) / 64;   // 64-thread blocks, so that a few thousand sites reach every SM
         // the wide kernel's energy slots start at zero (it runs only while some list is long)
@@ -1445,10 +1447,9 @@ static int launchEvaluation(ix_ctx* ctx, unsigned terms, double* outForces, doub
         else kSiteNeighbors<<<(C.numSites * 32 + tpb - 1) / tpb, tpb, 0, sa>>>(A, C);
         kClearFlag<<<1, 1, 0, sa>>>(A.flag);
         recordTiming(ctx, 2, sa);
-        kTriplesFast<<<ctx->atmFastBlocks, 32 * kAtmFastWarps, 0, sa>>>(A, C);
-        // the sites whose lists are too long for the fast kernel: the kernel returns at once when there are none
-        kTriplesWide<<<ctx->atmGridBlocks, 32 * kAtmWarps, sizeof(AtmWarpStorage) * kAtmWarps, sa>>>(
-            A, C, ctx->atmFastBlocks * kAtmFastWarps, A.flag + 2);
+        // the sites whose lists are too long for the fast kernel go to the wide one, which returns at once when there
+        // are none
+        launchTriples(A, C, ctx->atmFastBlocks, ctx->atmGridBlocks, A.flag + 2, sa);
         ctx->launches += 6;
         recordTiming(ctx, 3, sa);
         ctx->evAtm = ctx->profiling;
@@ -3061,7 +3062,7 @@ struct NoAllocScratch {
     double energy[4];
     double energyBlocks[4];      // the energy reduction's block sum (one block)
     unsigned reduceTicket;
-    int flag[3];
+    int flag[4];
     unsigned long long tripleCount;
 };
 
@@ -3206,6 +3207,7 @@ int ix_three_body_noalloc(int num_particles, const double* d_positions, const do
     C.twoBeta = (float)(2.0 * damping_scale);
     C.invCentroidRadius = centroid_damping_radius > 0 ? (float)(1.0 / centroid_damping_radius) : 0.0f;
     C.maxMove2 = 0.0f;
+    C.imageBC = tripleNeedsImages(C, cutoff);
     AtmBuffers A{};
     A.siteParams = S->siteParams;
     A.molecule = S->molecule;
@@ -3219,15 +3221,12 @@ int ix_three_body_noalloc(int num_particles, const double* d_positions, const do
     A.particleForce = S->particleForce;
     A.numParticles = num_particles;
     A.energyPartials = S->energyPartials;
-    A.tripleCount = &S->tripleCount;
+    A.tripleVisits = &S->tripleCount;
     if (num_sites > 0) {
         kSiteNeighbors<<<(num_sites * 32 + tpb - 1) / tpb, tpb, 0, st>>>(A, C);
         const int fastBlocks = (num_sites + kAtmFastWarps - 1) / kAtmFastWarps;
         const int blocks = std::max(1, std::min((num_sites + kAtmWarps - 1) / kAtmWarps, kNoAllocBlocks));
-        kTriplesFast<<<fastBlocks, 32 * kAtmFastWarps, 0, st>>>(A, C);
-        kTriplesWide<<<blocks, 32 * kAtmWarps, sizeof(AtmWarpStorage) * kAtmWarps, st>>>(A, C,
-                                                                                        fastBlocks * kAtmFastWarps,
-                                                                                        nullptr);
+        launchTriples(A, C, fastBlocks, blocks, nullptr, st);
         kNoAllocSpread<<<(num_sites + tpb - 1) / tpb, tpb, 0, st>>>(S, num_particles, num_sites, d_site_offsets,
                                                                    d_site_particles);
         kReduceEnergies<<<1, 256, 0, st>>>(nullptr, nullptr, 0, S->energyPartials,

@@ -42,22 +42,22 @@
 #ifndef IX_TUNE_PAIR_SKIN
 #define IX_TUNE_PAIR_SKIN 0.1f
 #endif
-// three-body: skin of the site lists, the longest list the fast triple kernel takes, (B, C) pairs per round
+// three-body: skin of the site lists, the longest index-ordered list the fast triple kernel takes
 #ifndef IX_TUNE_SITE_SKIN
 #define IX_TUNE_SITE_SKIN 0.1f
 #endif
 #ifndef IX_TUNE_ATM_FAST
 #define IX_TUNE_ATM_FAST 64
 #endif
-#ifndef IX_TUNE_ATM_ROUND
-#define IX_TUNE_ATM_ROUND 64
-#endif
 // three-body: minimum resident blocks of the fast triple kernel per SM (bounds its registers per thread)
 #ifndef IX_TUNE_ATM_MIN_BLOCKS
 #define IX_TUNE_ATM_MIN_BLOCKS 7
 #endif
-// three-body: 1 = the fast kernel adds each triple's B and C forces to per-neighbor 64-bit fixed-point sums in shared
-// memory (integer atomics, no rounds); 0 = it stores them per round and gathers them per neighbor
+// Named by recorded tuning files and read by no kernel: the triple kernels keep their forces in registers, without
+// rounds of stored forces and without shared-memory sums.
+#ifndef IX_TUNE_ATM_ROUND
+#define IX_TUNE_ATM_ROUND 64
+#endif
 #ifndef IX_TUNE_ATM_ACCUM
 #define IX_TUNE_ATM_ACCUM 0
 #endif

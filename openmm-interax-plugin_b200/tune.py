@@ -56,10 +56,7 @@ GROUPS = [
     ("pair table", [dict(IX_TUNE_PAIR_SHARED_TABLE_BYTES=b) for b in (0, 1024, 2048)]),
     ("pair columns", [dict(IX_TUNE_PAIR_COLUMN_TRANSPOSE=v) for v in (0, 1)]),
     ("pair skin", [dict(IX_TUNE_PAIR_SKIN=s) for s in (0.06, 0.08, 0.1, 0.12)]),
-    ("three-body", [dict(IX_TUNE_ATM_FAST=f, IX_TUNE_ATM_ROUND=r, IX_TUNE_ATM_MIN_BLOCKS=b, IX_TUNE_ATM_ACCUM=acc)
-                    for f, r, b, acc in ((64, 64, 7, 0), (64, 64, 8, 0), (64, 64, 10, 0), (32, 32, 12, 0),
-                                         (64, 32, 8, 0), (64, 128, 7, 0), (64, 128, 8, 0), (64, 256, 5, 0),
-                                         (64, 128, 7, 1))]),
+    ("three-body", [dict(IX_TUNE_ATM_FAST=f, IX_TUNE_ATM_MIN_BLOCKS=b) for f, b in ((64, 7), (64, 8), (32, 8))]),
     ("site skin", [dict(IX_TUNE_SITE_SKIN=s) for s in (0.05, 0.1, 0.15)]),
 ]
 
