@@ -35,7 +35,7 @@ struct AtmConfig {
     float twoBeta;               // 2 x damping scale
     float invCentroidRadius;     // 0 = no centroid damping
     float maxMove2;
-    int zeroSlots, zeroOffset;   // energy slots the fast kernel clears (those of a wide kernel that may not run)
+    int zeroSlots, zeroOffset;   // energy slots the centroid kernel clears (those of a wide kernel that may not run)
     int imageBC;                 // the displacement of C from B can need a minimum image of its own
 };
 
@@ -133,6 +133,7 @@ __device__ __forceinline__ float siteBoxDist2(const AtmConfig& C, float3 p, floa
 
 __global__ void kSiteCentroids(AtmBuffers A, AtmConfig C, const double* pos) {
     int s = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int k = s; k < C.zeroSlots; k += gridDim.x * blockDim.x) A.energyPartials[C.zeroOffset + k] = 0.0;
     bool moved = false;
     float3 w = make_float3(INFINITY, INFINITY, INFINITY), wMax = make_float3(-INFINITY, -INFINITY, -INFINITY);
     if (s < C.numSites) {
@@ -237,6 +238,7 @@ __global__ void __launch_bounds__(1024) kSiteCellSort(AtmBuffers A, AtmConfig C,
     const SiteCells& G = A.cells;
     const int numCells = G.nc[0] * G.nc[1] * G.nc[2];
     const int t = threadIdx.x, T = blockDim.x;
+    if (t == 0) A.flag[2] = 0;      // set again by the lists that follow
     for (int c = t; c < numCells; c += T) count[c] = 0;
     __syncthreads();
     for (int s = t; s < C.numSites; s += T) {
@@ -317,72 +319,72 @@ __global__ void __launch_bounds__(1024) kSiteCellSort(AtmBuffers A, AtmConfig C,
 __global__ void __launch_bounds__(256) kSiteNeighborsCells(AtmBuffers A, AtmConfig C) {
     if (*(volatile int*)A.flag == 0) return;
     __shared__ int cellFirst[8][32], cellEnd[8][32];   // per warp: each cell's first site and its end in the sequence
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (warp >= C.numSites) return;
-    const int a = warp;
     const SiteCells& G = A.cells;
-    const float4 pa = G.wrapped[a];
-    const int molA = __float_as_int(pa.w);
-    const float cut2 = C.listCutoff2 * (1.0f + 1e-4f);
-    const int cell = G.siteCell[a];
-    const int cx = cell % G.nc[0], cy = (cell / G.nc[0]) % G.nc[1], cz = cell / (G.nc[0] * G.nc[1]);
-    // lane k < 27 takes the cell (dx, dy, dz) = (k % 3, k / 3 % 3, k / 9) - 1, the order of three nested loops
-    int first = 0, n = 0;
-    if (lane < 27) {
-        const int x = (cx + lane % 3 - 1 + G.nc[0]) % G.nc[0], y = (cy + lane / 3 % 3 - 1 + G.nc[1]) % G.nc[1],
-                  z = (cz + lane / 9 - 1 + G.nc[2]) % G.nc[2];
-        const int c = (z * G.nc[1] + y) * G.nc[0] + x;
-        first = G.cellStart[c];
-        n = G.cellStart[c + 1] - first;
-    }
-    int end = n;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, end, o);
-        if (lane >= o) end += v;
-    }
-    const int total = __shfl_sync(0xffffffffu, end, 31);
-    cellFirst[w][lane] = first;
-    cellEnd[w][lane] = end;
-    __syncwarp();
-    int count = 0;
-    for (int k0 = 0; k0 < total; k0 += 32) {
-        const int k = k0 + lane;
-        int b = -1;
-        if (k < total) {
-            // the cell holding entry k: the first whose end exceeds k (binary search over the 27 ends)
-            int lo = 0, hi = 26;
-            while (lo < hi) {
-                const int mid = (lo + hi) >> 1;
-                if (cellEnd[w][mid] > k) hi = mid;
-                else lo = mid + 1;
+    for (int a = blockIdx.x * 8 + w; a < C.numSites; a += gridDim.x * 8) {
+        const float4 pa = G.wrapped[a];
+        const int molA = __float_as_int(pa.w);
+        const float cut2 = C.listCutoff2 * (1.0f + 1e-4f);
+        const int cell = G.siteCell[a];
+        const int cx = cell % G.nc[0], cy = (cell / G.nc[0]) % G.nc[1], cz = cell / (G.nc[0] * G.nc[1]);
+        // lane k < 27 takes the cell (dx, dy, dz) = (k % 3, k / 3 % 3, k / 9) - 1, the order of three nested loops
+        int first = 0, n = 0;
+        if (lane < 27) {
+            const int x = (cx + lane % 3 - 1 + G.nc[0]) % G.nc[0], y = (cy + lane / 3 % 3 - 1 + G.nc[1]) % G.nc[1],
+                      z = (cz + lane / 9 - 1 + G.nc[2]) % G.nc[2];
+            const int c = (z * G.nc[1] + y) * G.nc[0] + x;
+            first = G.cellStart[c];
+            n = G.cellStart[c + 1] - first;
+        }
+        int end = n;
+    #pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, end, o);
+            if (lane >= o) end += v;
+        }
+        const int total = __shfl_sync(0xffffffffu, end, 31);
+        cellFirst[w][lane] = first;
+        cellEnd[w][lane] = end;
+        __syncwarp();
+        int count = 0;
+        for (int k0 = 0; k0 < total; k0 += 32) {
+            const int k = k0 + lane;
+            int b = -1;
+            if (k < total) {
+                // the cell holding entry k: the first whose end exceeds k (binary search over the 27 ends)
+                int lo = 0, hi = 26;
+                while (lo < hi) {
+                    const int mid = (lo + hi) >> 1;
+                    if (cellEnd[w][mid] > k) hi = mid;
+                    else lo = mid + 1;
+                }
+                const int before = lo ? cellEnd[w][lo - 1] : 0;
+                b = G.cellSites[cellFirst[w][lo] + (k - before)];
             }
-            const int before = lo ? cellEnd[w][lo - 1] : 0;
-            b = G.cellSites[cellFirst[w][lo] + (k - before)];
+            bool near = false;
+            if (b >= 0 && siteAfter(G, 0, a, b)) {
+                const float4 pb = G.wrapped[b];
+                float dx = pb.x - pa.x, dy = pb.y - pa.y, dz = pb.z - pa.z;
+                dx -= C.boxf.a[0] * rintf(dx * C.boxf.inv[0]);
+                dy -= C.boxf.b[1] * rintf(dy * C.boxf.inv[1]);
+                dz -= C.boxf.c[2] * rintf(dz * C.boxf.inv[2]);
+                near = __float_as_int(pb.w) != molA && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < cut2;
+            }
+            const unsigned bal = __ballot_sync(0xffffffffu, near);
+            if (near) {
+                const int slot = count + __popc(bal & laneMaskLt());
+                if (slot < A.cap) A.nbr[(size_t)a * A.cap + slot] = b;
+            }
+            count += __popc(bal);
         }
-        bool near = false;
-        if (b >= 0 && siteAfter(G, 0, a, b)) {
-            const float4 pb = G.wrapped[b];
-            float dx = pb.x - pa.x, dy = pb.y - pa.y, dz = pb.z - pa.z;
-            dx -= C.boxf.a[0] * rintf(dx * C.boxf.inv[0]);
-            dy -= C.boxf.b[1] * rintf(dy * C.boxf.inv[1]);
-            dz -= C.boxf.c[2] * rintf(dz * C.boxf.inv[2]);
-            near = __float_as_int(pb.w) != molA && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < cut2;
+        if (lane == 0) {
+            A.nbrCount[a] = count;
+            if (count > A.cap) atomicOr(A.flag + 1, 1);
+            if (count > kAtmFastStaged || count > A.cap) atomicOr(A.flag + 2, 1);
+            if (a == 0) A.flag[3] = 0;
+            for (int d = 0; d < 3; d++) A.siteRef[3 * a + d] = A.sitePos[3 * a + d];
         }
-        const unsigned bal = __ballot_sync(0xffffffffu, near);
-        if (near) {
-            const int slot = count + __popc(bal & laneMaskLt());
-            if (slot < A.cap) A.nbr[(size_t)a * A.cap + slot] = b;
-        }
-        count += __popc(bal);
-    }
-    if (lane == 0) {
-        A.nbrCount[a] = count;
-        if (count > A.cap) atomicOr(A.flag + 1, 1);
-        if (count > kAtmFastStaged || count > A.cap) atomicOr(A.flag + 2, 1);
-        if (a == 0) A.flag[3] = 0;
-        for (int d = 0; d < 3; d++) A.siteRef[3 * a + d] = A.sitePos[3 * a + d];
+        __syncwarp();
     }
 }
 
@@ -624,8 +626,6 @@ __device__ __forceinline__ int stageTripleNeighborsScan(const AtmBuffers& A, con
 template <bool DAMP, bool IMAGE>
 __global__ void __launch_bounds__(32 * kAtmFastWarps, IX_TUNE_ATM_MIN_BLOCKS) kTriplesFast(AtmBuffers A, AtmConfig C) {
     __shared__ TripleStorage<DAMP, kAtmFastStaged> storage[kAtmFastWarps];
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < C.zeroSlots; k += gridDim.x * blockDim.x)
-        A.energyPartials[C.zeroOffset + k] = 0.0;
     auto& S = storage[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const int warp = blockIdx.x * kAtmFastWarps + (threadIdx.x >> 5);
@@ -727,15 +727,16 @@ __global__ void __launch_bounds__(32 * kAtmWarps) kTriplesWide(AtmBuffers A, Atm
     if (lane == 0 && visits) atomicAdd(A.tripleVisits, visits);
 }
 
-// The fast kernel, and the wide one where its grid is not empty.
+// The wide kernel where its grid is not empty, and the fast one.  The wide kernel mostly returns at once: it goes
+// first, while there is room on the SMs; behind the fast one it waited for the pair kernel's last blocks.
 template <bool DAMP, bool IMAGE>
 static void launchTriplesAs(const AtmBuffers& A, const AtmConfig& C, int fastBlocks, int wideBlocks, const int* gate,
                             cudaStream_t st) {
-    kTriplesFast<DAMP, IMAGE><<<fastBlocks, 32 * kAtmFastWarps, 0, st>>>(A, C);
     if (wideBlocks > 0)
         kTriplesWide<DAMP, IMAGE><<<wideBlocks, 32 * kAtmWarps,
                                     kAtmWarps * sizeof(TripleStorage<DAMP, kAtmMaxStaged>), st>>>(
             A, C, fastBlocks * kAtmFastWarps, gate);
+    kTriplesFast<DAMP, IMAGE><<<fastBlocks, 32 * kAtmFastWarps, 0, st>>>(A, C);
 }
 static void launchTriples(const AtmBuffers& A, const AtmConfig& C, int fastBlocks, int wideBlocks, const int* gate,
                           cudaStream_t st) {

@@ -220,7 +220,6 @@ struct ix_ctx {
     size_t uploadCap = 0, uploadUsed = 0;
     cudaStream_t stream = nullptr;
     cudaStream_t stream2 = nullptr;      // the three-body chain, forked from and joined back into `stream`
-    cudaStream_t streamBody = nullptr;   // captures the branches of conditional graph nodes
     cudaEvent_t evFork = nullptr, evJoin = nullptr;
     bool capturing = false;              // launches are being captured into a graph
     int numSMs = 148;
@@ -754,31 +753,6 @@ static int uploadPairParams(ix_ctx* ctx) {
     return IX_OK;
 }
 
-__global__ void kGatherParams(ListBuffers L, const float4* p0o, const float4* p1o, const float4* p2o,
-                              const float4* p3o, const int* flagso, float4* p0, float4* p1, float4* p2, float4* p3,
-                              int* flags) {
-    if (!rebuildRequested(L)) return;
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= L.np) return;
-    int i = L.sortedAtom[s];
-    if (i >= 0) {
-        p0[s] = p0o[i];
-        p1[s] = p1o[i];
-        p2[s] = p2o[i];
-        p3[s] = p3o[i];
-        flags[s] = flagso[i];
-    }
-    else {
-        p0[s] = make_float4(0, 0, 0, 0);
-        p1[s] = make_float4(0, 0, 0, 0);
-        p2[s] = make_float4(0, 0, 0, 0);
-        p3[s] = make_float4(0, 0, 0, 0);
-        flags[s] = 0;
-    }
-}
-
-__global__ void kClearFlag(int* flag) { *flag = 0; }
-
 // Estimated number of tiles of the list (the build reports overflows, and the host then grows the buffers).
 static long long estimateTiles(const ix_ctx* ctx, int nb) {
     if (ctx->method == IX_NO_CUTOFF) return (long long)nb * (nb + 1) / 2 + nb;
@@ -839,11 +813,25 @@ static int allocatePair(ix_ctx* ctx, long long tileCap) {
     IX_TRY(stageCopy(ctx, cellRank, rank.data(), numCells * sizeof(int)));
     L.cellRank = cellRank;
     IX_TRY(deviceAlloc(ctx, "cellKey", n, &L.cellKey));
-    IX_TRY(deviceAlloc(ctx, "cellCount", numCells, &L.cellCount));
-    IX_TRY(deviceAlloc(ctx, "cellStart", numCells + 1, &L.cellStart));
-    IX_TRY(deviceAlloc(ctx, "cellFill", numCells, &L.cellFill));
+    // read and written four cells at a time
+    IX_TRY(deviceAlloc(ctx, "cellCount", (numCells + 3) & ~3, &L.cellCount));
+    IX_TRY(deviceAlloc(ctx, "cellStart", (numCells + 3 & ~3) + 1, &L.cellStart));
+    IX_TRY(deviceAlloc(ctx, "cellArrival", n, &L.cellArrival));
+    IX_TRY(deviceAlloc(ctx, "listTicket", 1, &L.ticket));
+    // the counts and the ticket start at zero, the bounds at the ordered ints of +inf and -inf; each build leaves them so
+    IX_CUDA(ctx, cudaMemsetAsync(L.cellCount, 0, ((numCells + 3) & ~3) * sizeof(int), ctx->stream));
+    IX_CUDA(ctx, cudaMemsetAsync(L.ticket, 0, sizeof(unsigned), ctx->stream));
     IX_TRY(deviceAlloc(ctx, "order", n, &L.order));
     IX_TRY(deviceAlloc(ctx, "bboxMinMax", 8, &L.bboxMinMax));
+    {
+        int bounds[6];
+        for (int d = 0; d < 6; d++) {
+            const float v = d < 3 ? INFINITY : -INFINITY;
+            std::memcpy(&bounds[d], &v, sizeof(v));
+            if (bounds[d] < 0) bounds[d] ^= 0x7fffffff;
+        }
+        IX_TRY(stageCopy(ctx, L.bboxMinMax, bounds, sizeof(bounds)));
+    }
     IX_TRY(deviceAlloc(ctx, "refPos", 3 * (size_t)n, &L.refPos));
     IX_TRY(deviceAlloc(ctx, "sortedAtom", np, &L.sortedAtom));
     IX_TRY(deviceAlloc(ctx, "slotOf", n, &L.slotOf));
@@ -853,14 +841,17 @@ static int allocatePair(ix_ctx* ctx, long long tileCap) {
     IX_TRY(deviceAlloc(ctx, "bbox", 2 * (size_t)nb, &L.bbox));
     IX_TRY(deviceAlloc(ctx, "blockAtoms", nb, &L.blockAtoms));
     IX_TRY(deviceAlloc(ctx, "blockTiles", nb + 1, &L.blockTiles));
+    // an i-block of a liquid has some tens of candidate blocks in each share of its search
+    L.entryCap = G.useCutoff ? std::min((nb + 3) / 4 + 1, 96) : (nb + 3) / 4 + 1;
+    IX_TRY(deviceAlloc(ctx, "blockEntries", nb, &L.blockEntries));
+    IX_TRY(deviceAlloc(ctx, "entries", 4 * (size_t)nb * L.entryCap, &L.entries));
     if (tileCap > (long long)1 << 26) return fail(ctx, IX_ERR_INVALID, "neighbor list too large (%lld tiles)", tileCap);
     ctx->tileCap = (int)tileCap;
     L.tileCap = (int)tileCap;
     IX_TRY(deviceAlloc(ctx, "tileJ", 32 * (size_t)L.tileCap, &L.tileJ));
     IX_TRY(deviceAlloc(ctx, "tileIBlock", L.tileCap, &L.tileIBlock));
-    IX_TRY(deviceAlloc(ctx, "tileBucket", L.tileCap, &L.tileBucket));
-    IX_TRY(deviceAlloc(ctx, "tileOrder", L.tileCap, &L.tileOrder));
-    IX_TRY(deviceAlloc(ctx, "bucketCount", 33, &L.bucketCount));
+    IX_TRY(deviceAlloc(ctx, "bucketTiles", (size_t)kTileBuckets * L.tileCap, &L.bucketTiles));
+    IX_TRY(deviceAlloc(ctx, "bucketCount", kTileBuckets, &L.bucketCount));
     IX_TRY(deviceAlloc(ctx, "tileMask", 64 * (size_t)L.tileCap, &L.tileMask));
     IX_TRY(deviceAlloc(ctx, "numTiles", 1, &L.numTiles));
     IX_TRY(deviceAlloc(ctx, "taskCounter", 1, &L.taskCounter));
@@ -940,6 +931,25 @@ static void updateGeometry(ix_ctx* ctx) {
 // three-body setup
 // ---------------------------------------------------------------------------------------------------------------------
 
+// Resident blocks per SM of the fast triple kernel.  It runs beside the pair list and the pair kernel, whose persistent
+// grid fills what is left of each SM, so it gets its share of the two kernels' work, at least two blocks.  With as many
+// blocks as fit, the two ran one after the other: 103 + 19 us in an MD step of the 24,000-atom box, together 112 us now;
+// 371 + 159 us and 520 us for 96,000 atoms (0.8 nm; two to four blocks measure the same there).
+static int tripleBlocksPerSM(const ix_ctx* ctx) {
+    const int most = IX_TUNE_ATM_MIN_BLOCKS;
+    if (!ctx->pairShared) return most;
+    const double ns = (double)ctx->siteParams.size() / 3;
+    const double volume = ctx->atmPeriodic ? ctx->box[0] * ctx->box[4] * ctx->box[8] : 0.0;
+    auto neighbors = [&](double n, double cutoff) {      // half of those within the cutoff, of n at this density
+        return volume > 0.0 ? std::min(0.5 * n, n / volume * 2.0 / 3.0 * M_PI * cutoff * cutoff * cutoff) : 0.5 * n;
+    };
+    const double m = neighbors(ns, ctx->atmCutoff);
+    const double pairs = ctx->n * (ctx->method == IX_NO_CUTOFF ? 0.5 * ctx->n : neighbors(ctx->n, ctx->cutoff));
+    // issue slots: about 75 per 32 visits of a triple and 500 to stage a site, 550 per 32 pairs
+    const double triple = ns * (m * m * 75.0 / 32.0 + 500.0), pair = pairs * 550.0 / 32.0;
+    return std::min(most, std::max(2, (int)std::ceil(most * triple / (triple + pair))));
+}
+
 static int allocateAtm(ix_ctx* ctx) {
     const int ns = (int)ctx->siteParams.size() / 3;
     AtmBuffers& A = ctx->A;
@@ -1006,8 +1016,8 @@ static int allocateAtm(ix_ctx* ctx) {
     IX_TRY(deviceAlloc(ctx, "nbr", (size_t)ns * A.cap, &A.nbr));
     A.flag = ctx->dFlags + 4;
     A.numParticles = ctx->n;
-    // fast kernel: one warp per site; wide kernel (long lists): one wave of blocks over every (site, part) unit
-    ctx->atmFastBlocks = std::max(1, (ns + kAtmFastWarps - 1) / kAtmFastWarps);
+    // fast kernel: at most one warp per site; wide kernel (long lists): one wave of blocks over every (site, part) unit
+    ctx->atmFastBlocks = std::max(1, std::min((ns + kAtmFastWarps - 1) / kAtmFastWarps, tripleBlocksPerSM(ctx) * ctx->numSMs));
     ctx->atmGridBlocks = std::max(1, (int)std::min<long long>(((long long)ns * kAtmWideParts + kAtmWarps - 1) / kAtmWarps,
                                                               (long long)ctx->numSMs * 4));
     IX_TRY(deviceAlloc(ctx, "atmPartials", atmPartialCount(ctx), &ctx->dAtmPartials));
@@ -1090,6 +1100,7 @@ struct EnergyReduction {
     unsigned* ticket;
     unsigned long long* counts;
     int* taskCounter;
+    int *pairRebuild, *siteRebuild;      // rebuild flags to clear (null: none): every kernel that reads them has run
 };
 
 // One block (of `numBlocks`) of the energy reduction; 256 threads.
@@ -1146,6 +1157,8 @@ __device__ void reduceEnergiesBlock(const EnergyReduction& R, int block, int num
                 R.counts[1] = 0;
             }
             if (R.taskCounter) *R.taskCounter = 0;
+            if (R.pairRebuild) *R.pairRebuild = 0;
+            if (R.siteRebuild) *R.siteRebuild = 0;
         }
     }
 }
@@ -1154,7 +1167,7 @@ __global__ void kReduceEnergies(const double* pairPartials, const int* numPairPa
                                 const double* atmPartials, int numAtmWarps, double lrcEnergy, double* outEnergy,
                                 double* blockSums, unsigned* ticket, unsigned long long* counts, int* taskCounter) {
     const EnergyReduction R{pairPartials, numPairPartials, pairCap, atmPartials, numAtmWarps, lrcEnergy,
-                            outEnergy,    blockSums,       ticket,  counts,      taskCounter};
+                            outEnergy,    blockSums,       ticket,  counts,      taskCounter, nullptr, nullptr};
     reduceEnergiesBlock(R, blockIdx.x, gridDim.x);
 }
 
@@ -1307,10 +1320,6 @@ static PairTermConfig pairConfig(const ix_ctx* ctx, unsigned terms) {
 
 static int stageUploads(ix_ctx* ctx, unsigned terms);
 
-__global__ void kSetCondition(cudaGraphConditionalHandle handle, const int* flag) {
-    cudaGraphSetConditional(handle, *(volatile const int*)flag != 0 ? 1u : 0u);
-}
-
 // Profiling events: while capturing, external event-record nodes of the graph; launched directly, ordinary records.
 static void recordTiming(ix_ctx* ctx, int i, cudaStream_t s) {
     if (!ctx->profiling) return;
@@ -1320,57 +1329,6 @@ static void recordTiming(ix_ctx* ctx, int i, cudaStream_t s) {
 
 __global__ void kClearFlagIf(int* target, const int* gate) {
     if (*(volatile const int*)gate != 0) *target = 0;
-}
-
-// Launch `body` (a callable taking the stream to launch on) when *flag is set, else `orElse` (size 2) or nothing.
-// While the evaluation is being captured into a graph this is a conditional node whose branches are captured on the
-// context's third stream; the flag is read on the device each time the graph runs, so a step without a list rebuild
-// launches none of the rebuild kernels.  Launched directly, `body` runs, its kernels reading the flag themselves
-// (and `body` containing `orElse`'s work).  The launch counter keeps the kernels of the branch taken when the flag
-// is clear.
-template <class Body, class Else>
-static int launchConditional(ix_ctx* ctx, cudaStream_t st, const int* flag, Body body, Else orElse, int size) {
-    if (!ctx->capturing) return body(st);
-    cudaStreamCaptureStatus status;
-    cudaGraph_t graph = nullptr;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t numDeps = 0;
-    IX_CUDA(ctx, cudaStreamGetCaptureInfo(st, &status, nullptr, &graph, &deps, &numDeps));
-    cudaGraphConditionalHandle handle;
-    IX_CUDA(ctx, cudaGraphConditionalHandleCreate(&handle, graph, 0, cudaGraphCondAssignDefault));
-    kSetCondition<<<1, 1, 0, st>>>(handle, flag);
-    ctx->launches += 1;
-    IX_CUDA(ctx, cudaStreamGetCaptureInfo(st, &status, nullptr, &graph, &deps, &numDeps));
-    cudaGraphNodeParams params = {};
-    params.type = cudaGraphNodeTypeConditional;
-    params.conditional.handle = handle;
-    params.conditional.type = cudaGraphCondTypeIf;
-    params.conditional.size = (unsigned)size;
-    cudaGraphNode_t node;
-    IX_CUDA(ctx, cudaGraphAddNode(&node, graph, deps, numDeps, &params));
-    for (int k = 0; k < size; k++) {
-        IX_CUDA(ctx, cudaStreamBeginCaptureToGraph(ctx->streamBody, params.conditional.phGraph_out[k], nullptr,
-                                                   nullptr, 0, cudaStreamCaptureModeThreadLocal));
-        const long long before = ctx->launches;
-        const int rc = k == 0 ? body(ctx->streamBody) : orElse(ctx->streamBody);
-        cudaGraph_t captured = nullptr;
-        const cudaError_t e = cudaStreamEndCapture(ctx->streamBody, &captured);
-        if (k == 0) ctx->launches = before;
-        if (rc != IX_OK) return rc;
-        IX_CUDA(ctx, e);
-    }
-    IX_CUDA(ctx, cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies));
-    return IX_OK;
-}
-
-template <class Body>
-static int launchIf(ix_ctx* ctx, cudaStream_t st, const int* flag, Body body) {
-    return launchConditional(ctx, st, flag, body, body, 1);
-}
-
-template <class Body, class Else>
-static int launchIfElse(ix_ctx* ctx, cudaStream_t st, const int* flag, Body body, Else orElse) {
-    return launchConditional(ctx, st, flag, body, orElse, 2);
 }
 
 // Launch the whole evaluation on the context's stream.  Forces go to outForces (device, n x 3 doubles) and/or are
@@ -1435,22 +1393,22 @@ static int launchEvaluation(ix_ctx* ctx, unsigned terms, double* outForces, doub
                 }
         }
         kSiteCentroids<<<gS, 64, 0, sa>>>(A, C, ctx->dPos);
-        // site list rebuild when the centroid kernel set the flag: these kernels return at once otherwise (short
-        // launches cost less than a conditional graph node); the long-list flag is recomputed with the lists
-        kClearFlagIf<<<1, 1, 0, sa>>>(A.flag + 2, A.flag);
+        // site list rebuild when the centroid kernel set the flag: these kernels return at once otherwise.  The
+        // long-list flag is recomputed with the lists (the cell sort clears it)
         if (A.cells.nc[0]) {
             const int sharedSites = C.numSites <= kSiteSortSharedMax;
             kSiteCellSort<<<1, 1024, sharedSites ? C.numSites * sizeof(int) : 0, sa>>>(A, C, sharedSites);
-            kSiteNeighborsCells<<<(C.numSites * 32 + tpb - 1) / tpb, tpb, 0, sa>>>(A, C);
-            ctx->launches += 1;
+            kSiteNeighborsCells<<<std::min((C.numSites * 32 + tpb - 1) / tpb, ctx->numSMs * 2), tpb, 0, sa>>>(A, C);
         }
-        else kSiteNeighbors<<<(C.numSites * 32 + tpb - 1) / tpb, tpb, 0, sa>>>(A, C);
-        kClearFlag<<<1, 1, 0, sa>>>(A.flag);
+        else {
+            kClearFlagIf<<<1, 1, 0, sa>>>(A.flag + 2, A.flag);
+            kSiteNeighbors<<<(C.numSites * 32 + tpb - 1) / tpb, tpb, 0, sa>>>(A, C);
+        }
         recordTiming(ctx, 2, sa);
         // the sites whose lists are too long for the fast kernel go to the wide one, which returns at once when there
-        // are none
+        // are none and goes first
         launchTriples(A, C, ctx->atmFastBlocks, ctx->atmGridBlocks, A.flag + 2, sa);
-        ctx->launches += 6;
+        ctx->launches += 5;
         recordTiming(ctx, 3, sa);
         ctx->evAtm = ctx->profiling;
         IX_CUDA(ctx, cudaGetLastError());
@@ -1460,46 +1418,25 @@ static int launchEvaluation(ix_ctx* ctx, unsigned terms, double* outForces, doub
         ListBuffers& L = ctx->L;
         const int tpb = 256;
         const int gN = (n + tpb - 1) / tpb, gNp = (L.np + tpb - 1) / tpb;
-        const int gCells = (L.numCells + tpb - 1) / tpb;
         const bool stepStarted = kick != nullptr && kick->started;
         if (!stepStarted) {
-            kCheckDisplacement<<<gN, tpb, 0, st>>>(L, 0.25f * kPairSkin * kPairSkin);
+            // the displacement check and the current positions in the build frame
+            kRefreshPositions<<<gNp, tpb, 0, st>>>(L, 0.25f * kPairSkin * kPairSkin);
             ctx->launches += 1;
         }
-        // the current positions in the build frame, every step
-        auto refresh = [&](cudaStream_t s) {
-            kUpdateSortedPositions<<<gNp, tpb, 0, s>>>(L);
-            ctx->launches += 1;
-            return IX_OK;
-        };
-        // list rebuild (the displacement check set the flag): cell sort, then the tiles and their masks from the
-        // refreshed positions
-        auto rebuild = [&](cudaStream_t s) {
-            kResetCells<<<std::max(1, std::min(gCells, 1024)), tpb, 0, s>>>(L);
-            if (!ctx->G.periodic) kParticleBounds<<<gN, tpb, 0, s>>>(L);
-            kCellKeys<<<gN, tpb, 0, s>>>(L, ctx->G);
-            kScanCells<<<1, 1024, 0, s>>>(L);
-            kScatterCells<<<gN, tpb, 0, s>>>(L);
-            kSortWithinCells<<<gCells, tpb, 0, s>>>(L);
-            kSortedAtoms<<<gNp, tpb, 0, s>>>(L, ctx->G);
-            kGatherParams<<<gNp, tpb, 0, s>>>(L, ctx->dP0o, ctx->dP1o, ctx->dP2o, ctx->dP3o, ctx->dFlagso, ctx->dP0,
-                                              ctx->dP1, ctx->dP2, ctx->dP3, ctx->dFlagsSorted);
-            refresh(s);
-            kBlockBounds<<<(L.nb * 32 + tpb - 1) / tpb, tpb, 0, s>>>(L, ctx->G);
-            kListTiles<0><<<L.nb, kListThreads, 0, s>>>(L, ctx->G);
-            kScanTiles<<<1, 1024, 0, s>>>(L);
-            kListTiles<1><<<L.nb, kListThreads, 0, s>>>(L, ctx->G);
-            // grids no larger than the tiles need, so that a small system's launches leave the other SMs to the
-            // kernels of other streams
-            kTileMasks<<<std::min(ctx->numSMs * 8, std::max(1, (L.tileCap + kListWarps - 1) / kListWarps)), kListThreads,
-                         0, s>>>(L, ctx->G);
-            kTileOrder<<<std::min(ctx->numSMs, std::max(1, (L.tileCap + 255) / 256)), 256, 0, s>>>(L);
-            kClearFlag<<<1, 1, 0, s>>>(L.flag);
-            ctx->launches += ctx->G.periodic ? 14 : 15;
-            return IX_OK;
-        };
-        if (stepStarted) IX_TRY(launchIf(ctx, st, L.flag, rebuild));
-        else IX_TRY(launchIfElse(ctx, st, L.flag, rebuild, refresh));
+        // list rebuild (the displacement check or the host set the flag; else each kernel returns at once)
+        const SortedParams S{ctx->dP0o, ctx->dP1o, ctx->dP2o, ctx->dP3o, ctx->dFlagso, ctx->dP0,
+                             ctx->dP1,  ctx->dP2,  ctx->dP3,  ctx->dFlagsSorted};
+        if (!ctx->G.periodic) kParticleBounds<<<gN, tpb, 0, st>>>(L);
+        kCellKeys<<<(n + kCellThreads - 1) / kCellThreads, kCellThreads, 0, st>>>(L, ctx->G);
+        kScatterCells<<<gN, tpb, 0, st>>>(L);
+        kSortBlocks<<<gNp, tpb, 0, st>>>(L, ctx->G, S);
+        kListBlocks<<<(4 * L.nb + kListWarps - 1) / kListWarps, kListThreads, 0, st>>>(L, ctx->G);
+        // no more warps than tiles, and four blocks per SM at most: with eight the masks of 24,000 atoms take 37 us for
+        // 41, but a step without a rebuild waits 4.2 us for the blocks to return for 2.7
+        kTileMasks<<<std::min(ctx->numSMs * 4, std::max(1, (L.tileCap + kListWarps - 1) / kListWarps)),
+                     kListThreads, 0, st>>>(L, ctx->G);
+        ctx->launches += ctx->G.periodic ? 5 : 6;
         PairTermConfig C = pairConfig(ctx, terms);
         // the lean instantiation when no selected term has a soft core, a switching function or the order-2 overlap
         bool lean = true;
@@ -1567,7 +1504,8 @@ static int launchEvaluation(ix_ctx* ctx, unsigned terms, double* outForces, doub
     F.blocks = (n + 255) / 256;
     EnergyReduction R{doPair ? ctx->dPairPartials : nullptr, ctx->L.numTiles, ctx->L.tileCap,
                       doAtm ? ctx->dAtmPartials : nullptr, (int)atmPartialCount(ctx), lrcEnergy, outEnergy,
-                      ctx->dEnergyBlocks, ctx->dReduceTicket, ctx->dCounts, doPair ? ctx->L.taskCounter : nullptr};
+                      ctx->dEnergyBlocks, ctx->dReduceTicket, ctx->dCounts, doPair ? ctx->L.taskCounter : nullptr,
+                      doPair ? ctx->L.flag : nullptr, doAtm ? ctx->A.flag : nullptr};
     kFinish<<<F.blocks + kReduceBlocks, 256, 0, st>>>(F, R);
     ctx->launches += 1;
     IX_CUDA(ctx, cudaGetLastError());
@@ -1695,6 +1633,40 @@ static void releaseGraph(LaunchGraph& g) {
 // C ABI
 // ---------------------------------------------------------------------------------------------------------------------
 
+// The kernels that run beside one another on an SM ask for the same split of its memory between L1 and shared memory:
+// an SM changes the split only when it is empty, so a pair kernel's block did not start on it before the last triple
+// block had left (16 us of each step of the 24,000-atom box).
+static void sharedSplit() {
+    auto most = [](auto* kernel) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    };
+    most(kPairTiles<true, true, true>);
+    most(kPairTiles<true, false, true>);
+    most(kPairTiles<true, true, false>);
+    most(kPairTiles<true, false, false>);
+    most(kPairTiles<false, true, false>);
+    most(kPairTiles<false, false, false>);
+    most(kTriplesFast<false, false>);
+    most(kTriplesFast<false, true>);
+    most(kTriplesFast<true, false>);
+    most(kTriplesFast<true, true>);
+    most(kTriplesWide<false, false>);
+    most(kTriplesWide<false, true>);
+    most(kTriplesWide<true, false>);
+    most(kTriplesWide<true, true>);
+    most(kSiteCentroids);
+    most(kSiteNeighbors);
+    most(kSiteNeighborsCells);
+    most(kSiteCellSort);
+    most(kRefreshPositions);
+    most(kCellKeys);
+    most(kScatterCells);
+    most(kSortBlocks);
+    most(kListBlocks);
+    most(kTileMasks);
+    most(kFinish);
+}
+
 // The status block of a context (device, and a pinned host copy): flags (8 ints), term energies (4 doubles), counts
 // (4 unsigned long long).
 constexpr size_t kStatusBytes = 96;
@@ -1734,10 +1706,10 @@ static PinnedSlots& pinnedSlots() {
 static int ctxInitDevice(ix_ctx* ctx) {
     IX_CUDA(ctx, cudaSetDevice(ctx->device));
     IX_CUDA(ctx, cudaDeviceGetAttribute(&ctx->numSMs, cudaDevAttrMultiProcessorCount, ctx->device));
+    sharedSplit();
     // streams and events a server hands over from its pool are kept
     if ((!ctx->stream && cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess) ||
         (!ctx->stream2 && cudaStreamCreateWithFlags(&ctx->stream2, cudaStreamNonBlocking) != cudaSuccess) ||
-        (!ctx->streamBody && cudaStreamCreateWithFlags(&ctx->streamBody, cudaStreamNonBlocking) != cudaSuccess) ||
         (!ctx->evFork && cudaEventCreateWithFlags(&ctx->evFork, cudaEventDisableTiming) != cudaSuccess) ||
         (!ctx->evJoin && cudaEventCreateWithFlags(&ctx->evJoin, cudaEventDisableTiming) != cudaSuccess))
         return fail(ctx, IX_ERR_CUDA, "cudaStreamCreate failed");
@@ -1852,7 +1824,6 @@ void ix_ctx_destroy(ix_ctx* ctx) {
     if (ctx->evFork) cudaEventDestroy(ctx->evFork);
     if (ctx->evJoin) cudaEventDestroy(ctx->evJoin);
     if (ctx->stream2) cudaStreamDestroy(ctx->stream2);
-    if (ctx->streamBody) cudaStreamDestroy(ctx->streamBody);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
 }
@@ -2681,7 +2652,7 @@ static int softcoreWindows(ix_ctx* ctx, const std::string& name, int num_windows
         const double lrc = (D.present && (pairTerms & 1u) && D.lrcAlchCoef != 0) ? values[w] * D.lrcAlchCoef / volume
                                                                                  : 0.0;
         EnergyReduction R{dAlchEnergy, dAlchCount, std::max(numTasks, 1), nullptr, 0, lrc, dWinEnergy + 4 * (size_t)w,
-                          ctx->dEnergyBlocks, ctx->dReduceTicket, nullptr, ctx->L.taskCounter};
+                          ctx->dEnergyBlocks, ctx->dReduceTicket, nullptr, ctx->L.taskCounter, nullptr, nullptr};
         kFinish<<<F.blocks + kReduceBlocks, 256, 0, ctx->stream>>>(F, R);
         ctx->launches += numTasks ? 2 : 1;
         IX_CUDA(ctx, cudaGetLastError());

@@ -2,9 +2,15 @@
 // bounding boxes, and per i-block lists of "tiles" (one i-block x 32 candidate j particles within cutoff + skin of the
 // i-block's box).  Each tile carries its pair masks: bit j of row i is set when the pair (i, j) can interact before
 // the next rebuild (within cutoff + skin at build time, not excluded, j after i, some term gated on), and the
-// transposed column masks; the pair kernel visits only those pairs and needs no per-step candidate test.  Every
-// kernel of the build reads the rebuild flag and returns at once when it is clear, so the whole pipeline can be
-// launched every step (and captured in a CUDA graph) without a host round trip.
+// transposed column masks; the pair kernel visits only those pairs and needs no per-step candidate test.
+//
+// Every kernel of the build reads the rebuild flag and returns at once when it is clear, so the whole pipeline is
+// launched every step (and captured in a CUDA graph) without a host round trip.  The build is five kernels (six
+// without periodic boundaries), each as much as can be done before the next grid-wide dependency, with the scans in
+// the last block of the kernel that feeds them.  As a chain of fifteen kernels in the body of a conditional graph node
+// a step without a rebuild paid 9.5 us for the node (28 us where its other branch held the position refresh), and a
+// step with one waited 49 us for the body's first kernel and 115 us for the build (24,000 atoms); five launches that
+// return at once take 10 us beside the triple kernels, and the build takes 85 us.
 //
 // The reference gets its list from OpenMM (NonbondedUtilities, called at platforms/common/src/
 // CommonInteraxKernels.cpp:209) and, on the Reference platform, a voxel hash (ReferenceInteraxPairIxn.h:86-87).
@@ -48,8 +54,9 @@ struct ListBuffers {
     int* cellKey;               // n
     int* cellCount;             // numCells
     int* cellStart;             // numCells + 1
-    int* cellFill;              // numCells
-    int* order;                 // n: particles in cell order (within a cell by index after the per-cell sort)
+    int* cellArrival;           // n: place among its cell's particles, in the order the atomics took them
+    int* order;                 // n: particles in cell order (within a cell in order of arrival)
+    unsigned* ticket;           // blocks done, of the kernels whose last block scans (wraps to 0)
     const int* cellRank;        // dense cell index -> rank along the Hilbert curve
     int numCells;
     // sorted particles
@@ -60,14 +67,17 @@ struct ListBuffers {
     float4* sposf;              // np
     float4* bbox;               // nb x 2: center (xyz), half extent (xyz)
     // tiles
-    int* blockAtoms;            // nb: candidate j particles of each i-block
+    int4* blockAtoms;           // nb: candidate j particles of each i-block, in the four shares of its search
+    int4* blockEntries;         // nb: candidate blocks in each share
+    int4* entries;              // nb x 4 x entryCap: (block J, mask of its candidate particles, the share's candidates
+                                // before them)
+    int entryCap;               // per share
     int* blockTiles;            // nb + 1: exclusive scan of the tile counts, then the total
     int* tileJ;                 // tileCap x 32
     int* tileIBlock;            // tileCap
-    int* tileBucket;            // tileCap: each tile's candidate pairs / 32 (bits 0..5) and its rank in that bucket
-    int* bucketCount;           // 33: tiles per bucket
-    int* tileOrder;             // tileCap: the tiles by decreasing candidate count, the pair kernel's schedule (null:
-                                // list order), so that the last tiles the warps take are short
+    int* bucketCount;           // kTileBuckets: tiles by their number of candidate pairs (null: tileOrder)
+    int* bucketTiles;           // kTileBuckets x tileCap: the tiles of each bucket
+    int* tileOrder;             // numTiles: the tiles by decreasing candidate count (a batch's static list)
     unsigned* tileMask;         // tileCap x 64: row masks (per i lane, bit = j slot), then column masks (per j lane)
     int* numTiles;              // tiles to evaluate (0 after an overflow)
     int* taskCounter;           // next tile of the pair kernel's dynamic schedule (zeroed before each launch)
@@ -81,14 +91,29 @@ struct ListBuffers {
 
 __device__ __forceinline__ bool rebuildRequested(const ListBuffers& L) { return *(volatile int*)L.flag != 0; }
 
-// Displacement check: any particle moved more than half the skin since the last build sets the rebuild flag.
-__global__ void kCheckDisplacement(ListBuffers L, float maxMove2) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+// The pair kernel takes the tiles by decreasing number of candidate pairs, in steps of 64, so that the last tiles its
+// warps take are short.  The mask kernel appends each tile to its bucket; the order within a bucket follows the
+// atomics and varies from build to build, which changes no result: forces are summed in fixed point and energies go to
+// each tile's own slot.
+constexpr int kTileBuckets = 16;
+
+// Current positions in the build frame, and whether any particle moved more than half the skin since the last build,
+// which sets the rebuild flag (then, and where it is set already, the build writes the positions itself).  Padding
+// slots copy the last real particle's position, which keeps the blocks' boxes tight; they never interact.
+__global__ void kRefreshPositions(ListBuffers L, float maxMove2) {
+    if (rebuildRequested(L)) return;
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
     bool moved = false;
-    if (i < L.n) {
-        double dx = L.pos[3 * i] - L.refPos[3 * i];
-        double dy = L.pos[3 * i + 1] - L.refPos[3 * i + 1];
-        double dz = L.pos[3 * i + 2] - L.refPos[3 * i + 2];
+    if (s < L.np) {
+        const int src = s < L.n ? s : L.n - 1;
+        const int i = L.sortedAtom[src];
+        const double p[3] = {L.pos[3 * i], L.pos[3 * i + 1], L.pos[3 * i + 2]};
+        const double x = p[0] - L.shift[3 * src], y = p[1] - L.shift[3 * src + 1], z = p[2] - L.shift[3 * src + 2];
+        L.spos[3 * s] = x;
+        L.spos[3 * s + 1] = y;
+        L.spos[3 * s + 2] = z;
+        L.sposf[s] = make_float4((float)x, (float)y, (float)z, 0.0f);
+        const double dx = p[0] - L.refPos[3 * i], dy = p[1] - L.refPos[3 * i + 1], dz = p[2] - L.refPos[3 * i + 2];
         moved = (float)(dx * dx + dy * dy + dz * dz) > maxMove2;
     }
     if (__any_sync(0xffffffffu, moved) && (threadIdx.x & 31) == 0) atomicOr(L.flag, 1);
@@ -101,16 +126,47 @@ __device__ __forceinline__ int floatToOrdered(float f) {
 }
 __device__ __forceinline__ float orderedToFloat(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff); }
 
-__global__ void kResetCells(ListBuffers L) {
-    if (!rebuildRequested(L)) return;
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < L.numCells; c += gridDim.x * blockDim.x) {
-        L.cellCount[c] = 0;
-        L.cellFill[c] = 0;
+// Whether this block is the last of the grid to get here (all threads call it); the others' writes are then visible.
+__device__ __forceinline__ bool lastBlock(unsigned* ticket) {
+    __shared__ bool last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
     }
-    if (blockIdx.x == 0 && threadIdx.x < 6) {
-        int* mm = reinterpret_cast<int*>(L.bboxMinMax);
-        mm[threadIdx.x] = threadIdx.x < 3 ? floatToOrdered(INFINITY) : floatToOrdered(-INFINITY);
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
+}
+
+// Exclusive prefix of one value per thread over a block of T threads; `total` receives the sum.
+template <int T>
+__device__ __forceinline__ int blockPrefix(int v, int& total) {
+    __shared__ int warpSum[T / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
     }
+    if (lane == 31) warpSum[warp] = incl;
+    __syncthreads();
+    int before = 0;
+    total = 0;
+    for (int w = 0; w < T / 32; w++) {
+        before += w < warp ? warpSum[w] : 0;
+        total += warpSum[w];
+    }
+    __syncthreads();
+    return before + incl - v;
+}
+
+// Start values of the non-periodic bounding box.
+__device__ __forceinline__ void resetBounds(const ListBuffers& L) {
+    if (threadIdx.x < 6)
+        reinterpret_cast<int*>(L.bboxMinMax)[threadIdx.x] =
+            threadIdx.x < 3 ? floatToOrdered(INFINITY) : floatToOrdered(-INFINITY);
 }
 
 // Bounding box of all particles (non-periodic cell grids span it).
@@ -170,122 +226,67 @@ __device__ __forceinline__ int cellOf(const double w[3], const ListGeometry& G, 
     return (c[2] * G.nc[1] + c[1]) * G.nc[0] + c[0];
 }
 
-__global__ void kCellKeys(ListBuffers L, ListGeometry G) {
+// Cell of each particle, with its place among the cell's particles in the order of the atomics.  The last block scans
+// the counts into the cells' starts, and leaves the counts and the bounds as the next build needs them.
+constexpr int kCellThreads = 512;
+__global__ void __launch_bounds__(kCellThreads) kCellKeys(ListBuffers L, ListGeometry G) {
     if (!rebuildRequested(L)) return;
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= L.n) return;
-    double p[3] = {L.pos[3 * i], L.pos[3 * i + 1], L.pos[3 * i + 2]};
-    double w[3], s[3];
-    if (G.periodic) wrapIntoCell(p, G.box, w, s);
-    else {
-        for (int d = 0; d < 3; d++) w[d] = p[d];
+    const int t = threadIdx.x, i = blockIdx.x * kCellThreads + t;
+    if (i < L.n) {
+        double p[3] = {L.pos[3 * i], L.pos[3 * i + 1], L.pos[3 * i + 2]};
+        double w[3], s[3];
+        if (G.periodic) wrapIntoCell(p, G.box, w, s);
+        else {
+            for (int d = 0; d < 3; d++) w[d] = p[d];
+        }
+        const int key = L.cellRank[cellOf(w, G, L.bboxMinMax)];
+        L.cellKey[i] = key;
+        L.cellArrival[i] = atomicAdd(L.cellCount + key, 1);
     }
-    int key = L.cellRank[cellOf(w, G, L.bboxMinMax)];
-    L.cellKey[i] = key;
-    atomicAdd(L.cellCount + key, 1);
-}
-
-// Exclusive scan of the cell counts in one block of 1024 threads.
-__global__ void kScanCells(ListBuffers L) {
-    if (!rebuildRequested(L)) return;
-    __shared__ int partial[1024];
-    const int t = threadIdx.x;
-    const int per = (L.numCells + 1023) / 1024;
+    if (!lastBlock(L.ticket)) return;
+    // each thread a contiguous share of the cells, read four at a time (the arrays hold a multiple of four cells)
+    const int per = ((L.numCells + kCellThreads - 1) / kCellThreads + 3) & ~3;
     const int begin = min(t * per, L.numCells), end = min(begin + per, L.numCells);
+    int4* count = reinterpret_cast<int4*>(L.cellCount);
+    int4* start = reinterpret_cast<int4*>(L.cellStart);
     int sum = 0;
-    for (int c = begin; c < end; c++) sum += L.cellCount[c];
-    partial[t] = sum;
+    for (int c = begin; c < end; c += 4) {
+        const int4 v = __ldcg(count + (c >> 2));
+        sum += (v.x + v.y) + (v.z + v.w);
+    }
+    int total;
+    int run = blockPrefix<kCellThreads>(sum, total);
+    for (int c = begin; c < end; c += 4) {
+        const int4 v = __ldcg(count + (c >> 2));
+        count[c >> 2] = make_int4(0, 0, 0, 0);
+        start[c >> 2] = make_int4(run, run + v.x, run + v.x + v.y, run + v.x + v.y + v.z);
+        run += (v.x + v.y) + (v.z + v.w);
+    }
     __syncthreads();
-    for (int off = 1; off < 1024; off <<= 1) {
-        int v = t >= off ? partial[t - off] : 0;
-        __syncthreads();
-        partial[t] += v;
-        __syncthreads();
-    }
-    int run = partial[t] - sum;
-    for (int c = begin; c < end; c++) {
-        L.cellStart[c] = run;
-        run += L.cellCount[c];
-    }
-    if (t == 1023) L.cellStart[L.numCells] = partial[1023];
+    if (t == 0) L.cellStart[L.numCells] = total;
+    resetBounds(L);
 }
 
 __global__ void kScatterCells(ListBuffers L) {
     if (!rebuildRequested(L)) return;
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= L.n) return;
-    int key = L.cellKey[i];
-    int slot = L.cellStart[key] + atomicAdd(L.cellFill + key, 1);
-    L.order[slot] = i;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < L.n) L.order[L.cellStart[L.cellKey[i]] + L.cellArrival[i]] = i;
 }
 
-// Within each cell, order the particles by index, so that the sorted order does not depend on atomic timing.
-__global__ void kSortWithinCells(ListBuffers L) {
-    if (!rebuildRequested(L)) return;
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= L.numCells) return;
-    int b = L.cellStart[c], e = L.cellStart[c + 1];
-    for (int i = b + 1; i < e; i++) {
-        int v = L.order[i];
-        int j = i - 1;
-        while (j >= b && L.order[j] > v) {
-            L.order[j + 1] = L.order[j];
-            j--;
-        }
-        L.order[j + 1] = v;
-    }
-}
+// Per-particle arrays in original order and in sorted order.
+struct SortedParams {
+    const float4 *p0o, *p1o, *p2o, *p3o;
+    const int* flagso;
+    float4 *p0, *p1, *p2, *p3;
+    int* flags;
+};
 
-// Sorted particle data: original index, image shift that places the particle in the build frame, positions.
-__global__ void kSortedAtoms(ListBuffers L, ListGeometry G) {
-    if (!rebuildRequested(L)) return;
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= L.np) return;
-    if (s < L.n) {
-        int i = L.order[s];
-        L.sortedAtom[s] = i;
-        L.slotOf[i] = s;
-        double p[3] = {L.pos[3 * i], L.pos[3 * i + 1], L.pos[3 * i + 2]};
-        double w[3], sh[3] = {0, 0, 0};
-        if (G.periodic) wrapIntoCell(p, G.box, w, sh);
-        for (int d = 0; d < 3; d++) {
-            L.shift[3 * s + d] = sh[d];
-            L.refPos[3 * i + d] = p[d];
-        }
-    }
-    else {
-        L.sortedAtom[s] = -1;
-        for (int d = 0; d < 3; d++) L.shift[3 * s + d] = 0.0;
-    }
-}
-
-// Current positions in the build frame (every step, after a possible rebuild).  Padding slots copy the last real
-// particle's position, which keeps the blocks' boxes tight; they never interact.
-__global__ void kUpdateSortedPositions(ListBuffers L) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= L.np) return;
-    int src = s < L.n ? s : L.n - 1;
-    int i = L.sortedAtom[src];
-    double x = L.pos[3 * i] - L.shift[3 * src];
-    double y = L.pos[3 * i + 1] - L.shift[3 * src + 1];
-    double z = L.pos[3 * i + 2] - L.shift[3 * src + 2];
-    L.spos[3 * s] = x;
-    L.spos[3 * s + 1] = y;
-    L.spos[3 * s + 2] = z;
-    L.sposf[s] = make_float4((float)x, (float)y, (float)z, 0.0f);
-}
-
-// Bounding box of each block (one warp per block), from the build-time positions.
+// Bounding box of a block from the positions of its lanes.
 // The center's w is 1 when the block's tiles may place each j particle once, at its minimum image relative to the
 // block center, instead of taking the minimum image of every pair: that holds in a rectangular periodic box when
 // half of every box length exceeds the block's half extent plus the list cutoff plus the skin (room for the motion
 // between rebuilds), since then no interacting pair can need a different image.
-__global__ void kBlockBounds(ListBuffers L, ListGeometry G) {
-    if (!rebuildRequested(L)) return;
-    int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
-    if (warp >= L.nb) return;
-    float4 p = L.sposf[warp * 32 + lane];
+__device__ __forceinline__ void blockBounds(const ListBuffers& L, const ListGeometry& G, int block, int lane, float4 p) {
     float lo[3] = {warpMinF(p.x), warpMinF(p.y), warpMinF(p.z)};
     float hi[3] = {warpMaxF(p.x), warpMaxF(p.y), warpMaxF(p.z)};
     if (lane == 0) {
@@ -297,9 +298,68 @@ __global__ void kBlockBounds(ListBuffers L, ListGeometry G) {
             for (int d = 0; d < 3; d++) ok = ok && (half[d] + G.listCutoff + kPairSkin < 0.4999f * len[d]);
             shift = ok ? 1.0f : 0.0f;
         }
-        L.bbox[2 * warp] = make_float4(0.5f * (lo[0] + hi[0]), 0.5f * (lo[1] + hi[1]), 0.5f * (lo[2] + hi[2]), shift);
-        L.bbox[2 * warp + 1] = make_float4(half[0], half[1], half[2], 0.0f);
+        L.bbox[2 * block] = make_float4(0.5f * (lo[0] + hi[0]), 0.5f * (lo[1] + hi[1]), 0.5f * (lo[2] + hi[2]), shift);
+        L.bbox[2 * block + 1] = make_float4(half[0], half[1], half[2], 0.0f);
     }
+}
+
+// Block bounds from the current positions (batches, whose order never changes).
+__global__ void kBlockBounds(ListBuffers L, ListGeometry G) {
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (warp < L.nb) blockBounds(L, G, warp, lane, L.sposf[warp * 32 + lane]);
+}
+
+// The sorted particles, a warp per block of 32 slots: within each cell the particles by index, so that the order does
+// not depend on the atomics (slot k of a cell takes the particle that k others of the cell precede: a cell holds about
+// four), the image shift that places each in the build frame, its positions and parameters, and the block's box.
+__global__ void __launch_bounds__(256) kSortBlocks(ListBuffers L, ListGeometry G, SortedParams P) {
+    if (!rebuildRequested(L)) return;
+    const int lane = threadIdx.x & 31;
+    const int block = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (block >= L.nb) return;
+    const int s = block * 32 + lane, lastLane = min(31, L.n - 1 - block * 32);
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    double x[3] = {0.0, 0.0, 0.0};
+    int i = -1;
+    if (s < L.n) {
+        i = L.order[s];
+        const int key = L.cellKey[i], b = L.cellStart[key], e = L.cellStart[key + 1];
+        for (int a = b; a < e && e - b > 1; a++) {
+            const int v = L.order[a];
+            int before = 0;
+            for (int c = b; c < e; c++) before += L.order[c] < v;
+            if (before == s - b) {
+                i = v;
+                break;
+            }
+        }
+        L.slotOf[i] = s;
+        const double p[3] = {L.pos[3 * i], L.pos[3 * i + 1], L.pos[3 * i + 2]};
+        double w[3], sh[3] = {0, 0, 0};
+        if (G.periodic) wrapIntoCell(p, G.box, w, sh);
+        for (int d = 0; d < 3; d++) {
+            L.shift[3 * s + d] = sh[d];
+            L.refPos[3 * i + d] = p[d];
+            x[d] = p[d] - sh[d];
+        }
+    }
+    L.sortedAtom[s] = i;
+    for (int d = 0; d < 3; d++) {
+        const double last = __shfl_sync(0xffffffffu, x[d], lastLane);
+        if (i < 0) {
+            x[d] = last;
+            L.shift[3 * s + d] = 0.0;
+        }
+        L.spos[3 * s + d] = x[d];
+    }
+    const float4 f = make_float4((float)x[0], (float)x[1], (float)x[2], 0.0f);
+    L.sposf[s] = f;
+    P.p0[s] = i >= 0 ? P.p0o[i] : zero;
+    P.p1[s] = i >= 0 ? P.p1o[i] : zero;
+    P.p2[s] = i >= 0 ? P.p2o[i] : zero;
+    P.p3[s] = i >= 0 ? P.p3o[i] : zero;
+    P.flags[s] = i >= 0 ? P.flagso[i] : 0;
+    blockBounds(L, G, block, lane, f);
 }
 
 // Squared distance between the boxes of two blocks (rectangular minimum image when periodic); 0 if they overlap.
@@ -336,101 +396,200 @@ __device__ __forceinline__ bool isExcluded(const ListBuffers& L, int oi, int oj)
     return false;
 }
 
-constexpr int kListThreads = 256;                 // one thread block of 8 warps per i-block
+constexpr int kListThreads = 256;
 constexpr int kListWarps = kListThreads / 32;
 
-// Candidate j particles of one i-block (one thread block per i-block): the particles of the blocks J >= I whose box is
-// within the list cutoff of block I's box and whose own position is within it too, in the order (J, slot).  The blocks
-// are examined 256 at a time: each thread tests one block's box, the candidate blocks are compacted in block order, and
-// the warps take them round robin for the particle tests, so that the search of an i-block whose candidates crowd
-// into one index range is not serialised on one warp.  PASS 0 counts the candidates; PASS 1 writes their slots to the
-// i-block's tile rows and its tile headers.  Both passes make the same decisions, so the lists do not depend on
-// scheduling.
-template <int PASS>
-__global__ void __launch_bounds__(kListThreads) kListTiles(ListBuffers L, ListGeometry G) {
-    if (!rebuildRequested(L)) return;
-    __shared__ int candJ[kListThreads];
-    __shared__ unsigned keep[kListThreads];
-    __shared__ int offset[kListThreads];
-    __shared__ int warpTotal[kListWarps];
-    const int I = blockIdx.x;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+// The blocks an i-block pairs with are itself and the half of the others that follow it cyclically, so that every
+// i-block has about the same number of candidates (with the blocks J >= I the first had twice as many and the list
+// waited for it).  The number of those blocks, from I on:
+__device__ __forceinline__ int followingBlocks(int nb, int I) {
+    return nb / 2 + ((nb & 1) || I < nb / 2 ? 1 : 0);
+}
+
+// Share `part` of four of the candidate blocks of i-block I: every fourth block J that I pairs with, in cyclic order
+// (neighbors along the curve are neighbors in space, so contiguous shares would be uneven).  One warp; the boxes 32 at a
+// time (the next 32 loaded meanwhile), then the particles of the near blocks eight at a time, their loads and tests in
+// flight together.  group(J, mask): lane u < 8 holds the u-th of the eight blocks and its particles (mask) within the
+// list cutoff of block I's box (0: none, or no such block); until it returns false.
+template <class F>
+__device__ __forceinline__ void candidateBlocks(const ListBuffers& L, const ListGeometry& G, int I, int part, int lane,
+                                                F group) {
     const float4 ci = L.bbox[2 * I], ei = L.bbox[2 * I + 1];
     const float cut2 = G.useCutoff ? G.listCutoff * G.listCutoff : INFINITY;
-    int t0 = 0, t1 = 0;
-    if (PASS == 1) {
-        t0 = L.blockTiles[I];
-        t1 = L.blockTiles[I + 1];
-        if (t1 > L.tileCap) return;   // overflow: nothing is scheduled, the host grows the buffers and builds again
-    }
-    const long long base = 32LL * t0, last = 32LL * t1;
-    int count = 0;
-    for (int Jc = I; Jc < L.nb; Jc += kListThreads) {
-        // the candidate blocks of this chunk, in block order
-        const int J = Jc + tid;
-        const bool cand = J < L.nb && boxBoxDist2(ci, ei, L.bbox[2 * J], L.bbox[2 * J + 1], G) < cut2;
-        const unsigned b = __ballot_sync(0xffffffffu, cand);
-        if (lane == 0) warpTotal[warp] = __popc(b);
-        __syncthreads();
-        int before = 0, total = 0;
-        for (int w = 0; w < kListWarps; w++) {
-            const int c = warpTotal[w];
-            before += w < warp ? c : 0;
-            total += c;
-        }
-        if (cand) candJ[before + __popc(b & laneMaskLt())] = J;
-        __syncthreads();
-        // the particle tests of the candidate blocks
-        for (int k = warp; k < total; k += kListWarps) {
-            const int j = candJ[k] * 32 + lane;
-            bool in = L.sortedAtom[j] >= 0;
-            if (in && G.useCutoff) in = pointBoxDist2(L.sposf[j], ci, ei, G) < cut2;
-            const unsigned m = __ballot_sync(0xffffffffu, in);
-            if (lane == 0) keep[k] = m;
-        }
-        __syncthreads();
-        // offsets of the candidate blocks' particles: exclusive scan over the chunk
-        const int v = tid < total ? __popc(keep[tid]) : 0;
-        int incl = v;
+    const int follow = followingBlocks(L.nb, I);
+    auto blockAt = [&](int o) {
+        const int J = I + min(o, follow - 1);
+        return J < L.nb ? J : J - L.nb;
+    };
+    int J = blockAt(4 * lane + part);
+    float4 cj = L.bbox[2 * J], ej = L.bbox[2 * J + 1];
+    for (int o = part; o < follow; o += 128) {
+        const bool near = o + 4 * lane < follow && boxBoxDist2(ci, ei, cj, ej, G) < cut2;
+        unsigned todo = __ballot_sync(0xffffffffu, near);
+        J = blockAt(o + 128 + 4 * lane);
+        cj = L.bbox[2 * J];
+        ej = L.bbox[2 * J + 1];
+        while (todo) {
+            int Js[8];
+            float4 p[8];
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int u = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += u;
-        }
-        if (lane == 31) warpTotal[warp] = incl;
-        __syncthreads();
-        int wBefore = 0, chunkAtoms = 0;
-        for (int w = 0; w < kListWarps; w++) {
-            const int c = warpTotal[w];
-            wBefore += w < warp ? c : 0;
-            chunkAtoms += c;
-        }
-        if (tid < total) offset[tid] = count + wBefore + incl - v;
-        __syncthreads();
-        if (PASS == 1) {
-            for (int k = warp; k < total; k += kListWarps) {
-                const unsigned m = keep[k];
-                const long long pos = base + offset[k] + __popc(m & laneMaskLt());
-                if (((m >> lane) & 1u) && pos < last) L.tileJ[pos] = candJ[k] * 32 + lane;
+            for (int u = 0; u < 8; u++) {
+                Js[u] = todo ? blockAt(o + 4 * (__ffs(todo) - 1)) : -1;
+                todo &= todo - 1;
+                p[u] = L.sposf[32 * max(Js[u], 0) + lane];
             }
+            int myJ = -1;
+            unsigned mine = 0;
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const bool in = Js[u] >= 0 && 32 * Js[u] + lane < L.n &&
+                                (!G.useCutoff || pointBoxDist2(p[u], ci, ei, G) < cut2);
+                const unsigned m = __ballot_sync(0xffffffffu, in);
+                if (lane == u) {
+                    myJ = Js[u];
+                    mine = m;
+                }
+            }
+            if (!group(myJ, mine)) return;
         }
-        count += chunkAtoms;
-        __syncthreads();   // the shared arrays are refilled by the next chunk
-    }
-    if (PASS == 0) {
-        if (tid == 0) L.blockAtoms[I] = count;
-    }
-    else {
-        // tile headers: the i-block of each tile, padding (-1) after the last candidate of the last tile
-        for (int t = t0 + tid; t < t1; t += kListThreads) L.tileIBlock[t] = I;
-        const int rest = count & 31;
-        if (t1 > t0 && rest != 0 && tid >= rest && tid < 32) L.tileJ[last - 32 + tid] = -1;
     }
 }
 
-// Pair masks of the tiles, one warp per tile over the whole list (the tiles of an i-block vary in number, so a
-// per-i-block distribution would wait on the largest); lane = the tile's j lane, the i particles from shared memory.
-// A pair's bit is set when j's slot follows i's (each pair once), both are real particles gated on for a common term,
+// The candidates of each i-block, four warps per i-block, and in the last block the exclusive scan of the tile counts.
+// On overflow no tile is scheduled (nothing is written beyond the buffers); the host grows them and evaluates again.
+// Bound by latency: a warp's search is one chain of loads and tests.  A thread block per i-block with its candidates
+// shared among the warps through shared memory took 12.5 us for 24,000 atoms, and a second pass over the same
+// candidates to write the tiles another 15.6 (the mask kernel now finds its candidates from the entries); this takes
+// 24 us (41 with one warp per i-block), and half as many blocks return at once in a step without a rebuild.
+__global__ void __launch_bounds__(kListThreads) kListBlocks(ListBuffers L, ListGeometry G) {
+    if (!rebuildRequested(L)) return;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int unit = (blockIdx.x * kListThreads + tid) >> 5;
+    if (unit < 4 * L.nb) {
+        const int I = unit >> 2;
+        int atoms = 0, entries = 0;
+        candidateBlocks(L, G, I, unit & 3, lane, [&](int J, unsigned m) {
+            const unsigned have = __ballot_sync(0xffffffffu, m != 0);
+            int before = __popc(m);
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, before, o);
+                if (lane >= o) before += v;
+            }
+            const int at = entries + __popc(have & laneMaskLt());
+            if (m && at < L.entryCap)
+                L.entries[(size_t)unit * L.entryCap + at] = make_int4(J, (int)m, atoms + before - __popc(m), 0);
+            entries += __popc(have);
+            atoms += __shfl_sync(0xffffffffu, before, 7);
+            return true;
+        });
+        if (lane == 0) {
+            reinterpret_cast<int*>(L.blockAtoms)[unit] = atoms;
+            reinterpret_cast<int*>(L.blockEntries)[unit] = entries;
+        }
+    }
+    if (!lastBlock(L.ticket)) return;
+    auto tiles = [&](int c) {
+        const int4 a = __ldcg(L.blockAtoms + c);
+        return ((a.x + a.y) + (a.z + a.w) + 31) / 32;
+    };
+    const int per = (L.nb + kListThreads - 1) / kListThreads;
+    const int begin = min(tid * per, L.nb), end = min(begin + per, L.nb);
+    int sum = 0;
+    for (int c = begin; c < end; c++) sum += tiles(c);
+    int total;
+    int run = blockPrefix<kListThreads>(sum, total);
+    for (int c = begin; c < end; c++) {
+        L.blockTiles[c] = run;
+        run += tiles(c);
+    }
+    if (tid < kTileBuckets) L.bucketCount[tid] = 0;
+    if (tid == 0) {
+        L.blockTiles[L.nb] = total;
+        *L.numTiles = total > L.tileCap ? 0 : total;
+        if (total > L.tileCap) atomicOr(L.flag + 1, 1);
+    }
+}
+
+// The i-block of tile t: the last whose first tile is at or before t and that has tiles (a 32-way search by a warp).
+__device__ __forceinline__ int tileBlock(const ListBuffers& L, int t, int lane) {
+    int lo = 0, n = L.nb + 1;                        // blockTiles[lo] <= t < blockTiles[lo + n]
+    while (n > 1) {
+        const int step = (n + 31) / 32;
+        const int at = lo + lane * step;
+        const unsigned below = __ballot_sync(0xffffffffu, lane * step < n && L.blockTiles[at] <= t);
+        const int k = 31 - __clz(below);             // lane 0 always holds
+        lo += k * step;
+        n = min(step, n - k * step);
+    }
+    return lo;
+}
+
+// The candidates first .. first + 31 of i-block I to slots[0..31] (-1 after the last), by one warp: from the entries,
+// or by the search again where they did not fit (only in a box of very uneven density).
+__device__ __forceinline__ void tileCandidates(const ListBuffers& L, const ListGeometry& G, int I, int first, int lane,
+                                               int* slots) {
+    const unsigned lt = laneMaskLt();
+    slots[lane] = -1;
+    __syncwarp();
+    auto take = [&](int J, unsigned m, int at) {      // `at`: the place of the mask's first candidate in the tile
+        const int q = at + __popc(m & lt);
+        if (((m >> lane) & 1u) && q >= 0 && q < 32) slots[q] = 32 * J + lane;
+    };
+    const int4 n4 = L.blockEntries[I], a4 = L.blockAtoms[I];
+    const int counts[4] = {n4.x, n4.y, n4.z, n4.w}, atoms[4] = {a4.x, a4.y, a4.z, a4.w};
+    int base = 0;
+#pragma unroll
+    for (int part = 0; part < 4; part++) {
+        const int n = counts[part], lo = first - base;         // the tile's candidates among the share's: lo .. lo + 31
+        base += atoms[part];
+        if (lo <= -32 || lo >= atoms[part]) continue;
+        if (n <= L.entryCap) {
+            const int4* E = L.entries + (size_t)(4 * I + part) * L.entryCap;
+            for (int e0 = 0; e0 < n; e0 += 32) {
+                const int4 v = e0 + lane < n ? E[e0 + lane] : make_int4(0, 0, INT_MAX, 0);
+                const bool after = v.z >= lo + 32, mine = !after && v.z + __popc((unsigned)v.y) > lo;
+                for (unsigned b = __ballot_sync(0xffffffffu, mine); b; b &= b - 1) {
+                    const int k = __ffs(b) - 1;
+                    take(__shfl_sync(0xffffffffu, v.x, k), (unsigned)__shfl_sync(0xffffffffu, v.y, k),
+                         __shfl_sync(0xffffffffu, v.z, k) - lo);
+                }
+                if (__any_sync(0xffffffffu, after)) break;
+            }
+        }
+        else {
+            int before = 0;
+            candidateBlocks(L, G, I, part, lane, [&](int J, unsigned m) {
+                for (int u = 0; u < 8; u++) {
+                    const unsigned mu = __shfl_sync(0xffffffffu, m, u);
+                    take(__shfl_sync(0xffffffffu, J, u), mu, before - lo);
+                    before += __popc(mu);
+                }
+                return before < lo + 32;
+            });
+        }
+    }
+    __syncwarp();
+}
+
+// The 32 x 32 bit matrix whose row r is lane r's word, transposed (lane c receives bit r = bit c of lane r's word):
+// the off-diagonal blocks of 16, 8, 4, 2 and 1 exchanged between lane pairs.
+__device__ __forceinline__ unsigned transposeBits(unsigned x, int lane) {
+    const unsigned masks[5] = {0x0000ffffu, 0x00ff00ffu, 0x0f0f0f0fu, 0x33333333u, 0x55555555u};
+#pragma unroll
+    for (int k = 0; k < 5; k++) {
+        const int s = 16 >> k;
+        const unsigned m = masks[k];
+        const unsigned y = __shfl_xor_sync(0xffffffffu, x, s);
+        x = (lane & s) ? ((x & ~m) | ((y & ~m) >> s)) : ((x & m) | ((y & m) << s));
+    }
+    return x;
+}
+
+// The tiles, one warp per tile over the whole list (the tiles of an i-block vary in number, so a per-i-block
+// distribution would wait on the largest): its i-block and candidate j particles, and its pair masks; lane = the tile's
+// j lane, the i particles from shared memory.
+// A pair's bit is set when j is of another block or its slot follows i's (each pair once), both are real particles gated on for a common term,
 // the pair is not excluded and its build-time distance (minimum image) is within the list cutoff: then no pair outside
 // the masks can come within the cutoff before the displacement check requests the next build.  The tests that do not
 // depend on the distance are masks formed once per tile; where the i-block allows it (rectangular box, block small
@@ -440,13 +599,18 @@ __global__ void __launch_bounds__(kListThreads) kListTiles(ListBuffers L, ListGe
 __global__ void __launch_bounds__(kListThreads) kTileMasks(ListBuffers L, ListGeometry G) {
     if (!rebuildRequested(L)) return;
     __shared__ float4 ipos[kListWarps][32];   // xyz and the original index (as its bits)
+    __shared__ int slots[kListWarps][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // the margin covers the float rounding of the build-time distance
     const float cut2 = G.useCutoff ? G.listCutoff * G.listCutoff * (1.0f + 1e-5f) : INFINITY;
     const int numTiles = *L.numTiles;
     const int warps = (gridDim.x * blockDim.x) >> 5;
     for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < numTiles; t += warps) {
-        const int I = L.tileIBlock[t];
+        const int I = tileBlock(L, t, lane);
+        tileCandidates(L, G, I, 32 * (t - L.blockTiles[I]), lane, slots[warp]);
+        const int sj = slots[warp][lane];
+        L.tileJ[32LL * t + lane] = sj;
+        if (lane == 0) L.tileIBlock[t] = I;
         const int si = I * 32 + lane;
         const int oi = L.sortedAtom[si];
         const int fi = L.flags[si];
@@ -459,7 +623,6 @@ __global__ void __launch_bounds__(kListThreads) kTileMasks(ListBuffers L, ListGe
         const unsigned gateD = __ballot_sync(0xffffffffu, (fi & kFlagGateDisp) != 0);
         const unsigned gateE = __ballot_sync(0xffffffffu, (fi & kFlagGateExch) != 0);
         const unsigned gateS = __ballot_sync(0xffffffffu, (fi & kFlagGateSr) != 0);
-        const int sj = L.tileJ[32LL * t + lane];
         int oj = -1, fj = 0;
         float4 pj = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         int2 jr = make_int2(1, 0);
@@ -473,107 +636,51 @@ __global__ void __launch_bounds__(kListThreads) kTileMasks(ListBuffers L, ListGe
         if (oj >= 0) {
             column = iReal & (((fj & kFlagGateDisp) ? gateD : 0u) | ((fj & kFlagGateExch) ? gateE : 0u) |
                               ((fj & kFlagGateSr) ? gateS : 0u));
-            const int d = sj - I * 32;   // the i slots of the block below j's
-            column &= d >= 32 ? 0xffffffffu : (d <= 0 ? 0u : (1u << d) - 1u);
+            const int d = sj - I * 32;   // within the i-block itself, the i slots below j's
+            if (d >= 0 && d < 32) column &= (1u << d) - 1u;
         }
-        if (G.useCutoff && __any_sync(0xffffffffu, column != 0)) {
-            bool perPair = G.periodic;
-            const float4 c = L.bbox[2 * I];
-            if (G.periodic && c.w != 0.0f) {
-                pj.x -= G.boxf.a[0] * rintf((pj.x - c.x) * G.boxf.inv[0]);
-                pj.y -= G.boxf.b[1] * rintf((pj.y - c.y) * G.boxf.inv[1]);
-                pj.z -= G.boxf.c[2] * rintf((pj.z - c.z) * G.boxf.inv[2]);
-                perPair = false;
-            }
-            unsigned in = 0;
-#pragma unroll
+        // the pairs within the list cutoff, and those whose i lies in j's exclusion range, which are looked up
+        unsigned in = 0, suspect = 0;
+        const unsigned span = jr.x <= jr.y ? (unsigned)(jr.y - jr.x) : 0u;
+        const int low = jr.x <= jr.y ? jr.x : INT_MIN;          // no index is that low
+        const float4 c = L.bbox[2 * I];
+        if (G.periodic && c.w == 0.0f && G.useCutoff) {
+#pragma unroll 4
             for (int i = 0; i < 32; i++) {
                 const float4 q = ipos[warp][i];
                 float dx = pj.x - q.x, dy = pj.y - q.y, dz = pj.z - q.z;
-                if (perPair) minimumImageF(dx, dy, dz, G.boxf);
+                minimumImageF(dx, dy, dz, G.boxf);
                 if (fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < cut2) in |= 1u << i;
-            }
-            column &= in;
-        }
-        if (jr.x <= jr.y) {
-            for (unsigned m = column; m; m &= m - 1) {
-                const int i = __ffs(m) - 1;
-                const int o = __float_as_int(ipos[warp][i].w);
-                if (o >= jr.x && o <= jr.y && isExcluded(L, oj, o)) column &= ~(1u << i);
+                if ((unsigned)(__float_as_int(q.w) - low) <= span) suspect |= 1u << i;
             }
         }
-        unsigned row = 0;
-        for (int i = 0; i < 32; i++) {
-            const unsigned bits = __ballot_sync(0xffffffffu, (column >> i) & 1u);
-            if (lane == i) row = bits;
+        else {
+            if (G.periodic) {
+                pj.x -= G.boxf.a[0] * rintf((pj.x - c.x) * G.boxf.inv[0]);
+                pj.y -= G.boxf.b[1] * rintf((pj.y - c.y) * G.boxf.inv[1]);
+                pj.z -= G.boxf.c[2] * rintf((pj.z - c.z) * G.boxf.inv[2]);
+            }
+#pragma unroll
+            for (int i = 0; i < 32; i++) {
+                const float4 q = ipos[warp][i];
+                const float dx = pj.x - q.x, dy = pj.y - q.y, dz = pj.z - q.z;
+                if (fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < cut2) in |= 1u << i;
+                if ((unsigned)(__float_as_int(q.w) - low) <= span) suspect |= 1u << i;
+            }
         }
+        if (G.useCutoff) column &= in;
+        for (suspect &= column; suspect; suspect &= suspect - 1) {
+            const int i = __ffs(suspect) - 1;
+            if (isExcluded(L, oj, __float_as_int(ipos[warp][i].w))) column &= ~(1u << i);
+        }
+        const unsigned row = transposeBits(column, lane);
         L.tileMask[64LL * t + lane] = row;
         L.tileMask[64LL * t + 32 + lane] = column;
         const unsigned pairs = __reduce_add_sync(0xffffffffu, (unsigned)__popc(column));
-        if (lane == 0 && L.tileBucket) {
-            const int b = (int)(pairs >> 5);
-            L.tileBucket[t] = (int)((unsigned)b | ((unsigned)atomicAdd(L.bucketCount + b, 1) << 6));
+        if (lane == 0) {
+            const int b = min((int)(pairs >> 6), kTileBuckets - 1);
+            L.bucketTiles[(size_t)b * L.tileCap + atomicAdd(L.bucketCount + b, 1)] = t;
         }
-    }
-}
-
-// The pair kernel's schedule: the tiles by decreasing candidate count (a counting sort over 33 buckets of 32 pairs:
-// the mask kernel counted each bucket and gave each tile its rank in it; here each tile goes to its bucket's start plus
-// its rank).  The warps take tiles from a shared counter, so the kernel ends when the last tile taken ends; short tiles
-// last keep that tail short.  The order within a bucket follows the atomics and varies from build to build, which
-// changes no result: forces are summed in fixed point and energies go to each tile's own slot.
-__global__ void kTileOrder(ListBuffers L) {
-    if (!rebuildRequested(L)) return;
-    __shared__ int start[33];
-    if (threadIdx.x == 0) {
-        int run = 0;
-        for (int b = 32; b >= 0; b--) {
-            start[b] = run;
-            run += L.bucketCount[b];
-        }
-    }
-    __syncthreads();
-    const int n = *L.numTiles;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        const unsigned v = (unsigned)L.tileBucket[t];
-        L.tileOrder[start[v & 63u] + (int)(v >> 6)] = t;
-    }
-}
-
-// The exclusive scan of the i-blocks' tile counts (one block of 1024 threads).  On overflow no tile is scheduled
-// (nothing is written beyond the buffers); the host grows them and evaluates again.
-__global__ void kScanTiles(ListBuffers L) {
-    if (!rebuildRequested(L)) return;
-    __shared__ int partial[1024];
-    const int t = threadIdx.x;
-    const int per = (L.nb + 1023) / 1024;
-    const int begin = min(t * per, L.nb), end = min(begin + per, L.nb);
-    int sum = 0;
-    for (int c = begin; c < end; c++) {
-        const int tiles = (L.blockAtoms[c] + 31) / 32;
-        L.blockTiles[c] = tiles;
-        sum += tiles;
-    }
-    partial[t] = sum;
-    __syncthreads();
-    for (int off = 1; off < 1024; off <<= 1) {
-        const int v = t >= off ? partial[t - off] : 0;
-        __syncthreads();
-        partial[t] += v;
-        __syncthreads();
-    }
-    int run = partial[t] - sum;
-    for (int c = begin; c < end; c++) {
-        const int k = L.blockTiles[c];
-        L.blockTiles[c] = run;
-        run += k;
-    }
-    if (t < 33 && L.bucketCount) L.bucketCount[t] = 0;   // for the mask kernel's tile counts
-    if (t == 1023) {
-        const int total = partial[1023];
-        L.blockTiles[L.nb] = total;
-        *L.numTiles = total > L.tileCap ? 0 : total;
-        if (total > L.tileCap) atomicOr(L.flag + 1, 1);
     }
 }
 

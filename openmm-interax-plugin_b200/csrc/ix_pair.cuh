@@ -347,20 +347,6 @@ __device__ __forceinline__ bool pairInside(const float4& hi_i, const float4& lo_
     return withinCutoff(r2, hi_i, lo_i, hi_j, lo_j, perPairImage, C);
 }
 
-// The 32 x 32 bit matrix whose row r is lane r's word, transposed (lane c receives bit r = bit c of lane r's word):
-// the off-diagonal blocks of 16, 8, 4, 2 and 1 exchanged between lane pairs.
-__device__ __forceinline__ unsigned transposeBits(unsigned x, int lane) {
-    const unsigned masks[5] = {0x0000ffffu, 0x00ff00ffu, 0x0f0f0f0fu, 0x33333333u, 0x55555555u};
-#pragma unroll
-    for (int k = 0; k < 5; k++) {
-        const int s = 16 >> k;
-        const unsigned m = masks[k];
-        const unsigned y = __shfl_xor_sync(0xffffffffu, x, s);
-        x = (lane & s) ? ((x & ~m) | ((y & ~m) >> s)) : ((x & m) | ((y & m) << s));
-    }
-    return x;
-}
-
 // One queued pair: displacement, the cutoff test (CHECK: the queue holds candidates; else the pairs were filtered
 // when queued), the terms.  Returns the force on i (zero outside the cutoff) and counts the pair if it interacts.
 template <bool LEAN, bool TABLE, bool UNIFORM, bool CHECK>
@@ -491,6 +477,16 @@ __global__ void __launch_bounds__(32 * kPairWarps, IX_TUNE_PAIR_MIN_BLOCKS) kPai
         coef = reinterpret_cast<const PairCoef*>(pairShared);
     }
     const int numTasks = P.taskTiles ? P.numTasks : min(*L.numTiles, L.tileCap);
+    // the schedule: the buckets from the fullest tiles down, lane b the end of its bucket in the sequence of tasks
+    int bucketEnd = 0;
+    if (L.bucketCount) {
+        bucketEnd = lane < kTileBuckets ? L.bucketCount[kTileBuckets - 1 - lane] : 0;
+#pragma unroll
+        for (int o = 1; o < kTileBuckets; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, bucketEnd, o);
+            if (lane >= o) bucketEnd += v;
+        }
+    }
     const unsigned ltMask = laneMaskLt();
     unsigned long long pairs = 0;
     for (;;) {
@@ -498,7 +494,14 @@ __global__ void __launch_bounds__(32 * kPairWarps, IX_TUNE_PAIR_MIN_BLOCKS) kPai
         if (lane == 0) task = atomicAdd(L.taskCounter, 1);
         task = __shfl_sync(0xffffffffu, task, 0);
         if (task >= numTasks) break;
-        const int t = P.taskTiles ? P.taskTiles[task] : (L.tileOrder ? L.tileOrder[task] : task);
+        int t;
+        if (P.taskTiles) t = P.taskTiles[task];
+        else if (L.bucketCount) {
+            const int b = __ffs(__ballot_sync(0xffffffffu, task < bucketEnd)) - 1;
+            const int before = __shfl_sync(0xffffffffu, bucketEnd, max(b - 1, 0));
+            t = L.bucketTiles[(size_t)(kTileBuckets - 1 - b) * L.tileCap + (task - (b > 0 ? before : 0))];
+        }
+        else t = L.tileOrder[task];
         const int I = L.tileIBlock[t];
         const int iBase = I * 32;
         const float4 center = L.bbox[2 * I];

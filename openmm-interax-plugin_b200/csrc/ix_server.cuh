@@ -110,7 +110,7 @@ struct ServerUnit {
 
 // A context's streams and events, kept for the next context of the shard.
 struct StreamSet {
-    cudaStream_t stream = nullptr, stream2 = nullptr, body = nullptr;
+    cudaStream_t stream = nullptr, stream2 = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
 };
 
@@ -354,12 +354,11 @@ void retireContext(ix_server* S, ServerShard* H, ix_ctx* c) {
     StreamSet set;
     set.stream = c->stream;
     set.stream2 = c->stream2;
-    set.body = c->streamBody;
     set.fork = c->evFork;
     set.join = c->evJoin;
-    if (set.stream && set.stream2 && set.body && set.fork && set.join) {
+    if (set.stream && set.stream2 && set.fork && set.join) {
         H->streams.push_back(set);
-        c->stream = c->stream2 = c->streamBody = nullptr;
+        c->stream = c->stream2 = nullptr;
         c->evFork = c->evJoin = nullptr;
     }
     {
@@ -503,7 +502,6 @@ void launchContext(ix_server* S, ServerShard* H, ServerRequest* r) {
         H->streams.pop_back();
         c->stream = set.stream;
         c->stream2 = set.stream2;
-        c->streamBody = set.body;
         c->evFork = set.fork;
         c->evJoin = set.join;
     }
@@ -949,7 +947,6 @@ void shardLoop(ix_server* S, ServerShard* H) {
     for (const StreamSet& set : H->streams) {
         cudaStreamDestroy(set.stream);
         cudaStreamDestroy(set.stream2);
-        cudaStreamDestroy(set.body);
         cudaEventDestroy(set.fork);
         cudaEventDestroy(set.join);
     }
@@ -1055,7 +1052,6 @@ int ix_server_create(int device, double budget_bytes, int max_running, int threa
             StreamSet set;
             if (cudaStreamCreateWithFlags(&set.stream, cudaStreamNonBlocking) != cudaSuccess ||
                 cudaStreamCreateWithFlags(&set.stream2, cudaStreamNonBlocking) != cudaSuccess ||
-                cudaStreamCreateWithFlags(&set.body, cudaStreamNonBlocking) != cudaSuccess ||
                 cudaEventCreateWithFlags(&set.fork, cudaEventDisableTiming) != cudaSuccess ||
                 cudaEventCreateWithFlags(&set.join, cudaEventDisableTiming) != cudaSuccess) {
                 cudaGetLastError();
