@@ -80,6 +80,7 @@ struct ListBuffers {
     int* tileOrder;             // numTiles: the tiles by decreasing candidate count (a batch's static list)
     unsigned* tileMask;         // tileCap x 64: row masks (per i lane, bit = j slot), then column masks (per j lane)
     int* numTiles;              // tiles to evaluate (0 after an overflow)
+    int splitShift;             // each tile of 32 x 32 candidates is listed as 2^splitShift tiles of a share of its rows
     int* taskCounter;           // next tile of the pair kernel's dynamic schedule (zeroed before each launch)
     int tileCap;
     const int* flags;           // sorted particle flags (the term gates of each particle)
@@ -506,12 +507,13 @@ __global__ void __launch_bounds__(kListThreads) kListBlocks(ListBuffers L, ListG
     if (tid < kTileBuckets) L.bucketCount[tid] = 0;
     if (tid == 0) {
         L.blockTiles[L.nb] = total;
-        *L.numTiles = total > L.tileCap ? 0 : total;
-        if (total > L.tileCap) atomicOr(L.flag + 1, 1);
+        const bool fits = (long long)total << L.splitShift <= L.tileCap;
+        *L.numTiles = fits ? total << L.splitShift : 0;
+        if (!fits) atomicOr(L.flag + 1, 1);
     }
 }
 
-// The i-block of tile t: the last whose first tile is at or before t and that has tiles (a 32-way search by a warp).
+// The i-block of tile t (before the split): the last whose first tile is at or before t and that has tiles (a 32-way search by a warp).
 __device__ __forceinline__ int tileBlock(const ListBuffers& L, int t, int lane) {
     int lo = 0, n = L.nb + 1;                        // blockTiles[lo] <= t < blockTiles[lo + n]
     while (n > 1) {
@@ -603,14 +605,12 @@ __global__ void __launch_bounds__(kListThreads) kTileMasks(ListBuffers L, ListGe
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // the margin covers the float rounding of the build-time distance
     const float cut2 = G.useCutoff ? G.listCutoff * G.listCutoff * (1.0f + 1e-5f) : INFINITY;
-    const int numTiles = *L.numTiles;
+    const int numTiles = *L.numTiles >> L.splitShift;
     const int warps = (gridDim.x * blockDim.x) >> 5;
     for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < numTiles; t += warps) {
         const int I = tileBlock(L, t, lane);
         tileCandidates(L, G, I, 32 * (t - L.blockTiles[I]), lane, slots[warp]);
         const int sj = slots[warp][lane];
-        L.tileJ[32LL * t + lane] = sj;
-        if (lane == 0) L.tileIBlock[t] = I;
         const int si = I * 32 + lane;
         const int oi = L.sortedAtom[si];
         const int fi = L.flags[si];
@@ -674,12 +674,21 @@ __global__ void __launch_bounds__(kListThreads) kTileMasks(ListBuffers L, ListGe
             if (isExcluded(L, oj, __float_as_int(ipos[warp][i].w))) column &= ~(1u << i);
         }
         const unsigned row = transposeBits(column, lane);
-        L.tileMask[64LL * t + lane] = row;
-        L.tileMask[64LL * t + 32 + lane] = column;
-        const unsigned pairs = __reduce_add_sync(0xffffffffu, (unsigned)__popc(column));
-        if (lane == 0) {
-            const int b = min((int)(pairs >> 6), kTileBuckets - 1);
-            L.bucketTiles[(size_t)b * L.tileCap + atomicAdd(L.bucketCount + b, 1)] = t;
+        // listed whole, or as tiles that take a share of the rows each
+        const int rows = 32 >> L.splitShift;
+        for (int part = 0; part < 1 << L.splitShift; part++) {
+            const size_t out = ((size_t)t << L.splitShift) + part;
+            const unsigned mine = (0xffffffffu >> (32 - rows)) << (part * rows);
+            const unsigned some = column & mine;
+            L.tileJ[32 * out + lane] = sj;
+            L.tileMask[64 * out + lane] = (mine >> lane) & 1u ? row : 0u;
+            L.tileMask[64 * out + 32 + lane] = some;
+            const unsigned pairs = __reduce_add_sync(0xffffffffu, (unsigned)__popc(some));
+            if (lane == 0) {
+                L.tileIBlock[out] = I;
+                const int b = min((int)(pairs >> 6), kTileBuckets - 1);
+                L.bucketTiles[(size_t)b * L.tileCap + atomicAdd(L.bucketCount + b, 1)] = (int)out;
+            }
         }
     }
 }

@@ -88,6 +88,28 @@ def test_sizes_and_boundaries(n, kind):
         x = x + rng.uniform(-1, 1, size=(n, 3)) * (0.004 if step == 0 else 0.02) + (0.0 if step == 0 else 0.1)
 
 
+@pytest.mark.parametrize("n", [2304, 2305, 8192, 8193])
+def test_sizes_where_the_tiles_split_changes(n):
+    rng = np.random.default_rng(n)
+    side = int(np.ceil(n ** (1 / 3)))
+    box = np.eye(3) * side * 0.28
+    x = np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n] * 0.28
+    x = x + rng.uniform(-0.07, 0.07, size=x.shape)
+    system = _system(n, InteraxDispersionForce.CutoffPeriodic, 0.9, box)
+    ctx = Context(system)
+    ctx.setPositions(x)
+    state = ctx.getState()
+    e, f = pyoracle.evaluate(system, x, box)
+    e_err, f_err = errors(state.getPotentialEnergy(), state.getForces(), e, f)
+    assert e_err <= ENERGY_TOL and f_err <= FORCE_RMS_TOL, (e_err, f_err)
+    small = Context(system)
+    small.setListCapacity(16, 0)                                      # grown after an overflow: the same sums
+    small.setPositions(x)
+    again = small.getState()
+    assert np.array_equal(again.getForces(), state.getForces())
+    assert np.array_equal(again.getTermEnergies(), state.getTermEnergies())
+
+
 def test_dense_droplet_beyond_the_kept_entries():
     # 30,000 particles within 2 nm of a 20 nm box, most of them without parameters: every block is a candidate of every
     # other, more than the list keeps per block, and the tiles exceed the estimate from the mean density
