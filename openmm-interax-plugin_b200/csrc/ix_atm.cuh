@@ -728,23 +728,25 @@ __global__ void __launch_bounds__(32 * kAtmWarps) kTriplesWide(AtmBuffers A, Atm
 }
 
 // The wide kernel where its grid is not empty, and the fast one.  The wide kernel mostly returns at once: it goes
-// first, while there is room on the SMs; behind the fast one it waited for the pair kernel's last blocks.
+// first, while there is room on the SMs; behind the fast one it waited for the pair kernel's last blocks.  `before` (may
+// be null) is recorded ahead of the fast kernel.
 template <bool DAMP, bool IMAGE>
 static void launchTriplesAs(const AtmBuffers& A, const AtmConfig& C, int fastBlocks, int wideBlocks, const int* gate,
-                            cudaStream_t st) {
+                            cudaStream_t st, cudaEvent_t before) {
     if (wideBlocks > 0)
         kTriplesWide<DAMP, IMAGE><<<wideBlocks, 32 * kAtmWarps,
                                     kAtmWarps * sizeof(TripleStorage<DAMP, kAtmMaxStaged>), st>>>(
             A, C, fastBlocks * kAtmFastWarps, gate);
+    if (before) cudaEventRecord(before, st);
     kTriplesFast<DAMP, IMAGE><<<fastBlocks, 32 * kAtmFastWarps, 0, st>>>(A, C);
 }
 static void launchTriples(const AtmBuffers& A, const AtmConfig& C, int fastBlocks, int wideBlocks, const int* gate,
-                          cudaStream_t st) {
+                          cudaStream_t st, cudaEvent_t before = nullptr) {
     const bool damp = C.useTangToennies || C.invCentroidRadius > 0.0f;
-    if (damp && C.imageBC) launchTriplesAs<true, true>(A, C, fastBlocks, wideBlocks, gate, st);
-    else if (damp) launchTriplesAs<true, false>(A, C, fastBlocks, wideBlocks, gate, st);
-    else if (C.imageBC) launchTriplesAs<false, true>(A, C, fastBlocks, wideBlocks, gate, st);
-    else launchTriplesAs<false, false>(A, C, fastBlocks, wideBlocks, gate, st);
+    if (damp && C.imageBC) launchTriplesAs<true, true>(A, C, fastBlocks, wideBlocks, gate, st, before);
+    else if (damp) launchTriplesAs<true, false>(A, C, fastBlocks, wideBlocks, gate, st, before);
+    else if (C.imageBC) launchTriplesAs<false, true>(A, C, fastBlocks, wideBlocks, gate, st, before);
+    else launchTriplesAs<false, false>(A, C, fastBlocks, wideBlocks, gate, st, before);
 }
 
 // Each particle of a site receives the site force divided by the number of particles

@@ -753,12 +753,6 @@ static int uploadPairParams(ix_ctx* ctx) {
     return IX_OK;
 }
 
-// How far the tiles of a small system are split (ListBuffers::splitShift), by its size alone.  A tile is one warp's
-// work, about 30 us of dependent steps: with fewer tiles than the SMs hold warps (4,736) that is what the pair kernel
-// takes, whatever the system.  Evaluations of the pair terms back to back, whole / in two / in four: 648 atoms 57.5 /
-// 48.8 / 37.5 us, 2,100 atoms 62.4 / 60.9 / 51.6, 3,000 atoms 74.3 / 61.9 / 63.6, 7,800 atoms 83.3 / 76.2 / 88.3.
-static int tileSplit(int nb) { return nb <= 72 ? 2 : (nb <= 256 ? 1 : 0); }
-
 // Estimated number of tiles of the list (the build reports overflows, and the host then grows the buffers).
 static long long estimateTiles(const ix_ctx* ctx, int nb) {
     if (ctx->method == IX_NO_CUTOFF) return (long long)nb * (nb + 1) / 2 + nb;
@@ -847,14 +841,13 @@ static int allocatePair(ix_ctx* ctx, long long tileCap) {
     IX_TRY(deviceAlloc(ctx, "bbox", 2 * (size_t)nb, &L.bbox));
     IX_TRY(deviceAlloc(ctx, "blockAtoms", nb, &L.blockAtoms));
     IX_TRY(deviceAlloc(ctx, "blockTiles", nb + 1, &L.blockTiles));
-    // an i-block of a liquid has some tens of candidate blocks in each share of its search
-    L.entryCap = G.useCutoff ? std::min((nb + 3) / 4 + 1, 96) : (nb + 3) / 4 + 1;
+    // an i-block of a liquid has at most about 250 candidate blocks
+    L.entryCap = G.useCutoff ? std::min(nb, 384) : nb;
     IX_TRY(deviceAlloc(ctx, "blockEntries", nb, &L.blockEntries));
-    IX_TRY(deviceAlloc(ctx, "entries", 4 * (size_t)nb * L.entryCap, &L.entries));
+    IX_TRY(deviceAlloc(ctx, "entries", (size_t)nb * L.entryCap, &L.entries));
     if (tileCap > (long long)1 << 26) return fail(ctx, IX_ERR_INVALID, "neighbor list too large (%lld tiles)", tileCap);
     ctx->tileCap = (int)tileCap;
     L.tileCap = (int)tileCap;
-    L.splitShift = tileSplit(nb);
     IX_TRY(deviceAlloc(ctx, "tileJ", 32 * (size_t)L.tileCap, &L.tileJ));
     IX_TRY(deviceAlloc(ctx, "tileIBlock", L.tileCap, &L.tileIBlock));
     IX_TRY(deviceAlloc(ctx, "bucketTiles", (size_t)kTileBuckets * L.tileCap, &L.bucketTiles));
@@ -1414,7 +1407,7 @@ static int launchEvaluation(ix_ctx* ctx, unsigned terms, double* outForces, doub
         recordTiming(ctx, 2, sa);
         // the sites whose lists are too long for the fast kernel go to the wide one, which returns at once when there
         // are none and goes first
-        launchTriples(A, C, ctx->atmFastBlocks, ctx->atmGridBlocks, A.flag + 2, sa);
+        launchTriples(A, C, ctx->atmFastBlocks, ctx->atmGridBlocks, A.flag + 2, sa, fork ? ctx->evFork : nullptr);
         ctx->launches += 5;
         recordTiming(ctx, 3, sa);
         ctx->evAtm = ctx->profiling;
@@ -1438,12 +1431,17 @@ static int launchEvaluation(ix_ctx* ctx, unsigned terms, double* outForces, doub
         kCellKeys<<<(n + kCellThreads - 1) / kCellThreads, kCellThreads, 0, st>>>(L, ctx->G);
         kScatterCells<<<gN, tpb, 0, st>>>(L);
         kSortBlocks<<<gNp, tpb, 0, st>>>(L, ctx->G, S);
-        kListBlocks<<<(4 * L.nb + kListWarps - 1) / kListWarps, kListThreads, 0, st>>>(L, ctx->G);
+        // at most four blocks per SM: more gain nothing in a rebuild and return later in a step without one
+        kListBlocks<<<std::min(ctx->numSMs * 4, L.nb), kListThreads, 0, st>>>(L, ctx->G);
         // no more warps than tiles, and four blocks per SM at most: with eight the masks of 24,000 atoms take 37 us for
         // 41, but a step without a rebuild waits 4.2 us for the blocks to return for 2.7
         kTileMasks<<<std::min(ctx->numSMs * 4, std::max(1, (L.tileCap + kListWarps - 1) / kListWarps)),
                      kListThreads, 0, st>>>(L, ctx->G);
         ctx->launches += ctx->G.periodic ? 5 : 6;
+        // the pair kernel's persistent grid fills the SMs: the triple kernel, ready at the same time and on a stream of
+        // higher priority, is placed first (it was left to the end of the pair kernel when its chain came a microsecond
+        // later: 139 us for the two instead of 112)
+        if (fork) IX_CUDA(ctx, cudaStreamWaitEvent(st, ctx->evFork, 0));
         PairTermConfig C = pairConfig(ctx, terms);
         // the lean instantiation when no selected term has a soft core, a switching function or the order-2 overlap
         bool lean = true;
@@ -1525,7 +1523,7 @@ static int prepare(ix_ctx* ctx, unsigned terms) {
     if ((terms & 7u) && !ctx->pairAllocated) {
         updateGeometry(ctx);
         const int nb = (ctx->n + 31) / 32;
-        IX_TRY(allocatePair(ctx, ctx->tileCapRequest > 0 ? ctx->tileCapRequest : estimateTiles(ctx, nb) << tileSplit(nb)));
+        IX_TRY(allocatePair(ctx, ctx->tileCapRequest > 0 ? ctx->tileCapRequest : estimateTiles(ctx, nb)));
     }
     if ((terms & 8u) && !ctx->atmAllocated) IX_TRY(allocateAtm(ctx));
     return IX_OK;
@@ -1548,7 +1546,7 @@ static int checkOverflowFlags(ix_ctx* ctx, unsigned terms, const int* flags, boo
         long long tiles = 0;
         int cnt = 0;
         IX_CUDA(ctx, cudaMemcpy(&cnt, ctx->L.blockTiles + ctx->L.nb, sizeof(int), cudaMemcpyDeviceToHost));
-        tiles = std::max<long long>(2LL * ctx->tileCap, (long long)(1.3 * ((long long)cnt << ctx->L.splitShift)) + 64);
+        tiles = std::max<long long>(2LL * ctx->tileCap, (long long)(1.3 * cnt) + 64);
         int zero[4] = {1, 0, 0, 0};
         IX_CUDA(ctx, cudaMemcpy(ctx->dFlags, zero, sizeof(zero), cudaMemcpyHostToDevice));
         ctx->pairAllocated = false;
@@ -1708,6 +1706,13 @@ static PinnedSlots& pinnedSlots() {
     return *slots;
 }
 
+// A stream whose kernels are placed before those of other streams (the three-body chain's).
+static bool createUrgentStream(cudaStream_t* stream) {
+    int least = 0, greatest = 0;
+    return cudaDeviceGetStreamPriorityRange(&least, &greatest) == cudaSuccess &&
+           cudaStreamCreateWithPriority(stream, cudaStreamNonBlocking, greatest) == cudaSuccess;
+}
+
 // The device side of a context: streams, events and the buffers every evaluation uses (through ctx->arena when a
 // server owns the context).  A context described on the host only (a server request) gets it on admission.
 static int ctxInitDevice(ix_ctx* ctx) {
@@ -1716,7 +1721,7 @@ static int ctxInitDevice(ix_ctx* ctx) {
     sharedSplit();
     // streams and events a server hands over from its pool are kept
     if ((!ctx->stream && cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess) ||
-        (!ctx->stream2 && cudaStreamCreateWithFlags(&ctx->stream2, cudaStreamNonBlocking) != cudaSuccess) ||
+        (!ctx->stream2 && !createUrgentStream(&ctx->stream2)) ||
         (!ctx->evFork && cudaEventCreateWithFlags(&ctx->evFork, cudaEventDisableTiming) != cudaSuccess) ||
         (!ctx->evJoin && cudaEventCreateWithFlags(&ctx->evJoin, cudaEventDisableTiming) != cudaSuccess))
         return fail(ctx, IX_ERR_CUDA, "cudaStreamCreate failed");

@@ -67,11 +67,10 @@ struct ListBuffers {
     float4* sposf;              // np
     float4* bbox;               // nb x 2: center (xyz), half extent (xyz)
     // tiles
-    int4* blockAtoms;           // nb: candidate j particles of each i-block, in the four shares of its search
-    int4* blockEntries;         // nb: candidate blocks in each share
-    int4* entries;              // nb x 4 x entryCap: (block J, mask of its candidate particles, the share's candidates
-                                // before them)
-    int entryCap;               // per share
+    int* blockAtoms;            // nb: candidate j particles of each i-block
+    int* blockEntries;          // nb: candidate blocks of each i-block
+    int4* entries;              // nb x entryCap: (block J, mask of its candidate particles, candidates before them)
+    int entryCap;
     int* blockTiles;            // nb + 1: exclusive scan of the tile counts, then the total
     int* tileJ;                 // tileCap x 32
     int* tileIBlock;            // tileCap
@@ -80,7 +79,6 @@ struct ListBuffers {
     int* tileOrder;             // numTiles: the tiles by decreasing candidate count (a batch's static list)
     unsigned* tileMask;         // tileCap x 64: row masks (per i lane, bit = j slot), then column masks (per j lane)
     int* numTiles;              // tiles to evaluate (0 after an overflow)
-    int splitShift;             // each tile of 32 x 32 candidates is listed as 2^splitShift tiles of a share of its rows
     int* taskCounter;           // next tile of the pair kernel's dynamic schedule (zeroed before each launch)
     int tileCap;
     const int* flags;           // sorted particle flags (the term gates of each particle)
@@ -400,100 +398,64 @@ __device__ __forceinline__ bool isExcluded(const ListBuffers& L, int oi, int oj)
 constexpr int kListThreads = 256;
 constexpr int kListWarps = kListThreads / 32;
 
-// The blocks an i-block pairs with are itself and the half of the others that follow it cyclically, so that every
-// i-block has about the same number of candidates (with the blocks J >= I the first had twice as many and the list
-// waited for it).  The number of those blocks, from I on:
-__device__ __forceinline__ int followingBlocks(int nb, int I) {
-    return nb / 2 + ((nb & 1) || I < nb / 2 ? 1 : 0);
-}
-
-// Share `part` of four of the candidate blocks of i-block I: every fourth block J that I pairs with, in cyclic order
-// (neighbors along the curve are neighbors in space, so contiguous shares would be uneven).  One warp; the boxes 32 at a
-// time (the next 32 loaded meanwhile), then the particles of the near blocks eight at a time, their loads and tests in
-// flight together.  group(J, mask): lane u < 8 holds the u-th of the eight blocks and its particles (mask) within the
-// list cutoff of block I's box (0: none, or no such block); until it returns false.
-template <class F>
-__device__ __forceinline__ void candidateBlocks(const ListBuffers& L, const ListGeometry& G, int I, int part, int lane,
-                                                F group) {
-    const float4 ci = L.bbox[2 * I], ei = L.bbox[2 * I + 1];
-    const float cut2 = G.useCutoff ? G.listCutoff * G.listCutoff : INFINITY;
-    const int follow = followingBlocks(L.nb, I);
-    auto blockAt = [&](int o) {
-        const int J = I + min(o, follow - 1);
-        return J < L.nb ? J : J - L.nb;
-    };
-    int J = blockAt(4 * lane + part);
-    float4 cj = L.bbox[2 * J], ej = L.bbox[2 * J + 1];
-    for (int o = part; o < follow; o += 128) {
-        const bool near = o + 4 * lane < follow && boxBoxDist2(ci, ei, cj, ej, G) < cut2;
-        unsigned todo = __ballot_sync(0xffffffffu, near);
-        J = blockAt(o + 128 + 4 * lane);
-        cj = L.bbox[2 * J];
-        ej = L.bbox[2 * J + 1];
-        while (todo) {
-            int Js[8];
-            float4 p[8];
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-                Js[u] = todo ? blockAt(o + 4 * (__ffs(todo) - 1)) : -1;
-                todo &= todo - 1;
-                p[u] = L.sposf[32 * max(Js[u], 0) + lane];
-            }
-            int myJ = -1;
-            unsigned mine = 0;
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const bool in = Js[u] >= 0 && 32 * Js[u] + lane < L.n &&
-                                (!G.useCutoff || pointBoxDist2(p[u], ci, ei, G) < cut2);
-                const unsigned m = __ballot_sync(0xffffffffu, in);
-                if (lane == u) {
-                    myJ = Js[u];
-                    mine = m;
-                }
-            }
-            if (!group(myJ, mine)) return;
-        }
-    }
-}
-
-// The candidates of each i-block, four warps per i-block, and in the last block the exclusive scan of the tile counts.
-// On overflow no tile is scheduled (nothing is written beyond the buffers); the host grows them and evaluates again.
-// Bound by latency: a warp's search is one chain of loads and tests.  A thread block per i-block with its candidates
-// shared among the warps through shared memory took 12.5 us for 24,000 atoms, and a second pass over the same
-// candidates to write the tiles another 15.6 (the mask kernel now finds its candidates from the entries); this takes
-// 24 us (41 with one warp per i-block), and half as many blocks return at once in a step without a rebuild.
+// The candidates of each i-block: the particles of the blocks J >= I whose box is within the list cutoff of block I's box
+// and whose own position is within it too, in the order (J, slot).  One thread block per i-block: the blocks are
+// examined 256 at a time, each thread testing one block's box; the candidate blocks are compacted in block order and
+// the warps take them round robin for the particle tests (neighbors along the curve are neighbors in space, so
+// contiguous shares would be uneven: 37 us for 24,000 atoms).  The entries hold what the mask kernel needs to find the
+// candidates of a tile; a second pass over the same candidates to write the tiles had taken 15.6 us.  The last block
+// scans the tile counts.  On overflow no tile is scheduled (nothing is written beyond the buffers); the host grows
+// them and evaluates again.
 __global__ void __launch_bounds__(kListThreads) kListBlocks(ListBuffers L, ListGeometry G) {
     if (!rebuildRequested(L)) return;
-    const int tid = threadIdx.x, lane = tid & 31;
-    const int unit = (blockIdx.x * kListThreads + tid) >> 5;
-    if (unit < 4 * L.nb) {
-        const int I = unit >> 2;
+    __shared__ int candJ[kListThreads];
+    __shared__ unsigned keep[kListThreads];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const float cut2 = G.useCutoff ? G.listCutoff * G.listCutoff : INFINITY;
+    for (int I = blockIdx.x; I < L.nb; I += gridDim.x) {
+        const float4 ci = L.bbox[2 * I], ei = L.bbox[2 * I + 1];
         int atoms = 0, entries = 0;
-        candidateBlocks(L, G, I, unit & 3, lane, [&](int J, unsigned m) {
-            const unsigned have = __ballot_sync(0xffffffffu, m != 0);
-            int before = __popc(m);
+        for (int Jc = I; Jc < L.nb; Jc += kListThreads) {
+            // the candidate blocks of this chunk, in block order
+            const int J = Jc + tid;
+            const bool cand = J < L.nb && boxBoxDist2(ci, ei, L.bbox[2 * J], L.bbox[2 * J + 1], G) < cut2;
+            int total;
+            const int at = blockPrefix<kListThreads>(cand, total);
+            if (cand) candJ[at] = J;
+            __syncthreads();
+            // the particle tests of the candidate blocks, four blocks' loads in flight
+            for (int k0 = warp; k0 < total; k0 += 4 * kListWarps) {
+                float4 p[4];
 #pragma unroll
-            for (int o = 1; o < 8; o <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, before, o);
-                if (lane >= o) before += v;
+                for (int u = 0; u < 4; u++) p[u] = L.sposf[32 * candJ[min(k0 + u * kListWarps, total - 1)] + lane];
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const int k = k0 + u * kListWarps;
+                    const bool in = k < total && 32 * candJ[min(k, total - 1)] + lane < L.n &&
+                                    (!G.useCutoff || pointBoxDist2(p[u], ci, ei, G) < cut2);
+                    const unsigned m = __ballot_sync(0xffffffffu, in);
+                    if (lane == 0 && k < total) keep[k] = m;
+                }
             }
-            const int at = entries + __popc(have & laneMaskLt());
-            if (m && at < L.entryCap)
-                L.entries[(size_t)unit * L.entryCap + at] = make_int4(J, (int)m, atoms + before - __popc(m), 0);
-            entries += __popc(have);
-            atoms += __shfl_sync(0xffffffffu, before, 7);
-            return true;
-        });
-        if (lane == 0) {
-            reinterpret_cast<int*>(L.blockAtoms)[unit] = atoms;
-            reinterpret_cast<int*>(L.blockEntries)[unit] = entries;
+            __syncthreads();
+            // entries (in the upper bits) and candidates of the chunk before each candidate block
+            const unsigned m = tid < total ? keep[tid] : 0u;
+            int sum;
+            const int before = blockPrefix<kListThreads>(__popc(m) + (m ? 1 << 16 : 0), sum);
+            const int e = entries + (before >> 16);
+            if (m && e < L.entryCap)
+                L.entries[(size_t)I * L.entryCap + e] = make_int4(candJ[tid], (int)m, atoms + (before & 0xffff), 0);
+            entries += sum >> 16;
+            atoms += sum & 0xffff;
+            __syncthreads();   // the shared arrays are refilled by the next chunk
+        }
+        if (tid == 0) {
+            L.blockAtoms[I] = atoms;
+            L.blockEntries[I] = entries;
         }
     }
     if (!lastBlock(L.ticket)) return;
-    auto tiles = [&](int c) {
-        const int4 a = __ldcg(L.blockAtoms + c);
-        return ((a.x + a.y) + (a.z + a.w) + 31) / 32;
-    };
+    auto tiles = [&](int c) { return (__ldcg(L.blockAtoms + c) + 31) / 32; };
     const int per = (L.nb + kListThreads - 1) / kListThreads;
     const int begin = min(tid * per, L.nb), end = min(begin + per, L.nb);
     int sum = 0;
@@ -507,13 +469,12 @@ __global__ void __launch_bounds__(kListThreads) kListBlocks(ListBuffers L, ListG
     if (tid < kTileBuckets) L.bucketCount[tid] = 0;
     if (tid == 0) {
         L.blockTiles[L.nb] = total;
-        const bool fits = (long long)total << L.splitShift <= L.tileCap;
-        *L.numTiles = fits ? total << L.splitShift : 0;
-        if (!fits) atomicOr(L.flag + 1, 1);
+        *L.numTiles = total > L.tileCap ? 0 : total;
+        if (total > L.tileCap) atomicOr(L.flag + 1, 1);
     }
 }
 
-// The i-block of tile t (before the split): the last whose first tile is at or before t and that has tiles (a 32-way search by a warp).
+// The i-block of tile t: the last whose first tile is at or before t and that has tiles (a 32-way search by a warp).
 __device__ __forceinline__ int tileBlock(const ListBuffers& L, int t, int lane) {
     int lo = 0, n = L.nb + 1;                        // blockTiles[lo] <= t < blockTiles[lo + n]
     while (n > 1) {
@@ -538,37 +499,34 @@ __device__ __forceinline__ void tileCandidates(const ListBuffers& L, const ListG
         const int q = at + __popc(m & lt);
         if (((m >> lane) & 1u) && q >= 0 && q < 32) slots[q] = 32 * J + lane;
     };
-    const int4 n4 = L.blockEntries[I], a4 = L.blockAtoms[I];
-    const int counts[4] = {n4.x, n4.y, n4.z, n4.w}, atoms[4] = {a4.x, a4.y, a4.z, a4.w};
-    int base = 0;
-#pragma unroll
-    for (int part = 0; part < 4; part++) {
-        const int n = counts[part], lo = first - base;         // the tile's candidates among the share's: lo .. lo + 31
-        base += atoms[part];
-        if (lo <= -32 || lo >= atoms[part]) continue;
-        if (n <= L.entryCap) {
-            const int4* E = L.entries + (size_t)(4 * I + part) * L.entryCap;
-            for (int e0 = 0; e0 < n; e0 += 32) {
-                const int4 v = e0 + lane < n ? E[e0 + lane] : make_int4(0, 0, INT_MAX, 0);
-                const bool after = v.z >= lo + 32, mine = !after && v.z + __popc((unsigned)v.y) > lo;
-                for (unsigned b = __ballot_sync(0xffffffffu, mine); b; b &= b - 1) {
-                    const int k = __ffs(b) - 1;
-                    take(__shfl_sync(0xffffffffu, v.x, k), (unsigned)__shfl_sync(0xffffffffu, v.y, k),
-                         __shfl_sync(0xffffffffu, v.z, k) - lo);
-                }
-                if (__any_sync(0xffffffffu, after)) break;
+    const int n = L.blockEntries[I];
+    if (n <= L.entryCap) {
+        const int4* E = L.entries + (size_t)I * L.entryCap;
+        for (int e0 = 0; e0 < n; e0 += 32) {
+            const int4 v = e0 + lane < n ? E[e0 + lane] : make_int4(0, 0, INT_MAX, 0);
+            const bool after = v.z >= first + 32, mine = !after && v.z + __popc((unsigned)v.y) > first;
+            for (unsigned b = __ballot_sync(0xffffffffu, mine); b; b &= b - 1) {
+                const int k = __ffs(b) - 1;
+                take(__shfl_sync(0xffffffffu, v.x, k), (unsigned)__shfl_sync(0xffffffffu, v.y, k),
+                     __shfl_sync(0xffffffffu, v.z, k) - first);
             }
+            if (__any_sync(0xffffffffu, after)) break;
         }
-        else {
-            int before = 0;
-            candidateBlocks(L, G, I, part, lane, [&](int J, unsigned m) {
-                for (int u = 0; u < 8; u++) {
-                    const unsigned mu = __shfl_sync(0xffffffffu, m, u);
-                    take(__shfl_sync(0xffffffffu, J, u), mu, before - lo);
-                    before += __popc(mu);
-                }
-                return before < lo + 32;
-            });
+    }
+    else {
+        const float4 ci = L.bbox[2 * I], ei = L.bbox[2 * I + 1];
+        const float cut2 = G.useCutoff ? G.listCutoff * G.listCutoff : INFINITY;
+        int before = 0;
+        for (int Jc = I; Jc < L.nb && before < first + 32; Jc += 32) {
+            const int J = Jc + lane;
+            const bool near = J < L.nb && boxBoxDist2(ci, ei, L.bbox[2 * J], L.bbox[2 * J + 1], G) < cut2;
+            for (unsigned todo = __ballot_sync(0xffffffffu, near); todo; todo &= todo - 1) {
+                const int K = Jc + __ffs(todo) - 1, j = 32 * K + lane;
+                const bool in = j < L.n && (!G.useCutoff || pointBoxDist2(L.sposf[j], ci, ei, G) < cut2);
+                const unsigned m = __ballot_sync(0xffffffffu, in);
+                take(K, m, before - first);
+                before += __popc(m);
+            }
         }
     }
     __syncwarp();
@@ -591,7 +549,7 @@ __device__ __forceinline__ unsigned transposeBits(unsigned x, int lane) {
 // The tiles, one warp per tile over the whole list (the tiles of an i-block vary in number, so a per-i-block
 // distribution would wait on the largest): its i-block and candidate j particles, and its pair masks; lane = the tile's
 // j lane, the i particles from shared memory.
-// A pair's bit is set when j is of another block or its slot follows i's (each pair once), both are real particles gated on for a common term,
+// A pair's bit is set when j's slot follows i's (each pair once), both are real particles gated on for a common term,
 // the pair is not excluded and its build-time distance (minimum image) is within the list cutoff: then no pair outside
 // the masks can come within the cutoff before the displacement check requests the next build.  The tests that do not
 // depend on the distance are masks formed once per tile; where the i-block allows it (rectangular box, block small
@@ -605,12 +563,14 @@ __global__ void __launch_bounds__(kListThreads) kTileMasks(ListBuffers L, ListGe
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // the margin covers the float rounding of the build-time distance
     const float cut2 = G.useCutoff ? G.listCutoff * G.listCutoff * (1.0f + 1e-5f) : INFINITY;
-    const int numTiles = *L.numTiles >> L.splitShift;
+    const int numTiles = *L.numTiles;
     const int warps = (gridDim.x * blockDim.x) >> 5;
     for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < numTiles; t += warps) {
         const int I = tileBlock(L, t, lane);
         tileCandidates(L, G, I, 32 * (t - L.blockTiles[I]), lane, slots[warp]);
         const int sj = slots[warp][lane];
+        L.tileJ[32LL * t + lane] = sj;
+        if (lane == 0) L.tileIBlock[t] = I;
         const int si = I * 32 + lane;
         const int oi = L.sortedAtom[si];
         const int fi = L.flags[si];
@@ -636,8 +596,8 @@ __global__ void __launch_bounds__(kListThreads) kTileMasks(ListBuffers L, ListGe
         if (oj >= 0) {
             column = iReal & (((fj & kFlagGateDisp) ? gateD : 0u) | ((fj & kFlagGateExch) ? gateE : 0u) |
                               ((fj & kFlagGateSr) ? gateS : 0u));
-            const int d = sj - I * 32;   // within the i-block itself, the i slots below j's
-            if (d >= 0 && d < 32) column &= (1u << d) - 1u;
+            const int d = sj - I * 32;   // the i slots of the block below j's
+            column &= d >= 32 ? 0xffffffffu : (d <= 0 ? 0u : (1u << d) - 1u);
         }
         // the pairs within the list cutoff, and those whose i lies in j's exclusion range, which are looked up
         unsigned in = 0, suspect = 0;
@@ -674,21 +634,12 @@ __global__ void __launch_bounds__(kListThreads) kTileMasks(ListBuffers L, ListGe
             if (isExcluded(L, oj, __float_as_int(ipos[warp][i].w))) column &= ~(1u << i);
         }
         const unsigned row = transposeBits(column, lane);
-        // listed whole, or as tiles that take a share of the rows each
-        const int rows = 32 >> L.splitShift;
-        for (int part = 0; part < 1 << L.splitShift; part++) {
-            const size_t out = ((size_t)t << L.splitShift) + part;
-            const unsigned mine = (0xffffffffu >> (32 - rows)) << (part * rows);
-            const unsigned some = column & mine;
-            L.tileJ[32 * out + lane] = sj;
-            L.tileMask[64 * out + lane] = (mine >> lane) & 1u ? row : 0u;
-            L.tileMask[64 * out + 32 + lane] = some;
-            const unsigned pairs = __reduce_add_sync(0xffffffffu, (unsigned)__popc(some));
-            if (lane == 0) {
-                L.tileIBlock[out] = I;
-                const int b = min((int)(pairs >> 6), kTileBuckets - 1);
-                L.bucketTiles[(size_t)b * L.tileCap + atomicAdd(L.bucketCount + b, 1)] = (int)out;
-            }
+        L.tileMask[64LL * t + lane] = row;
+        L.tileMask[64LL * t + 32 + lane] = column;
+        const unsigned pairs = __reduce_add_sync(0xffffffffu, (unsigned)__popc(column));
+        if (lane == 0) {
+            const int b = min((int)(pairs >> 6), kTileBuckets - 1);
+            L.bucketTiles[(size_t)b * L.tileCap + atomicAdd(L.bucketCount + b, 1)] = t;
         }
     }
 }

@@ -1051,7 +1051,7 @@ int ix_server_create(int device, double budget_bytes, int max_running, int threa
         for (int i = 0; i < S->maxRunning; i++) {
             StreamSet set;
             if (cudaStreamCreateWithFlags(&set.stream, cudaStreamNonBlocking) != cudaSuccess ||
-                cudaStreamCreateWithFlags(&set.stream2, cudaStreamNonBlocking) != cudaSuccess ||
+                !createUrgentStream(&set.stream2) ||
                 cudaEventCreateWithFlags(&set.fork, cudaEventDisableTiming) != cudaSuccess ||
                 cudaEventCreateWithFlags(&set.join, cudaEventDisableTiming) != cudaSuccess) {
                 cudaGetLastError();

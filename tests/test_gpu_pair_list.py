@@ -88,8 +88,8 @@ def test_sizes_and_boundaries(n, kind):
         x = x + rng.uniform(-1, 1, size=(n, 3)) * (0.004 if step == 0 else 0.02) + (0.0 if step == 0 else 0.1)
 
 
-@pytest.mark.parametrize("n", [2304, 2305, 8192, 8193])
-def test_sizes_where_the_tiles_split_changes(n):
+@pytest.mark.parametrize("n", [2305, 8193])
+def test_larger_lists_and_their_growth(n):
     rng = np.random.default_rng(n)
     side = int(np.ceil(n ** (1 / 3)))
     box = np.eye(3) * side * 0.28
