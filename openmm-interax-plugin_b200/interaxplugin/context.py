@@ -301,8 +301,7 @@ class Context:
     # -- MD -----------------------------------------------------------------------------------------------------
     def runVelocityVerlet(self, steps, dt, velocities):
         """Run `steps` velocity-Verlet steps of `dt` ps on the device; returns (positions, velocities, energy)."""
-        n = self._system.getNumParticles()
-        masses = _capi.arr([self._system.getParticleMass(i) for i in range(n)], np.float64)
+        masses = self._system._masses_array()
         self._check(self._lib.ix_md_set_masses(self._ctx, _capi.ptr(masses)))
         pos = self._positions.copy()
         vel = _capi.arr(velocities, np.float64).copy()

@@ -5,6 +5,8 @@ InteraxShortRangeForce.h:59-162 and InteraxThreeBodyForce.h:75-258 (and the SWIG
 which exposes the same class and method names).  These objects only hold parameters; a Context uploads them to the
 device through the C-ABI, which performs the validation the reference performs at Context creation.
 """
+import numpy as np
+
 
 class OpenMMException(Exception):
     """Raised where the reference throws OpenMM::OpenMMException, with the same messages."""
@@ -319,6 +321,7 @@ class System:
 
     def __init__(self):
         self._masses = []
+        self._mass_array = None     # the masses as an array, made when asked for and dropped when they change
         self._forces = []
         self._constraints = []
         self._box = [(2.0, 0.0, 0.0), (0.0, 2.0, 0.0), (0.0, 0.0, 2.0)]
@@ -336,6 +339,7 @@ class System:
 
     def addParticle(self, mass):
         self._masses.append(float(mass))
+        self._mass_array = None
         return len(self._masses) - 1
 
     def getNumParticles(self):
@@ -343,6 +347,11 @@ class System:
 
     def getParticleMass(self, index):
         return self._masses[index]
+
+    def _masses_array(self):
+        if self._mass_array is None:
+            self._mass_array = np.array(self._masses, dtype=np.float64)
+        return self._mass_array
 
     def addForce(self, force):
         self._forces.append(force)

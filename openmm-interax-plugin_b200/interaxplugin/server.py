@@ -72,7 +72,7 @@ class Server:
             describe_forces(rec, None, system, lambda rc: None, keep)
             n = system.getNumParticles()
             box = _capi.arr(np.asarray(system.getDefaultPeriodicBoxVectors()).reshape(9), np.float64)
-            mass = _capi.arr([system.getParticleMass(i) for i in range(n)], np.float64)
+            mass = system._masses_array()
             t = (system, n, box, mass, rec.calls, keep)
             self._templates[id(system)] = t
         return t
