@@ -1332,6 +1332,28 @@ __global__ void kClearFlagIf(int* target, const int* gate) {
     if (*(volatile const int*)gate != 0) *target = 0;
 }
 
+// Systems of at most this many blocks of 32 particles take a thread block per tile (kPairTilesSmall).  Evaluations of the
+// pair terms back to back, a warp per tile and a block per tile: 24 atoms 37.1 and 36.6 us, 648 atoms 53.6 and 37.0,
+// 1,500 atoms 61.5 and 40.9, 3,000 atoms 74.1 and 56.3, 4,500 atoms 79.9 and 63.6, 7,800 atoms 87.4 and 86.1, 24,000
+// atoms 137 and 186.
+constexpr int kSmallBlocks = 192;
+
+// The pair kernel's instance for the configuration: lean (no soft core, switching function or order-2 overlap), from
+// the class-pair table, uniform (no gates or scales), and the form for small systems.
+static void launchPairTiles(bool lean, bool table, bool uniform, bool small, int grid, int tiles, size_t dyn,
+                            cudaStream_t st, const ListBuffers& L, const PairBuffers& P, const PairTermConfig& C) {
+    auto run = [&](auto* tileKernel, auto* smallKernel, size_t shared) {
+        if (small) smallKernel<<<std::max(tiles, 1), kTileThreads, shared, st>>>(L, P, C);
+        else tileKernel<<<grid, 32 * kPairWarps, shared, st>>>(L, P, C);
+    };
+    if (lean && table && uniform) run(kPairTiles<true, true, true>, kPairTilesSmall<true, true, true>, dyn);
+    else if (lean && uniform) run(kPairTiles<true, false, true>, kPairTilesSmall<true, false, true>, 0);
+    else if (lean && table) run(kPairTiles<true, true>, kPairTilesSmall<true, true>, dyn);
+    else if (lean) run(kPairTiles<true, false>, kPairTilesSmall<true, false>, 0);
+    else if (table) run(kPairTiles<false, true>, kPairTilesSmall<false, true>, dyn);
+    else run(kPairTiles<false, false>, kPairTilesSmall<false, false>, 0);
+}
+
 // Launch the whole evaluation on the context's stream.  Forces go to outForces (device, n x 3 doubles) and/or are
 // added to addFixed; energies to outEnergy (device, 4 doubles).
 // The second velocity half kick of an MD step, done by the evaluation's finishing kernel.
@@ -1468,12 +1490,7 @@ static int launchEvaluation(ix_ctx* ctx, unsigned terms, double* outForces, doub
         const size_t dyn = table && tableBytes <= (size_t)IX_TUNE_PAIR_SHARED_TABLE_BYTES ? tableBytes : 0;
         P.coefShared = dyn > 0;
         C.coefShared = P.coefShared;
-        if (lean && table && uniform) kPairTiles<true, true, true><<<grid, 32 * kPairWarps, dyn, st>>>(L, P, C);
-        else if (lean && uniform) kPairTiles<true, false, true><<<grid, 32 * kPairWarps, 0, st>>>(L, P, C);
-        else if (lean && table) kPairTiles<true, true><<<grid, 32 * kPairWarps, dyn, st>>>(L, P, C);
-        else if (lean) kPairTiles<true, false><<<grid, 32 * kPairWarps, 0, st>>>(L, P, C);
-        else if (table) kPairTiles<false, true><<<grid, 32 * kPairWarps, dyn, st>>>(L, P, C);
-        else kPairTiles<false, false><<<grid, 32 * kPairWarps, 0, st>>>(L, P, C);
+        launchPairTiles(lean, table, uniform, ctx->L.nb <= kSmallBlocks, grid, L.tileCap, dyn, st, L, P, C);
         ctx->launches += 1;
         recordTiming(ctx, 1, st);
         ctx->evPair = ctx->profiling;
@@ -1652,6 +1669,12 @@ static void sharedSplit() {
     most(kPairTiles<true, false, false>);
     most(kPairTiles<false, true, false>);
     most(kPairTiles<false, false, false>);
+    most(kPairTilesSmall<true, true, true>);
+    most(kPairTilesSmall<true, false, true>);
+    most(kPairTilesSmall<true, true, false>);
+    most(kPairTilesSmall<true, false, false>);
+    most(kPairTilesSmall<false, true, false>);
+    most(kPairTilesSmall<false, false, false>);
     most(kTriplesFast<false, false>);
     most(kTriplesFast<false, true>);
     most(kTriplesFast<true, false>);

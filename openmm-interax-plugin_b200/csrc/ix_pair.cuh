@@ -279,7 +279,8 @@ struct PairWarpStorage {
     unsigned short colList[kPairColumnLists ? 1024 : 1];   // queue positions of each column's pairs, column by column
 };
 
-__device__ __forceinline__ void stageParticle(PairWarpStorage& S, int side, int lane, int s, double cx, double cy,
+template <class Storage>
+__device__ __forceinline__ void stageParticle(Storage& S, int side, int lane, int s, double cx, double cy,
                                               double cz, bool shiftImage, const PairTermConfig& C,
                                               const ListBuffers& L, const PairBuffers& P) {
     if (s >= 0) {
@@ -349,8 +350,8 @@ __device__ __forceinline__ bool pairInside(const float4& hi_i, const float4& lo_
 
 // One queued pair: displacement, the cutoff test (CHECK: the queue holds candidates; else the pairs were filtered
 // when queued), the terms.  Returns the force on i (zero outside the cutoff) and counts the pair if it interacts.
-template <bool LEAN, bool TABLE, bool UNIFORM, bool CHECK>
-__device__ __forceinline__ float4 computeQueuedPair(PairWarpStorage& S, int entry, int iBase, bool perPairImage,
+template <bool LEAN, bool TABLE, bool UNIFORM, bool CHECK, class Storage>
+__device__ __forceinline__ float4 computeQueuedPair(Storage& S, int entry, int iBase, bool perPairImage,
                                                     const PairTermConfig& C, const ListBuffers& L,
                                                     const PairBuffers& P, const PairCoef* coef, float e[3],
                                                     unsigned& pairs) {
@@ -644,6 +645,129 @@ __global__ void __launch_bounds__(32 * kPairWarps, IX_TUNE_PAIR_MIN_BLOCKS) kPai
     }
     for (int o = 16; o > 0; o >>= 1) pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
     if (lane == 0 && pairs) atomicAdd(P.pairCount, pairs);
+}
+
+// The pair kernel of small systems: a thread block per tile.  A tile is about 30 us of dependent steps for one warp, and
+// a system with fewer tiles than the SMs hold warps pays that whatever its size; four warps that share a tile's work
+// take half as long (33 us a launch for 648 atoms, and 16.4; 31 and 16.4 for 750 atoms without a cutoff).  Every force
+// is the one kPairTiles gives, to the last bit: the pairs are queued in the same order, each pair's force is kept, and
+// each particle's sum runs over them in the same sequence (a tile of rows split among tasks would change the sums).
+// Shared memory for all of a tile's forces (22 KB a block) and the idle threads of the gather make it the slower one
+// where tiles abound (kSmallBlocks).
+constexpr int kTileThreads = 128;
+struct PairTileStorage {
+    float4 hi[2][32], lo[2][32];
+    int jslot[32];
+    int rowStart[32];
+    unsigned rowMask[32];
+    unsigned short queue[1024];
+    float4 force[1024];
+    double energy[kTileThreads / 32][3];
+};
+
+template <bool LEAN, bool TABLE, bool UNIFORM = false>
+__global__ void __launch_bounds__(kTileThreads) kPairTilesSmall(ListBuffers L, PairBuffers P, PairTermConfig C) {
+    __shared__ PairTileStorage S;
+    extern __shared__ float4 pairShared[];
+    constexpr bool PREFILTER = !(LEAN && TABLE);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const PairCoef* coef = P.coef;
+    if (TABLE && P.coefShared) {
+        const int words = P.numClasses * P.numClasses * (int)(sizeof(PairCoef) / sizeof(float4));
+        const float4* src = reinterpret_cast<const float4*>(P.coef);
+        for (int k = tid; k < words; k += kTileThreads) pairShared[k] = __ldg(src + k);
+        coef = reinterpret_cast<const PairCoef*>(pairShared);
+    }
+    const int numTasks = P.taskTiles ? P.numTasks : min(*L.numTiles, L.tileCap);
+    const unsigned ltMask = laneMaskLt();
+    unsigned pairs = 0;
+    for (int task = blockIdx.x; task < numTasks; task += gridDim.x) {
+        const int t = P.taskTiles ? P.taskTiles[task] : task;
+        const int I = L.tileIBlock[t];
+        const int iBase = I * 32;
+        const float4 center = L.bbox[2 * I];
+        const bool shiftImage = C.periodic && center.w != 0.0f;
+        const bool perPairImage = C.periodic && !shiftImage;
+        const int jslot = L.tileJ[32 * t + lane];
+        __syncthreads();      // the last tile's shared data has been read
+        if (warp == 0) {
+            S.rowMask[lane] = L.tileMask[64 * t + lane];
+            stageParticle(S, 0, lane, iBase + lane, center.x, center.y, center.z, false, C, L, P);
+        }
+        else if (warp == 1) stageParticle(S, 1, lane, jslot, center.x, center.y, center.z, shiftImage, C, L, P);
+        __syncthreads();
+        // each warp eight rows: the candidates kept, as the warp-per-tile kernel keeps them
+        for (int r = 8 * warp; r < 8 * warp + 8; r++) {
+            bool in = (S.rowMask[r] >> lane) & 1u;
+            if (C.alchOnlyBit)
+                in = in && ((__float_as_int(S.hi[0][r].w) ^ __float_as_int(S.hi[1][lane].w)) & C.alchOnlyBit) != 0;
+            if (PREFILTER && C.useCutoff && in)
+                in = pairInside(S.hi[0][r], S.lo[0][r], S.hi[1][lane], S.lo[1][lane], perPairImage, C);
+            const unsigned m = __ballot_sync(0xffffffffu, in);
+            __syncwarp();
+            if (lane == 0) S.rowMask[r] = m;
+        }
+        __syncthreads();
+        // every warp forms the rows' offsets; each queues its rows
+        const unsigned row = S.rowMask[lane];
+        const int count = __popc(row);
+        int start = count;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, start, o);
+            if (lane >= o) start += v;
+        }
+        const int total = __shfl_sync(0xffffffffu, start, 31);
+        start -= count;
+        if (warp == 0) S.rowStart[lane] = start;
+        for (int r = 8 * warp; r < 8 * warp + 8; r++) {
+            const unsigned m = __shfl_sync(0xffffffffu, row, r);
+            const int first = __shfl_sync(0xffffffffu, start, r);
+            if ((m >> lane) & 1u) S.queue[first + __popc(m & ltMask)] = (unsigned short)((r << 5) | lane);
+        }
+        __syncthreads();
+        float e[3] = {0.0f, 0.0f, 0.0f};
+        for (int p = tid; p < total; p += kTileThreads)
+            S.force[p] = computeQueuedPair<LEAN, TABLE, UNIFORM, !PREFILTER>(S, S.queue[p], iBase, perPairImage, C, L,
+                                                                             P, coef, e, pairs);
+        for (int k = 0; k < 3; k++) {
+            const double sum = warpSumD((double)e[k]);
+            if (lane == 0) S.energy[warp][k] = sum;
+        }
+        __syncthreads();
+        float f[3] = {0.0f, 0.0f, 0.0f};
+        if (warp == 0) {
+            // i side: the row's pairs
+            for (int q = start; q < start + count; q++) {
+                const float4 v = S.force[q];
+                f[0] += v.x;
+                f[1] += v.y;
+                f[2] += v.z;
+            }
+            flushForce(f, iBase + lane, L.np, P.forceFixed);
+        }
+        else if (warp == 1) {
+            // j side: the pair (i, lane) of each row that holds it
+#pragma unroll 4
+            for (int i = 0; i < 32; i++) {
+                const unsigned m = S.rowMask[i];
+                if (!((m >> lane) & 1u)) continue;
+                const float4 v = S.force[S.rowStart[i] + __popc(m & ltMask)];
+                f[0] -= v.x;
+                f[1] -= v.y;
+                f[2] -= v.z;
+            }
+            flushForce(f, jslot, L.np, P.forceFixed);
+        }
+        else if (warp == 2 && lane < 3) {
+            double sum = 0.0;
+            for (int w = 0; w < kTileThreads / 32; w++) sum += S.energy[w][lane];
+            P.taskEnergy[3 * (P.taskTiles ? task : t) + lane] = sum;
+        }
+    }
+    unsigned long long all = pairs;
+    for (int o = 16; o > 0; o >>= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
+    if (lane == 0 && all) atomicAdd(P.pairCount, all);
 }
 
 }  // namespace ix
