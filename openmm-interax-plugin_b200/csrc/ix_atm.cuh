@@ -486,7 +486,7 @@ __device__ __forceinline__ void storeNeighbor(TripleStorage<DAMP, N>& S, const A
 // triangular index, stored both forces in shared memory and gathered them per neighbor, 425 issue slots per 32 pairs.
 // Kernel times on one B200, both triple kernels, before and now: 96,000-atom box, 0.8 nm, 13.6 M triples: 421 and
 // 159 us; 24,000 atoms, 0.6 nm, 0.46 M triples: 24 and 19 us; 648 atoms: 15.7 and 10.9 us.
-template <bool DAMP, bool IMAGE, int N>
+template <bool DAMP, bool IMAGE, bool ALCH, int N>
 __device__ __forceinline__ void siteTriples(const TripleStorage<DAMP, N>& S, const AtmBuffers& A, const AtmConfig& C,
                                             const float4& pa, int cFirst, int cStep, int cEnd, int bBegin, int bEnd,
                                             int lane, float (&fa)[3], float& energy,
@@ -512,6 +512,7 @@ __device__ __forceinline__ void siteTriples(const TripleStorage<DAMP, N>& S, con
             if (!(w < C.cutoff2)) continue;
             float c9 = (pb.y * pc.y) * kA * fmaf(pa.y, rcpApprox(pb.x + pc.x), 1.0f);
             if (pb.z != 0.0f || pc.z != 0.0f) c9 *= lambdaBC;
+            else if (ALCH && pa.w == 0.0f) continue;
             if (c9 == 0.0f) continue;
             const float p = fmaf(xb.x, xc.x, fmaf(xb.y, xc.y, xb.z * xc.z));
             const float q = fmaf(xb.x, cx, fmaf(xb.y, cy, xb.z * cz));
@@ -623,7 +624,7 @@ __device__ __forceinline__ int stageTripleNeighborsScan(const AtmBuffers& A, con
     return m;
 }
 
-template <bool DAMP, bool IMAGE>
+template <bool DAMP, bool IMAGE, bool ALCH>
 __global__ void __launch_bounds__(32 * kAtmFastWarps, IX_TUNE_ATM_MIN_BLOCKS) kTriplesFast(AtmBuffers A, AtmConfig C) {
     __shared__ TripleStorage<DAMP, kAtmFastStaged> storage[kAtmFastWarps];
     auto& S = storage[threadIdx.x >> 5];
@@ -636,6 +637,12 @@ __global__ void __launch_bounds__(32 * kAtmFastWarps, IX_TUNE_ATM_MIN_BLOCKS) kT
         const int n = A.nbrCount[a];
         if (n > fastMax || n > A.cap) continue;        // the wide kernel takes this site
         const float4 pa = A.siteParams[a];
+        if (ALCH && pa.w == 0.0f) {
+            // only the triples with an alchemical site: most sites have none
+            bool any = false;
+            for (int k = lane; k < n; k += 32) any |= A.siteParams[A.nbr[(size_t)a * A.cap + k]].w != 0.0f;
+            if (!__any_sync(0xffffffffu, any)) continue;
+        }
         __syncwarp();
         const int m = stageTripleNeighbors(A, C, a, n, lane, 0, kAtmFastStaged,
                                            [&](int slot, int b, float x, float y, float z) {
@@ -644,7 +651,7 @@ __global__ void __launch_bounds__(32 * kAtmFastWarps, IX_TUNE_ATM_MIN_BLOCKS) kT
         __syncwarp();
         float fa[3] = {0.0f, 0.0f, 0.0f};
         float eSite = 0.0f;
-        siteTriples<DAMP, IMAGE>(S, A, C, pa, 0, 8, m, 0, m, lane, fa, eSite, visits);
+        siteTriples<DAMP, IMAGE, ALCH>(S, A, C, pa, 0, 8, m, 0, m, lane, fa, eSite, visits);
         addSiteForce(A, C, a, lane, fa);
         eAcc += (double)eSite;
     }
@@ -667,7 +674,7 @@ constexpr int kAtmWideParts = 8;
 // Energies go to energyPartials[partialsOffset + warp]: with a grid of one warp per unit, one slot per unit (unit =
 // site x kAtmWideParts + part).
 // `gate` (may be null): the kernel returns at once unless *gate is set (a list longer than the fast kernel takes).
-template <bool DAMP, bool IMAGE>
+template <bool DAMP, bool IMAGE, bool ALCH>
 __global__ void __launch_bounds__(32 * kAtmWarps) kTriplesWide(AtmBuffers A, AtmConfig C, int partialsOffset,
                                                                const int* gate) {
     if (gate && *(volatile const int*)gate == 0) return;
@@ -697,7 +704,7 @@ __global__ void __launch_bounds__(32 * kAtmWarps) kTriplesWide(AtmBuffers A, Atm
         const int m = stage(0, 0, kAtmMaxStaged);
         __syncwarp();
         if (m <= kAtmMaxStaged) {
-            siteTriples<DAMP, IMAGE>(S, A, C, pa, 8 * part, 8 * kAtmWideParts, m, 0, m, lane, fa, energy, visits);
+            siteTriples<DAMP, IMAGE, ALCH>(S, A, C, pa, 8 * part, 8 * kAtmWideParts, m, 0, m, lane, fa, energy, visits);
             eAcc += (double)energy;
         }
         else {
@@ -712,7 +719,7 @@ __global__ void __launch_bounds__(32 * kAtmWarps) kTriplesWide(AtmBuffers A, Atm
                     __syncwarp();
                     const int b0 = J == I ? 0 : kAtmChunk;
                     energy = 0.0f;
-                    siteTriples<DAMP, IMAGE>(S, A, C, pa, 8 * part, 8 * kAtmWideParts, cI, b0, b0 + cJ, lane, fa,
+                    siteTriples<DAMP, IMAGE, ALCH>(S, A, C, pa, 8 * part, 8 * kAtmWideParts, cI, b0, b0 + cJ, lane, fa,
                                              energy, visits);
                     eAcc += (double)energy;
                 }
@@ -729,24 +736,25 @@ __global__ void __launch_bounds__(32 * kAtmWarps) kTriplesWide(AtmBuffers A, Atm
 
 // The wide kernel where its grid is not empty, and the fast one.  The wide kernel mostly returns at once: it goes
 // first, while there is room on the SMs; behind the fast one it waited for the pair kernel's last blocks.  `before` (may
-// be null) is recorded ahead of the fast kernel.
-template <bool DAMP, bool IMAGE>
+// be null) is recorded ahead of the fast kernel.  ALCH: only the triples with an alchemical site.
+template <bool DAMP, bool IMAGE, bool ALCH>
 static void launchTriplesAs(const AtmBuffers& A, const AtmConfig& C, int fastBlocks, int wideBlocks, const int* gate,
                             cudaStream_t st, cudaEvent_t before) {
     if (wideBlocks > 0)
-        kTriplesWide<DAMP, IMAGE><<<wideBlocks, 32 * kAtmWarps,
+        kTriplesWide<DAMP, IMAGE, ALCH><<<wideBlocks, 32 * kAtmWarps,
                                     kAtmWarps * sizeof(TripleStorage<DAMP, kAtmMaxStaged>), st>>>(
             A, C, fastBlocks * kAtmFastWarps, gate);
     if (before) cudaEventRecord(before, st);
-    kTriplesFast<DAMP, IMAGE><<<fastBlocks, 32 * kAtmFastWarps, 0, st>>>(A, C);
+    kTriplesFast<DAMP, IMAGE, ALCH><<<fastBlocks, 32 * kAtmFastWarps, 0, st>>>(A, C);
 }
+template <bool ALCH>
 static void launchTriples(const AtmBuffers& A, const AtmConfig& C, int fastBlocks, int wideBlocks, const int* gate,
                           cudaStream_t st, cudaEvent_t before = nullptr) {
     const bool damp = C.useTangToennies || C.invCentroidRadius > 0.0f;
-    if (damp && C.imageBC) launchTriplesAs<true, true>(A, C, fastBlocks, wideBlocks, gate, st, before);
-    else if (damp) launchTriplesAs<true, false>(A, C, fastBlocks, wideBlocks, gate, st, before);
-    else if (C.imageBC) launchTriplesAs<false, true>(A, C, fastBlocks, wideBlocks, gate, st, before);
-    else launchTriplesAs<false, false>(A, C, fastBlocks, wideBlocks, gate, st, before);
+    if (damp && C.imageBC) launchTriplesAs<true, true, ALCH>(A, C, fastBlocks, wideBlocks, gate, st, before);
+    else if (damp) launchTriplesAs<true, false, ALCH>(A, C, fastBlocks, wideBlocks, gate, st, before);
+    else if (C.imageBC) launchTriplesAs<false, true, ALCH>(A, C, fastBlocks, wideBlocks, gate, st, before);
+    else launchTriplesAs<false, false, ALCH>(A, C, fastBlocks, wideBlocks, gate, st, before);
 }
 
 // Each particle of a site receives the site force divided by the number of particles

@@ -529,7 +529,7 @@ int enqueueBatch(ix_batch* b) {
         const AtmConfig& C = b->atmC;
         const int gS = (b->numSites + tpb - 1) / tpb;
         kSiteCentroids<<<gS, tpb, 0, st>>>(A, C, b->dPos);
-        launchTriples(A, C, b->atmFastBlocks, b->atmWideBlocks, nullptr, st);
+        launchTriples<false>(A, C, b->atmFastBlocks, b->atmWideBlocks, nullptr, st);
         kSpreadSiteForces<<<gS, tpb, 0, st>>>(A, C);
     }
     kFinalize<<<(b->numParticles + tpb - 1) / tpb, tpb, 0, st>>>(b->numParticles, L.np, L.slotOf, b->P.forceFixed,

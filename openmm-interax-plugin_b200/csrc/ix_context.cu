@@ -1332,6 +1332,43 @@ __global__ void kClearFlagIf(int* target, const int* gate) {
     if (*(volatile const int*)gate != 0) *target = 0;
 }
 
+// The configuration of the three-body kernels at the context's parameters, and the cell grid of the site-list search.
+static AtmConfig atmConfig(ix_ctx* ctx) {
+    AtmBuffers& A = ctx->A;
+    AtmConfig C{};
+    C.numSites = (int)ctx->siteParams.size() / 3;
+    C.periodic = ctx->atmPeriodic;
+    C.box = makeBox(ctx->box);
+    C.boxf = makeBoxF(C.box);
+    C.cutoff2 = (float)(ctx->atmCutoff * ctx->atmCutoff);
+    const double lc = ctx->atmCutoff + kSiteSkin;
+    C.listCutoff2 = (float)(lc * lc);
+    C.scale = (float)ctx->atmScale;
+    C.lambda = (float)lambdaOf(ctx, ctx->atmAlchName, ctx->atmAnyAlch);
+    C.useTangToennies = ctx->atmDamping == IX_TANG_TOENNIES;
+    C.twoBeta = (float)(2.0 * ctx->atmDampingScale);
+    C.invCentroidRadius = ctx->atmCentroidRadius > 0 ? (float)(1.0 / ctx->atmCentroidRadius) : 0.0f;
+    C.maxMove2 = 0.25f * kSiteSkin * kSiteSkin;
+    C.imageBC = tripleNeedsImages(C, ctx->atmCutoff);
+    // the wide kernel's energy slots start at zero (it runs only while some list is long)
+    C.zeroSlots = ctx->atmGridBlocks * kAtmWarps;
+    C.zeroOffset = ctx->atmFastBlocks * kAtmFastWarps;
+    // the cell grid of the list search in a rectangular periodic box with at least three cells per edge
+    A.cells.nc[0] = A.cells.nc[1] = A.cells.nc[2] = 0;
+    if (C.periodic && !C.box.triclinic && A.cells.cellStart) {
+        const double width = ctx->atmCutoff + kSiteSkin + 1e-3;   // room for the float rounding of the binning
+        const double len[3] = {ctx->box[0], ctx->box[4], ctx->box[8]};
+        int nc[3];
+        for (int d = 0; d < 3; d++) nc[d] = (int)std::floor(len[d] / width);
+        if (nc[0] >= 3 && nc[1] >= 3 && nc[2] >= 3 && (long long)nc[0] * nc[1] * nc[2] <= kSiteCellMax)
+            for (int d = 0; d < 3; d++) {
+                A.cells.nc[d] = nc[d];
+                A.cells.cellsPerNm[d] = (float)(nc[d] / len[d]);
+            }
+    }
+    return C;
+}
+
 // Systems of at most this many blocks of 32 particles take a thread block per tile (kPairTilesSmall).  Evaluations of the
 // pair terms back to back, a warp per tile and a block per tile: 24 atoms 37.1 and 36.6 us, 648 atoms 53.6 and 37.0,
 // 1,500 atoms 61.5 and 40.9, 3,000 atoms 74.1 and 56.3, 4,500 atoms 79.9 and 63.6, 7,800 atoms 87.4 and 86.1, 24,000
@@ -1382,39 +1419,9 @@ static int launchEvaluation(ix_ctx* ctx, unsigned terms, double* outForces, doub
     }
     if (doAtm) {
         AtmBuffers& A = ctx->A;
-        AtmConfig C{};
-        C.numSites = (int)ctx->siteParams.size() / 3;
-        C.periodic = ctx->atmPeriodic;
-        C.box = makeBox(ctx->box);
-        C.boxf = makeBoxF(C.box);
-        C.cutoff2 = (float)(ctx->atmCutoff * ctx->atmCutoff);
-        double lc = ctx->atmCutoff + kSiteSkin;
-        C.listCutoff2 = (float)(lc * lc);
-        C.scale = (float)ctx->atmScale;
-        C.lambda = (float)lambdaOf(ctx, ctx->atmAlchName, ctx->atmAnyAlch);
-        C.useTangToennies = ctx->atmDamping == IX_TANG_TOENNIES;
-        C.twoBeta = (float)(2.0 * ctx->atmDampingScale);
-        C.invCentroidRadius = ctx->atmCentroidRadius > 0 ? (float)(1.0 / ctx->atmCentroidRadius) : 0.0f;
-        C.maxMove2 = 0.25f * kSiteSkin * kSiteSkin;
-        C.imageBC = tripleNeedsImages(C, ctx->atmCutoff);
+        const AtmConfig C = atmConfig(ctx);
         const int tpb = 256;
         const int gS = (C.numSites + 63) / 64;   // 64-thread blocks, so that a few thousand sites reach every SM
-        // the wide kernel's energy slots start at zero (it runs only while some list is long)
-        C.zeroSlots = ctx->atmGridBlocks * kAtmWarps;
-        C.zeroOffset = ctx->atmFastBlocks * kAtmFastWarps;
-        // the cell grid of the list search in a rectangular periodic box with at least three cells per edge
-        A.cells.nc[0] = A.cells.nc[1] = A.cells.nc[2] = 0;
-        if (C.periodic && !C.box.triclinic && A.cells.cellStart) {
-            const double width = ctx->atmCutoff + kSiteSkin + 1e-3;   // room for the float rounding of the binning
-            const double len[3] = {ctx->box[0], ctx->box[4], ctx->box[8]};
-            int nc[3];
-            for (int d = 0; d < 3; d++) nc[d] = (int)std::floor(len[d] / width);
-            if (nc[0] >= 3 && nc[1] >= 3 && nc[2] >= 3 && (long long)nc[0] * nc[1] * nc[2] <= kSiteCellMax)
-                for (int d = 0; d < 3; d++) {
-                    A.cells.nc[d] = nc[d];
-                    A.cells.cellsPerNm[d] = (float)(nc[d] / len[d]);
-                }
-        }
         kSiteCentroids<<<gS, 64, 0, sa>>>(A, C, ctx->dPos);
         // site list rebuild when the centroid kernel set the flag: these kernels return at once otherwise.  The
         // long-list flag is recomputed with the lists (the cell sort clears it)
@@ -1430,7 +1437,7 @@ static int launchEvaluation(ix_ctx* ctx, unsigned terms, double* outForces, doub
         recordTiming(ctx, 2, sa);
         // the sites whose lists are too long for the fast kernel go to the wide one, which returns at once when there
         // are none and goes first
-        launchTriples(A, C, ctx->atmFastBlocks, ctx->atmGridBlocks, A.flag + 2, sa, fork ? ctx->evFork : nullptr);
+        launchTriples<false>(A, C, ctx->atmFastBlocks, ctx->atmGridBlocks, A.flag + 2, sa, fork ? ctx->evFork : nullptr);
         ctx->launches += 5;
         recordTiming(ctx, 3, sa);
         ctx->evAtm = ctx->profiling;
@@ -1669,20 +1676,30 @@ static void sharedSplit() {
     most(kPairTiles<true, false, false>);
     most(kPairTiles<false, true, false>);
     most(kPairTiles<false, false, false>);
+    most(kPairWindows<true>);
+    most(kPairWindows<false>);
     most(kPairTilesSmall<true, true, true>);
     most(kPairTilesSmall<true, false, true>);
     most(kPairTilesSmall<true, true, false>);
     most(kPairTilesSmall<true, false, false>);
     most(kPairTilesSmall<false, true, false>);
     most(kPairTilesSmall<false, false, false>);
-    most(kTriplesFast<false, false>);
-    most(kTriplesFast<false, true>);
-    most(kTriplesFast<true, false>);
-    most(kTriplesFast<true, true>);
-    most(kTriplesWide<false, false>);
-    most(kTriplesWide<false, true>);
-    most(kTriplesWide<true, false>);
-    most(kTriplesWide<true, true>);
+    most(kTriplesFast<false, false, false>);
+    most(kTriplesFast<false, false, true>);
+    most(kTriplesFast<false, true, false>);
+    most(kTriplesFast<false, true, true>);
+    most(kTriplesFast<true, false, false>);
+    most(kTriplesFast<true, false, true>);
+    most(kTriplesFast<true, true, false>);
+    most(kTriplesFast<true, true, true>);
+    most(kTriplesWide<false, false, false>);
+    most(kTriplesWide<false, false, true>);
+    most(kTriplesWide<false, true, false>);
+    most(kTriplesWide<false, true, true>);
+    most(kTriplesWide<true, false, false>);
+    most(kTriplesWide<true, false, true>);
+    most(kTriplesWide<true, true, false>);
+    most(kTriplesWide<true, true, true>);
     most(kSiteCentroids);
     most(kSiteNeighbors);
     most(kSiteNeighborsCells);
@@ -2554,19 +2571,41 @@ __global__ void kWindowForces(size_t n3, int num_windows, const double* __restri
     }
 }
 
-// out[w] += base + a0 + lambda_w (a1 - a0) (a0, a1 may be null): the λ-independent and linear parts of the windows'
-// forces added to their alchemical-pair parts.
-__global__ void kWindowCombine(size_t n3, int num_windows, const double* __restrict__ lambdas,
-                               const double* __restrict__ base, const double* __restrict__ a0,
-                               const double* __restrict__ a1, double* __restrict__ out) {
-    for (int w = blockIdx.y; w < num_windows; w += gridDim.y) {
-        const double lam = lambdas[w];
-        double* o = out + (size_t)w * n3;
-        for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < n3; k += (size_t)gridDim.x * blockDim.x) {
-            double v = base[k];
-            if (a0) v += fma(lam, a1[k] - a0[k], a0[k]);
-            o[k] += v;
+// out[w] = base + lambda_w slope + own_w: the forces of each window from those at 0, the slope of the terms linear in
+// the parameter (may be null) and the window's own alchemical pairs (fixed point in sorted slots, 3 x np per window; may
+// be null).
+__global__ void kWindowResults(int n, int np, int num_windows, const double* __restrict__ lambdas,
+                               const double* __restrict__ base, const double* __restrict__ slope,
+                               const long long* __restrict__ own, const int* __restrict__ slotOf,
+                               double* __restrict__ out) {
+    const size_t n3 = 3 * (size_t)n;
+    for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < n3; k += (size_t)gridDim.x * blockDim.x) {
+        const double f0 = base[k], f1 = slope ? slope[k] : 0.0;
+        const long long* mine = own ? own + k % 3 * np + slotOf[k / 3] : nullptr;
+#pragma unroll 4
+        for (int w = blockIdx.y; w < num_windows; w += gridDim.y) {
+            double v = fma(lambdas[w], f1, f0);
+            if (mine) v += (double)mine[(size_t)w * 3 * np] * (1.0 / kFixedScale);
+            out[w * n3 + k] = v;
         }
+    }
+}
+
+// Each window's energies of its alchemical pairs: a block per window adds the sums of its blocks in a fixed order.
+__global__ void __launch_bounds__(128) kWindowEnergies(int numBlocks, const double* blockEnergy, double* out) {
+    __shared__ double sums[4][3];
+    const double* e = blockEnergy + (size_t)blockIdx.x * 3 * numBlocks;
+    double s[3] = {0.0, 0.0, 0.0};
+    for (int t = threadIdx.x; t < numBlocks; t += 128)
+        for (int k = 0; k < 3; k++) s[k] += e[3 * (size_t)t + k];
+    for (int k = 0; k < 3; k++) {
+        s[k] = warpSumD(s[k]);
+        if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5][k] = s[k];
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        const int k = threadIdx.x;
+        out[3 * blockIdx.x + k] = (sums[0][k] + sums[1][k]) + (sums[2][k] + sums[3][k]);
     }
 }
 
@@ -2596,131 +2635,216 @@ static LaunchGraph& windowGraph(ix_ctx* ctx, unsigned terms, double value) {
     return ctx->graphWindows[ctx->windowNext++ % ctx->graphWindows.size()];
 }
 
-// One pass over the windows (see computeWindows).  redo: a neighbor list overflowed after the first window and was
-// grown; the pass must be repeated.
-// Soft-core windows when every pair term uses the window parameter with the same alchemical particles: the pair terms
-// are evaluated once at 0, where the alchemical pairs contribute nothing (their scale is the parameter), the
-// three-body term at 0 and 1 (it is linear), and each window adds only its alchemical pairs: the pair kernel over the
-// tiles that hold an alchemical particle, keeping the pairs with exactly one (the same kernel and terms as a full
-// evaluation at that value).  The long-range correction's alchemical part joins each window's energy.
-static int softcoreWindows(ix_ctx* ctx, const std::string& name, int num_windows, const double* values,
-                           double* energies, double* d_forces) {
+// The slope of the terms linear in the window parameter, as FP64 forces: those of the alchemical triples (in the site
+// forces) and, when `pairs`, of the alchemical pairs (in P.forceFixed); and the triples' energy and count.
+static int windowSlope(ix_ctx* ctx, bool atm, bool pairs, double* dSlope, double* dEnergy) {
+    FinishForces F{};
+    F.n = ctx->n;
+    F.np = ctx->L.np;
+    F.slotOf = ctx->L.slotOf;
+    F.pairForce = pairs ? ctx->P.forceFixed : nullptr;
+    F.siteForce = atm ? ctx->A.siteForce : nullptr;
+    F.numSites = (int)ctx->siteParams.size() / 3;
+    F.siteOffsets = ctx->A.siteOffsets;
+    F.particleSiteStart = ctx->dParticleSiteStart;
+    F.particleSites = ctx->dParticleSites;
+    F.outForces = dSlope;
+    F.blocks = (ctx->n + 255) / 256;
+    EnergyReduction R{nullptr, nullptr, 0, atm ? ctx->dAtmPartials : nullptr, (int)atmPartialCount(ctx), 0.0, dEnergy,
+                      ctx->dEnergyBlocks, ctx->dReduceTicket, atm ? ctx->dCounts : nullptr, nullptr, nullptr, nullptr};
+    kFinish<<<F.blocks + kReduceBlocks, 256, 0, ctx->stream>>>(F, R);
+    ctx->launches += 1;
+    IX_CUDA(ctx, cudaGetLastError());
+    return IX_OK;
+}
+
+// Buffers of alchemicalWindows.
+struct WindowBuffers {
+    double *lambda, *slope, *report, *blockEnergy;
+    long long* own;
+    unsigned char* marks;
+    PairTermConfig* configs;
+    unsigned long long* pairScratch;
+    int group, blocks;           // windows evaluated together, thread blocks of each
+};
+static const char* const kWindowBufferNames[] = {"windowSlope", "windowReport",  "windowBlockEnergy", "windowOwn",
+                                                 "windowTileMarks", "windowConfigs", "windowPairScratch"};
+
+static int windowBuffers(ix_ctx* ctx, int num_windows, int passes, bool softcore, bool slope, WindowBuffers& B) {
+    const size_t np = (size_t)ctx->L.np;
+    B = WindowBuffers{};
+    // windows evaluated together: their force rows take 512 MB at most
+    B.group = std::max(1, std::min({passes, 64, (int)((size_t(512) << 20) / (24 * std::max<size_t>(np, 1)))}));
+    // eight blocks an SM over all of them (what is resident; 16 and 32 measured the same), 64 a window at least
+    B.blocks = std::max(1, std::min(ctx->L.tileCap, std::max(64, ctx->numSMs * 8 / B.group)));
+    IX_TRY(deviceAlloc(ctx, "windowLambda", (size_t)num_windows, &B.lambda));
+    IX_TRY(deviceAlloc(ctx, "windowReport", 6 + 3 * (size_t)passes, &B.report));
+    if (slope) IX_TRY(deviceAlloc(ctx, "windowSlope", 3 * (size_t)ctx->n, &B.slope));
+    if (!passes) return IX_OK;
+    IX_TRY(deviceAlloc(ctx, "windowBlockEnergy", 3 * (size_t)B.blocks * B.group, &B.blockEnergy));
+    if (softcore) IX_TRY(deviceAlloc(ctx, "windowOwn", 3 * np * B.group, &B.own));
+    IX_TRY(deviceAlloc(ctx, "windowTileMarks", (size_t)ctx->L.tileCap, &B.marks));
+    IX_TRY(deviceAlloc(ctx, "windowConfigs", (size_t)passes, &B.configs));
+    IX_TRY(deviceAlloc(ctx, "windowPairScratch", 1, &B.pairScratch));
+    return IX_OK;
+}
+
+// The windows by their alchemical part, when the pair terms that depend on the parameter (`dependent`) have the same
+// alchemical particles: one evaluation of everything at 0, where their alchemical pairs and triples contribute nothing
+// (their scale is the parameter), and the alchemical pairs and triples alone.  The triples are linear in the parameter
+// and are evaluated once, at 1, and so are the pairs without a soft core; with one they are evaluated once per window,
+// all windows in one launch.  The pair kernel takes the tiles that hold an alchemical particle and keeps the pairs with
+// exactly one, the triple kernel keeps the triples with an alchemical site.  The long-range correction's alchemical part
+// joins each window's energy. Before, the linear case was two whole
+// evaluations and the other a launch and a finish per window, between evaluations of the pairs at 0 and of the triples
+// at 0 and 1: 16 windows of a 96,000-atom box 1197 us and 748 now, 12 soft-core windows of 12,297 atoms 704 and 211.
+// What is left is the evaluation at 0 (590 and 116 us) and, behind it, the alchemical triples (66 and 28 us, most of it
+// reading the lists that hold no alchemical site) or the alchemical pairs (19 and 43 us).
+// fits: false when the buffers did not fit (nothing was done).  redo: as for windowsPass.
+static int alchemicalWindows(ix_ctx* ctx, const std::string& name, unsigned dependent, bool softcore, int num_windows,
+                             const double* values, double* energies, double* d_forces, bool& fits, bool& redo) {
     const size_t n3 = 3 * (size_t)ctx->n;
-    const unsigned terms = selectedTerms(ctx, -1), pairTerms = terms & 7u;
-    const bool atmLinear = (terms & 8u) && ctx->atmAnyAlch && ctx->atmAlchName == name;
+    const unsigned terms = selectedTerms(ctx, -1);
+    const bool atm = (terms & 8u) && ctx->atmAnyAlch && ctx->atmAlchName == name;
+    const int passes = !dependent ? 0 : (softcore ? num_windows : 1);
+    const bool slope = atm || (passes && !softcore);
+    cudaStream_t st = ctx->stream;
     int bit = 0;
     for (int t = 0; t < 3 && !bit; t++)
-        if ((pairTerms >> t) & 1u) bit = 1 << t;
-    double *dBase = nullptr, *dA0 = nullptr, *dA1 = nullptr, *dLambda = nullptr, *dWinEnergy = nullptr;
-    double* dAlchEnergy = nullptr;
-    int* dAlchCount = nullptr;
-    unsigned long long* dPairScratch = nullptr;
-    IX_TRY(deviceAlloc(ctx, "windowLambda", (size_t)num_windows, &dLambda));
-    IX_TRY(deviceAlloc(ctx, "windowEnergy", 4 * (size_t)num_windows, &dWinEnergy));
-    IX_TRY(deviceAlloc(ctx, "windowAlchCount", 1, &dAlchCount));
-    IX_TRY(deviceAlloc(ctx, "windowPairScratch", 1, &dPairScratch));
-    if (d_forces) {
-        IX_TRY(deviceAlloc(ctx, "windowBase", n3, &dBase));
-        if (terms & 8u) IX_TRY(deviceAlloc(ctx, "windowA0", n3, &dA0));
-        if (atmLinear) IX_TRY(deviceAlloc(ctx, "windowSlope", n3, &dA1));
+        if ((dependent >> t) & 1u) bit = 1 << t;
+    IX_TRY(prepare(ctx, terms));
+    WindowBuffers B;
+    fits = windowBuffers(ctx, num_windows, passes, softcore, slope && d_forces, B) == IX_OK;
+    if (!fits) {
+        cudaGetLastError();
+        for (const char* buffer : kWindowBufferNames) {
+            arenaFree(ctx->arena, ctx->buffers[buffer].p);
+            ctx->buffers.erase(buffer);
+        }
+        bumpVersion(ctx);
+        return IX_OK;
     }
-    // the pair terms at 0 (the lists are built for these positions here), the three-body term at 0 and 1
-    double eP[4], eA0[4] = {0, 0, 0, 0}, eA1[4] = {0, 0, 0, 0};
+    // everything at 0: forces in dOutForces, energies and counts in the status block, the lists built for these positions
+    double e0[4] = {0, 0, 0, 0};
+    long long pairs = 0, triples = 0;
     ctx->parameters[name] = 0.0;
-    IX_TRY(evaluateResident(ctx, pairTerms, eP, &windowGraph(ctx, pairTerms, 0.0), 0.0));
-    const long long pairs = ctx->lastPairs;
-    if (d_forces)
-        IX_CUDA(ctx, cudaMemcpyAsync(dBase, ctx->dOutForces, n3 * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
-    long long triples = 0;
-    if (terms & 8u) {
-        IX_TRY(evaluateResident(ctx, 8u, eA0, &windowGraph(ctx, 8u, 0.0), 0.0));
+    if (!ctx->hostStatus) ctx->hostStatus = pinnedSlots().take();
+    unsigned char* hs = ctx->hostStatus;
+    LaunchGraph& graph = windowGraph(ctx, terms, 0.0);
+    if (hs) {
+        IX_TRY(enqueueResident(ctx, terms, graph, 0.0));
+        IX_CUDA(ctx, cudaMemcpyAsync(hs, ctx->dFlags, kStatusBytes, cudaMemcpyDeviceToHost, st));
+    }
+    else {
+        IX_TRY(evaluateResident(ctx, terms, e0, &graph, 0.0));
+        pairs = ctx->lastPairs;
         triples = ctx->lastTriples;
-        if (d_forces)
-            IX_CUDA(ctx, cudaMemcpyAsync(dA0, ctx->dOutForces, n3 * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
-        if (atmLinear) {
-            ctx->parameters[name] = 1.0;
-            IX_TRY(evaluateResident(ctx, 8u, eA1, &windowGraph(ctx, 8u, 1.0), 1.0));
-            if (d_forces)
-                IX_CUDA(ctx, cudaMemcpyAsync(dA1, ctx->dOutForces, n3 * sizeof(double), cudaMemcpyDeviceToDevice,
-                                             ctx->stream));
-        }
-        else std::memcpy(eA1, eA0, sizeof(eA0));
+        IX_TRY(windowBuffers(ctx, num_windows, passes, softcore, slope && d_forces, B));   // the tile list may have grown
     }
-    // the tiles that hold an alchemical particle, in tile order
-    int numTiles = 0;
-    IX_CUDA(ctx, cudaMemcpy(&numTiles, ctx->L.numTiles, sizeof(int), cudaMemcpyDeviceToHost));
-    numTiles = std::min(numTiles, ctx->tileCap);
-    unsigned char* dMarks = nullptr;
-    IX_TRY(deviceAlloc(ctx, "windowTileMarks", std::max(numTiles, 1), &dMarks));
-    kMarkAlchemicalTiles<<<ctx->numSMs * 8, 256, 0, ctx->stream>>>(ctx->L, ctx->P.flags, bit, dMarks);
-    ctx->launches += 1;
-    std::vector<unsigned char> marks(std::max(numTiles, 1));
-    IX_CUDA(ctx, cudaMemcpyAsync(marks.data(), dMarks, numTiles, cudaMemcpyDeviceToHost, ctx->stream));
-    IX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    std::vector<int> tiles;
-    for (int t = 0; t < numTiles; t++)
-        if (marks[t]) tiles.push_back(t);
-    const int numTasks = (int)tiles.size();
-    int* dTiles = nullptr;
-    IX_TRY(deviceAlloc(ctx, "windowTiles", std::max(numTasks, 1), &dTiles));
-    IX_TRY(deviceAlloc(ctx, "windowAlchEnergy", 3 * (size_t)std::max(numTasks, 1), &dAlchEnergy));
-    if (numTasks) IX_TRY(stageCopy(ctx, dTiles, tiles.data(), tiles.size() * sizeof(int)));
-    IX_TRY(stageCopy(ctx, dAlchCount, &numTasks, sizeof(int)));
-    // each window: its alchemical pairs, then their forces and energies
-    const PairTerm& D = ctx->term[0];
-    const double volume = ctx->box[0] * ctx->box[4] * ctx->box[8];
-    const int n = ctx->n;
-    for (int w = 0; w < num_windows; w++) {
-        ctx->parameters[name] = values[w];
-        PairTermConfig C = pairConfig(ctx, pairTerms);
-        C.alchOnlyBit = bit;
-        PairBuffers P = ctx->P;
-        P.taskTiles = dTiles;
-        P.numTasks = numTasks;
-        P.taskEnergy = dAlchEnergy;
-        P.pairCount = dPairScratch;
-        const bool table = P.coef != nullptr && C.overlapMethod[1] == 0 && C.overlapMethod[2] == 0;
-        if (numTasks) {
-            if (table) kPairTiles<false, true><<<ctx->pairGridBlocks, 32 * kPairWarps, 0, ctx->stream>>>(ctx->L, P, C);
-            else kPairTiles<false, false><<<ctx->pairGridBlocks, 32 * kPairWarps, 0, ctx->stream>>>(ctx->L, P, C);
+    IX_TRY(stageCopy(ctx, B.lambda, values, num_windows * sizeof(double)));
+    ctx->parameters[name] = 1.0;
+    // the alchemical triples at 1, beside the pairs
+    const bool fork = atm && passes && !ctx->serialize;
+    if (atm) {
+        cudaStream_t sa = fork ? ctx->stream2 : st;
+        if (fork) {
+            IX_CUDA(ctx, cudaEventRecord(ctx->evFork, st));
+            IX_CUDA(ctx, cudaStreamWaitEvent(sa, ctx->evFork, 0));
         }
-        FinishForces F{};
-        F.n = n;
-        F.np = ctx->L.np;
-        F.slotOf = ctx->L.slotOf;
-        F.pairForce = ctx->P.forceFixed;
-        F.outForces = d_forces ? d_forces + (size_t)w * n3 : nullptr;
-        F.blocks = (n + 255) / 256;
-        const double lrc = (D.present && (pairTerms & 1u) && D.lrcAlchCoef != 0) ? values[w] * D.lrcAlchCoef / volume
-                                                                                 : 0.0;
-        EnergyReduction R{dAlchEnergy, dAlchCount, std::max(numTasks, 1), nullptr, 0, lrc, dWinEnergy + 4 * (size_t)w,
-                          ctx->dEnergyBlocks, ctx->dReduceTicket, nullptr, ctx->L.taskCounter, nullptr, nullptr};
-        kFinish<<<F.blocks + kReduceBlocks, 256, 0, ctx->stream>>>(F, R);
-        ctx->launches += numTasks ? 2 : 1;
-        IX_CUDA(ctx, cudaGetLastError());
+        const AtmConfig C = atmConfig(ctx);
+        kSiteCentroids<<<(C.numSites + 63) / 64, 64, 0, sa>>>(ctx->A, C, ctx->dPos);   // clears the site forces
+        launchTriples<true>(ctx->A, C, ctx->atmFastBlocks, ctx->atmGridBlocks, ctx->A.flag + 2, sa);
+        ctx->launches += 3;
+        if (fork) IX_CUDA(ctx, cudaEventRecord(ctx->evJoin, sa));
     }
-    std::vector<double> alch(4 * (size_t)num_windows);
-    IX_CUDA(ctx, cudaMemcpyAsync(alch.data(), dWinEnergy, alch.size() * sizeof(double), cudaMemcpyDeviceToHost,
-                                 ctx->stream));
-    if (d_forces) {
-        IX_TRY(stageCopy(ctx, dLambda, values, num_windows * sizeof(double)));
-        const unsigned bx = (unsigned)std::max<size_t>(std::min<size_t>((n3 + 255) / 256, 1184), 1);
-        const dim3 grid(bx, (unsigned)std::min(num_windows, 65535));
-        kWindowCombine<<<grid, 256, 0, ctx->stream>>>(n3, num_windows, dLambda, dBase, dA0, atmLinear ? dA1 : dA0,
-                                                      d_forces);
+    const unsigned bx = (unsigned)std::max<size_t>(std::min<size_t>((n3 + 255) / 256, 1184), 1);
+    // a small system's windows are spread over more blocks
+    auto results = [&](int count) { return dim3(bx, std::max(1u, std::min((unsigned)count, 592u / bx))); };
+    PairBuffers P = ctx->P;
+    bool table = P.coef != nullptr;
+    if (passes) {
+        std::vector<PairTermConfig> configs(passes);
+        for (int w = 0; w < passes; w++) {
+            ctx->parameters[name] = softcore ? values[w] : 1.0;
+            configs[w] = pairConfig(ctx, dependent);
+            configs[w].alchOnlyBit = bit;
+            configs[w].coefShared = 0;
+        }
+        for (int t = 1; t < 3; t++)
+            if ((dependent >> t) & 1u) table = table && configs[0].overlapMethod[t] == 0;
+        IX_TRY(stageCopy(ctx, B.configs, configs.data(), configs.size() * sizeof(PairTermConfig)));
+        kMarkAlchemicalTiles<<<ctx->numSMs * 8, 256, 0, st>>>(ctx->L, ctx->P.flags, bit, B.marks);
         ctx->launches += 1;
-        IX_CUDA(ctx, cudaGetLastError());
+        if (softcore) P.forceFixed = B.own;
+        P.taskEnergy = B.blockEnergy;
+        P.pairCount = B.pairScratch;
+        P.coefShared = 0;
     }
-    IX_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    auto joinedSlope = [&]() {
+        if (fork) IX_CUDA(ctx, cudaStreamWaitEvent(st, ctx->evJoin, 0));
+        IX_TRY(windowSlope(ctx, atm, passes && !softcore, B.slope, B.report));
+        // the count of the alchemical triples beside their energy
+        if (atm)
+            IX_CUDA(ctx, cudaMemcpyAsync(B.report + 4, ctx->dCounts + 2, 16, cudaMemcpyDeviceToDevice, st));
+        return (int)IX_OK;
+    };
+    for (int w0 = 0; w0 < passes; w0 += B.group) {
+        const int count = std::min(B.group, passes - w0);
+        const dim3 grid((unsigned)B.blocks, (unsigned)count);
+        if (softcore) IX_CUDA(ctx, cudaMemsetAsync(B.own, 0, 3 * (size_t)ctx->L.np * count * sizeof(long long), st));
+        if (table) kPairWindows<true><<<grid, kTileThreads, 0, st>>>(ctx->L, P, B.configs + w0, B.marks);
+        else kPairWindows<false><<<grid, kTileThreads, 0, st>>>(ctx->L, P, B.configs + w0, B.marks);
+        kWindowEnergies<<<count, 128, 0, st>>>(B.blocks, B.blockEnergy, B.report + 6 + 3 * (size_t)w0);
+        ctx->launches += 2;
+        if (w0 == 0 && slope) IX_TRY(joinedSlope());
+        if (d_forces && softcore) {
+            kWindowResults<<<results(count), 256, 0, st>>>(ctx->n, ctx->L.np, count, B.lambda + w0, ctx->dOutForces,
+                                                           B.slope, B.own, ctx->L.slotOf, d_forces + w0 * n3);
+            ctx->launches += 1;
+        }
+    }
+    if (!passes && slope) IX_TRY(joinedSlope());
+    if (d_forces && !(passes && softcore)) {
+        kWindowResults<<<results(num_windows), 256, 0, st>>>(ctx->n, ctx->L.np, num_windows, B.lambda, ctx->dOutForces,
+                                                             B.slope, nullptr, nullptr, d_forces);
+        ctx->launches += 1;
+    }
+    IX_CUDA(ctx, cudaGetLastError());
+    std::vector<double> report(6 + 3 * (size_t)passes, 0.0);
+    IX_CUDA(ctx, cudaMemcpyAsync(report.data(), B.report, report.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+    IX_CUDA(ctx, cudaStreamSynchronize(st));
+    if (hs) {
+        IX_TRY(checkOverflowFlags(ctx, terms, reinterpret_cast<const int*>(hs), redo));
+        if (redo) return IX_OK;
+        unsigned long long c[2];
+        std::memcpy(e0, hs + 32, sizeof(e0));
+        std::memcpy(c, hs + 64 + 2 * sizeof(unsigned long long), sizeof(c));
+        for (int t = 0; t < 4; t++)
+            if (!((terms >> t) & 1u)) e0[t] = 0.0;
+        pairs = (terms & 7u) ? (long long)c[0] : 0;
+        triples = (terms & 8u) ? (long long)c[1] : 0;
+    }
+    const PairTerm& D = ctx->term[0];
+    const double lrc = (dependent & 1u) && D.lrcAlchCoef != 0 ? D.lrcAlchCoef / (ctx->box[0] * ctx->box[4] * ctx->box[8]) : 0.0;
     for (int w = 0; w < num_windows; w++) {
-        for (int k = 0; k < 3; k++) energies[4 * w + k] = eP[k] + alch[4 * (size_t)w + k];
-        energies[4 * w + 3] = eA0[3] + values[w] * (eA1[3] - eA0[3]);
+        const double* own = report.data() + 6 + (softcore ? 3 * (size_t)w : 0);
+        for (int k = 0; k < 3; k++) energies[4 * w + k] = e0[k] + (passes ? (softcore ? own[k] : values[w] * own[k]) : 0.0);
+        energies[4 * w] += values[w] * lrc;
+        energies[4 * w + 3] = e0[3] + (atm ? values[w] * report[3] : 0.0);
+    }
+    if (atm && !softcore) {
+        // without a soft core the count is that of the parameter at 1
+        unsigned long long alchemical;
+        std::memcpy(&alchemical, &report[5], sizeof(alchemical));
+        triples += (long long)alchemical;
     }
     ctx->lastPairs = pairs;
     ctx->lastTriples = triples;
     return IX_OK;
 }
 
+// One pass over the windows (see computeWindows).  redo: a neighbor list overflowed and was grown; the pass must be
+// repeated.
 static int windowsPass(ix_ctx* ctx, const std::string& name, int num_windows, const double* values, double* energies,
                        double* d_forces, bool& redo) {
     redo = false;
@@ -2732,18 +2856,25 @@ static int windowsPass(ix_ctx* ctx, const std::string& name, int num_windows, co
         pairNonlinear = pairNonlinear || (T.present && T.anyAlch && T.alchName == name && T.softcoreRadius > 0);
     }
     const unsigned pairTerms = terms & 7u;
-    if (pairNonlinear) {
-        // every pair term on the window parameter with a soft core and the same alchemical particles: only the
-        // alchemical pairs are evaluated per window
-        bool same = true;
-        const PairTerm* first = nullptr;
-        for (int t = 0; t < 3 && same; t++) {
-            const PairTerm& T = ctx->term[t];
-            if (!((pairTerms >> t) & 1u)) continue;
-            same = T.anyAlch && T.alchName == name && T.softcoreRadius > 0 && (!first || T.alch == first->alch);
-            if (!first) first = &T;
+    // when the pair terms on the window parameter share their alchemical particles and all or none have a soft core, only
+    // their alchemical part is evaluated beside everything at 0
+    unsigned dependent = 0;
+    bool same = terms != 0, softcore = false;
+    const PairTerm* first = nullptr;
+    for (int t = 0; t < 3; t++) {
+        const PairTerm& T = ctx->term[t];
+        if (!((pairTerms >> t) & 1u) || !T.anyAlch || T.alchName != name) continue;
+        dependent |= 1u << t;
+        if (!first) {
+            first = &T;
+            softcore = T.softcoreRadius > 0;
         }
-        if (same) return softcoreWindows(ctx, name, num_windows, values, energies, d_forces);
+        same = same && T.alch == first->alch && (T.softcoreRadius > 0) == softcore;
+    }
+    if (same) {
+        bool fits = true;
+        IX_TRY(alchemicalWindows(ctx, name, dependent, softcore, num_windows, values, energies, d_forces, fits, redo));
+        if (fits) return IX_OK;
     }
     const unsigned linearTerms = pairNonlinear ? (terms & 8u) : terms;
     double *dLin0 = nullptr, *dLin1 = nullptr, *dLambda = nullptr, *dWinEnergy = nullptr;
@@ -2817,11 +2948,13 @@ static int windowsPass(ix_ctx* ctx, const std::string& name, int num_windows, co
 }
 
 // The context evaluated at several values of one alchemical parameter, forces left on the device (d_forces, n x 3
-// per window, or null).  Terms whose alchemical scaling is linear in the parameter (pairs with exactly one
-// alchemical particle and no soft core, triples with an alchemical site, the long-range correction coef + lambda
-// alchCoef) are evaluated at 0 and 1 and interpolated for every window by kWindowForces; pair terms with a soft core
-// (the alchemical pairs' distances depend on the parameter) are evaluated at every window, back to back.  Each value
-// has its own cached graph, so repeated window sets replay without capturing.  The parameter keeps its value.
+// per window, or null): by the terms' alchemical part (alchemicalWindows) where the pair terms on the parameter share
+// their alchemical particles.  Elsewhere, and where its buffers do not fit, the terms whose scaling is linear in the
+// parameter (pairs with exactly one alchemical particle and no soft core, triples with an alchemical site, the
+// long-range correction coef + lambda alchCoef) are evaluated at 0 and 1 and interpolated for every window by
+// kWindowForces, and pair terms with a soft core (the alchemical pairs' distances depend on the parameter) are evaluated
+// at every window, back to back.  Each value has its own cached graph, so repeated window sets replay without capturing.
+// The parameter keeps its value.
 static int computeWindows(ix_ctx* ctx, const char* parameter, int num_windows, const double* values, double* energies,
                           double* d_forces) {
     NvtxRange nvtxRange("ix_compute_windows");
@@ -2837,7 +2970,7 @@ static int computeWindows(ix_ctx* ctx, const char* parameter, int num_windows, c
     const bool hadValue = saved != ctx->parameters.end();
     const double oldValue = hadValue ? saved->second : 0.0;
     int rc = IX_OK;
-    for (int attempt = 0; attempt < 3; attempt++) {
+    for (int attempt = 0; attempt < 4; attempt++) {
         bool redo = false;
         rc = windowsPass(ctx, name, num_windows, values, energies, d_forces, redo);
         if (rc != IX_OK || !redo) break;
@@ -3239,7 +3372,7 @@ int ix_three_body_noalloc(int num_particles, const double* d_positions, const do
         kSiteNeighbors<<<(num_sites * 32 + tpb - 1) / tpb, tpb, 0, st>>>(A, C);
         const int fastBlocks = (num_sites + kAtmFastWarps - 1) / kAtmFastWarps;
         const int blocks = std::max(1, std::min((num_sites + kAtmWarps - 1) / kAtmWarps, kNoAllocBlocks));
-        launchTriples(A, C, fastBlocks, blocks, nullptr, st);
+        launchTriples<false>(A, C, fastBlocks, blocks, nullptr, st);
         kNoAllocSpread<<<(num_sites + tpb - 1) / tpb, tpb, 0, st>>>(S, num_particles, num_sites, d_site_offsets,
                                                                    d_site_particles);
         kReduceEnergies<<<1, 256, 0, st>>>(nullptr, nullptr, 0, S->energyPartials,

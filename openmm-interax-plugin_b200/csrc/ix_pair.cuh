@@ -51,7 +51,7 @@ struct PairTermConfig {
     double cutoff;
     Box box;
     BoxFF boxff;
-    int alchOnlyBit;             // nonzero: only the pairs with exactly one particle carrying this alchemical flag bit
+    int alchOnlyBit;             // kPairWindows: only the pairs with exactly one particle carrying this alchemical flag bit
     int coefShared;              // the class-pair table is read from its copy in shared memory
 };
 
@@ -67,8 +67,6 @@ struct PairBuffers {
     const PairCoef* coef;        // class-pair coefficients (numClasses^2), or null
     int numClasses;
     int coefShared;              // the launch gives dynamic shared memory for the table: it is staged there
-    const int* taskTiles;        // null: every tile is a task; else the tiles of the tasks (energies go to task slots)
-    int numTasks;
 };
 
 // Bits 8..15 of a particle's flags hold its parameter class when the class tables are in use.
@@ -477,7 +475,7 @@ __global__ void __launch_bounds__(32 * kPairWarps, IX_TUNE_PAIR_MIN_BLOCKS) kPai
         __syncthreads();
         coef = reinterpret_cast<const PairCoef*>(pairShared);
     }
-    const int numTasks = P.taskTiles ? P.numTasks : min(*L.numTiles, L.tileCap);
+    const int numTasks = min(*L.numTiles, L.tileCap);
     // the schedule: the buckets from the fullest tiles down, lane b the end of its bucket in the sequence of tasks
     int bucketEnd = 0;
     if (L.bucketCount) {
@@ -496,8 +494,7 @@ __global__ void __launch_bounds__(32 * kPairWarps, IX_TUNE_PAIR_MIN_BLOCKS) kPai
         task = __shfl_sync(0xffffffffu, task, 0);
         if (task >= numTasks) break;
         int t;
-        if (P.taskTiles) t = P.taskTiles[task];
-        else if (L.bucketCount) {
+        if (L.bucketCount) {
             const int b = __ffs(__ballot_sync(0xffffffffu, task < bucketEnd)) - 1;
             const int before = __shfl_sync(0xffffffffu, bucketEnd, max(b - 1, 0));
             t = L.bucketTiles[(size_t)(kTileBuckets - 1 - b) * L.tileCap + (task - (b > 0 ? before : 0))];
@@ -517,14 +514,6 @@ __global__ void __launch_bounds__(32 * kPairWarps, IX_TUNE_PAIR_MIN_BLOCKS) kPai
             __syncwarp();
             stageParticle(S, 0, lane, iBase + lane, cx, cy, cz, false, C, L, P);
             stageParticle(S, 1, lane, jslot, cx, cy, cz, shiftImage, C, L, P);
-            if (C.alchOnlyBit) {
-                // keep the pairs with exactly one alchemical particle
-                const bool ia = (__float_as_int(S.hi[0][lane].w) & C.alchOnlyBit) != 0;
-                const bool ja = (__float_as_int(S.hi[1][lane].w) & C.alchOnlyBit) != 0;
-                const unsigned iAlch = __ballot_sync(0xffffffffu, ia), jAlch = __ballot_sync(0xffffffffu, ja);
-                row &= ia ? ~jAlch : jAlch;
-                column &= ja ? ~iAlch : iAlch;
-            }
             __syncwarp();
             if (PREFILTER && C.useCutoff) {
                 // the row's candidates within the cutoff at the current positions
@@ -638,7 +627,7 @@ __global__ void __launch_bounds__(32 * kPairWarps, IX_TUNE_PAIR_MIN_BLOCKS) kPai
             // the tile's energies: a fixed reduction tree over the lanes, one slot per tile
             for (int k = 0; k < 3; k++) {
                 const double sum = warpSumD((double)e[k]);
-                if (lane == 0) P.taskEnergy[3 * (P.taskTiles ? task : t) + k] = sum;
+                if (lane == 0) P.taskEnergy[3 * t + k] = sum;
             }
         }
         flushForce(fi, iBase + lane, L.np, P.forceFixed);
@@ -665,12 +654,107 @@ struct PairTileStorage {
     double energy[kTileThreads / 32][3];
 };
 
+// One tile by a thread block: its forces to P.forceFixed, its energies to `sum` of the lanes 0..2 of warp 2.  ALCH: only
+// its pairs with exactly one alchemical particle (C.alchOnlyBit).
+template <bool LEAN, bool TABLE, bool UNIFORM, bool ALCH>
+__device__ __forceinline__ void pairTileOfBlock(PairTileStorage& S, const ListBuffers& L, const PairBuffers& P,
+                                                const PairTermConfig& C, const PairCoef* coef, int t, unsigned& pairs,
+                                                double& sum) {
+    constexpr bool PREFILTER = !(LEAN && TABLE);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const unsigned ltMask = laneMaskLt();
+    const int I = L.tileIBlock[t];
+    const int iBase = I * 32;
+    const float4 center = L.bbox[2 * I];
+    const bool shiftImage = C.periodic && center.w != 0.0f;
+    const bool perPairImage = C.periodic && !shiftImage;
+    const int jslot = L.tileJ[32 * t + lane];
+    __syncthreads();      // the last tile's shared data has been read
+    if (warp == 0) {
+        S.rowMask[lane] = L.tileMask[64 * t + lane];
+        stageParticle(S, 0, lane, iBase + lane, center.x, center.y, center.z, false, C, L, P);
+    }
+    else if (warp == 1) stageParticle(S, 1, lane, jslot, center.x, center.y, center.z, shiftImage, C, L, P);
+    __syncthreads();
+    // each warp eight rows: the candidates kept, as the warp-per-tile kernel keeps them
+    for (int r = 8 * warp; r < 8 * warp + 8; r++) {
+        bool in = (S.rowMask[r] >> lane) & 1u;
+        if (ALCH)
+            in = in && ((__float_as_int(S.hi[0][r].w) ^ __float_as_int(S.hi[1][lane].w)) & C.alchOnlyBit) != 0;
+        if (PREFILTER && C.useCutoff && in)
+            in = pairInside(S.hi[0][r], S.lo[0][r], S.hi[1][lane], S.lo[1][lane], perPairImage, C);
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        __syncwarp();
+        if (lane == 0) S.rowMask[r] = m;
+    }
+    __syncthreads();
+    // every warp forms the rows' offsets; each queues its rows
+    const unsigned row = S.rowMask[lane];
+    const int count = __popc(row);
+    int start = count;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, start, o);
+        if (lane >= o) start += v;
+    }
+    const int total = __shfl_sync(0xffffffffu, start, 31);
+    start -= count;
+    if (warp == 0) S.rowStart[lane] = start;
+    for (int r = 8 * warp; r < 8 * warp + 8; r++) {
+        const unsigned m = __shfl_sync(0xffffffffu, row, r);
+        const int first = __shfl_sync(0xffffffffu, start, r);
+        if ((m >> lane) & 1u) S.queue[first + __popc(m & ltMask)] = (unsigned short)((r << 5) | lane);
+    }
+    __syncthreads();
+    float e[3] = {0.0f, 0.0f, 0.0f};
+    for (int p = tid; p < total; p += kTileThreads)
+        S.force[p] = computeQueuedPair<LEAN, TABLE, UNIFORM, !PREFILTER>(S, S.queue[p], iBase, perPairImage, C, L,
+                                                                         P, coef, e, pairs);
+    for (int k = 0; k < 3; k++) {
+        const double part = warpSumD((double)e[k]);
+        if (lane == 0) S.energy[warp][k] = part;
+    }
+    __syncthreads();
+    float f[3] = {0.0f, 0.0f, 0.0f};
+    if (warp == 0) {
+        // i side: the row's pairs
+        for (int q = start; q < start + count; q++) {
+            const float4 v = S.force[q];
+            f[0] += v.x;
+            f[1] += v.y;
+            f[2] += v.z;
+        }
+        flushForce(f, iBase + lane, L.np, P.forceFixed);
+    }
+    else if (warp == 1) {
+        // j side: the pair (i, lane) of each row that holds it
+#pragma unroll 4
+        for (int i = 0; i < 32; i++) {
+            const unsigned m = S.rowMask[i];
+            if (!((m >> lane) & 1u)) continue;
+            const float4 v = S.force[S.rowStart[i] + __popc(m & ltMask)];
+            f[0] -= v.x;
+            f[1] -= v.y;
+            f[2] -= v.z;
+        }
+        flushForce(f, jslot, L.np, P.forceFixed);
+    }
+    else if (warp == 2 && lane < 3) {
+        for (int w = 0; w < kTileThreads / 32; w++) sum += S.energy[w][lane];
+    }
+}
+
+__device__ __forceinline__ void addPairCount(const PairBuffers& P, unsigned pairs) {
+    unsigned long long all = pairs;
+    for (int o = 16; o > 0; o >>= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
+    if ((threadIdx.x & 31) == 0 && all) atomicAdd(P.pairCount, all);
+}
+
 template <bool LEAN, bool TABLE, bool UNIFORM = false>
 __global__ void __launch_bounds__(kTileThreads) kPairTilesSmall(ListBuffers L, PairBuffers P, PairTermConfig C) {
     __shared__ PairTileStorage S;
     extern __shared__ float4 pairShared[];
-    constexpr bool PREFILTER = !(LEAN && TABLE);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x;
     const PairCoef* coef = P.coef;
     if (TABLE && P.coefShared) {
         const int words = P.numClasses * P.numClasses * (int)(sizeof(PairCoef) / sizeof(float4));
@@ -678,96 +762,57 @@ __global__ void __launch_bounds__(kTileThreads) kPairTilesSmall(ListBuffers L, P
         for (int k = tid; k < words; k += kTileThreads) pairShared[k] = __ldg(src + k);
         coef = reinterpret_cast<const PairCoef*>(pairShared);
     }
-    const int numTasks = P.taskTiles ? P.numTasks : min(*L.numTiles, L.tileCap);
-    const unsigned ltMask = laneMaskLt();
+    const int numTasks = min(*L.numTiles, L.tileCap);
     unsigned pairs = 0;
-    for (int task = blockIdx.x; task < numTasks; task += gridDim.x) {
-        const int t = P.taskTiles ? P.taskTiles[task] : task;
-        const int I = L.tileIBlock[t];
-        const int iBase = I * 32;
-        const float4 center = L.bbox[2 * I];
-        const bool shiftImage = C.periodic && center.w != 0.0f;
-        const bool perPairImage = C.periodic && !shiftImage;
-        const int jslot = L.tileJ[32 * t + lane];
-        __syncthreads();      // the last tile's shared data has been read
-        if (warp == 0) {
-            S.rowMask[lane] = L.tileMask[64 * t + lane];
-            stageParticle(S, 0, lane, iBase + lane, center.x, center.y, center.z, false, C, L, P);
-        }
-        else if (warp == 1) stageParticle(S, 1, lane, jslot, center.x, center.y, center.z, shiftImage, C, L, P);
-        __syncthreads();
-        // each warp eight rows: the candidates kept, as the warp-per-tile kernel keeps them
-        for (int r = 8 * warp; r < 8 * warp + 8; r++) {
-            bool in = (S.rowMask[r] >> lane) & 1u;
-            if (C.alchOnlyBit)
-                in = in && ((__float_as_int(S.hi[0][r].w) ^ __float_as_int(S.hi[1][lane].w)) & C.alchOnlyBit) != 0;
-            if (PREFILTER && C.useCutoff && in)
-                in = pairInside(S.hi[0][r], S.lo[0][r], S.hi[1][lane], S.lo[1][lane], perPairImage, C);
-            const unsigned m = __ballot_sync(0xffffffffu, in);
-            __syncwarp();
-            if (lane == 0) S.rowMask[r] = m;
-        }
-        __syncthreads();
-        // every warp forms the rows' offsets; each queues its rows
-        const unsigned row = S.rowMask[lane];
-        const int count = __popc(row);
-        int start = count;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, start, o);
-            if (lane >= o) start += v;
-        }
-        const int total = __shfl_sync(0xffffffffu, start, 31);
-        start -= count;
-        if (warp == 0) S.rowStart[lane] = start;
-        for (int r = 8 * warp; r < 8 * warp + 8; r++) {
-            const unsigned m = __shfl_sync(0xffffffffu, row, r);
-            const int first = __shfl_sync(0xffffffffu, start, r);
-            if ((m >> lane) & 1u) S.queue[first + __popc(m & ltMask)] = (unsigned short)((r << 5) | lane);
-        }
-        __syncthreads();
-        float e[3] = {0.0f, 0.0f, 0.0f};
-        for (int p = tid; p < total; p += kTileThreads)
-            S.force[p] = computeQueuedPair<LEAN, TABLE, UNIFORM, !PREFILTER>(S, S.queue[p], iBase, perPairImage, C, L,
-                                                                             P, coef, e, pairs);
-        for (int k = 0; k < 3; k++) {
-            const double sum = warpSumD((double)e[k]);
-            if (lane == 0) S.energy[warp][k] = sum;
-        }
-        __syncthreads();
-        float f[3] = {0.0f, 0.0f, 0.0f};
-        if (warp == 0) {
-            // i side: the row's pairs
-            for (int q = start; q < start + count; q++) {
-                const float4 v = S.force[q];
-                f[0] += v.x;
-                f[1] += v.y;
-                f[2] += v.z;
-            }
-            flushForce(f, iBase + lane, L.np, P.forceFixed);
-        }
-        else if (warp == 1) {
-            // j side: the pair (i, lane) of each row that holds it
-#pragma unroll 4
-            for (int i = 0; i < 32; i++) {
-                const unsigned m = S.rowMask[i];
-                if (!((m >> lane) & 1u)) continue;
-                const float4 v = S.force[S.rowStart[i] + __popc(m & ltMask)];
-                f[0] -= v.x;
-                f[1] -= v.y;
-                f[2] -= v.z;
-            }
-            flushForce(f, jslot, L.np, P.forceFixed);
-        }
-        else if (warp == 2 && lane < 3) {
-            double sum = 0.0;
-            for (int w = 0; w < kTileThreads / 32; w++) sum += S.energy[w][lane];
-            P.taskEnergy[3 * (P.taskTiles ? task : t) + lane] = sum;
-        }
+    for (int t = blockIdx.x; t < numTasks; t += gridDim.x) {
+        double sum = 0.0;
+        pairTileOfBlock<LEAN, TABLE, UNIFORM, false>(S, L, P, C, coef, t, pairs, sum);
+        if (tid >= 64 && tid < 67) P.taskEnergy[3 * t + (tid - 64)] = sum;
     }
-    unsigned long long all = pairs;
-    for (int o = 16; o > 0; o >>= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
-    if (lane == 0 && all) atomicAdd(P.pairCount, all);
+    addPairCount(P, pairs);
+}
+
+// The alchemical pairs (exactly one particle with the flag) of several configurations at once, a row of blocks each:
+// configuration y with forces to row y of forceFixed (3 x np each) and the energies of its blocks to row y of taskEnergy
+// (3 x gridDim.x each, summed in order afterwards).  A block takes every gridDim.x-th tile and does those that are
+// marked (they hold an alchemical particle).  What bounds it is the chain of a tile, of whose thousand pairs a few dozen
+// are kept: 12 windows of a box of 12,297 atoms with 60 alchemical ones take 43 us in one launch (8 to 32 blocks an SM:
+// the same), and took a launch and a finish each, about 40 us a window.
+template <bool TABLE>
+__global__ void __launch_bounds__(kTileThreads) kPairWindows(ListBuffers L, PairBuffers P, const PairTermConfig* configs,
+                                                             const unsigned char* marks) {
+    static_assert(sizeof(PairTermConfig) % sizeof(int) == 0, "copied as ints");
+    __shared__ PairTileStorage S;
+    __shared__ PairTermConfig C;
+    __shared__ int tiles[kTileThreads];
+    __shared__ int marked[kTileThreads / 32];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int* src = reinterpret_cast<const int*>(configs + blockIdx.y);
+    for (int k = tid; k < (int)(sizeof(PairTermConfig) / sizeof(int)); k += kTileThreads)
+        reinterpret_cast<int*>(&C)[k] = src[k];
+    P.forceFixed += (size_t)blockIdx.y * 3 * L.np;
+    const int numTiles = min(*L.numTiles, L.tileCap);
+    unsigned pairs = 0;
+    double sum = 0.0;
+    for (int t0 = blockIdx.x; t0 < numTiles; t0 += kTileThreads * gridDim.x) {
+        const int t = t0 + tid * gridDim.x;
+        const bool mine = t < numTiles && marks[t] != 0;
+        const unsigned m = __ballot_sync(0xffffffffu, mine);
+        if (lane == 0) marked[warp] = __popc(m);
+        __syncthreads();
+        int at = __popc(m & laneMaskLt()), count = 0;
+        for (int w = 0; w < kTileThreads / 32; w++) {
+            if (w < warp) at += marked[w];
+            count += marked[w];
+        }
+        if (mine) tiles[at] = t;
+        __syncthreads();
+        for (int k = 0; k < count; k++)
+            pairTileOfBlock<false, TABLE, false, true>(S, L, P, C, P.coef, tiles[k], pairs, sum);
+        __syncthreads();      // the list has been read
+    }
+    if (tid >= 64 && tid < 67) P.taskEnergy[3 * ((size_t)blockIdx.y * gridDim.x + blockIdx.x) + (tid - 64)] = sum;
+    addPairCount(P, pairs);
 }
 
 }  // namespace ix
