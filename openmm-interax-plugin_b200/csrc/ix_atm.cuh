@@ -156,7 +156,12 @@ __global__ void kSiteCentroids(AtmBuffers A, AtmConfig C, const double* pos) {
         w = siteWrapped(C, c[0], c[1], c[2]);
         wMax = w;
     }
-    if (__any_sync(0xffffffffu, moved) && (threadIdx.x & 31) == 0) atomicOr(A.flag, 1);
+    // a rebuild clears the long-list flag, which the lists set again (the host requests a rebuild by the flag alone)
+    if (__any_sync(0xffffffffu, moved) && (threadIdx.x & 31) == 0) {
+        atomicOr(A.flag, 1);
+        A.flag[2] = 0;
+    }
+    else if (s == 0 && *(volatile int*)A.flag != 0) A.flag[2] = 0;
     if (A.chunkBox) {
         // the box of this warp's 32 sites (blocks are whole warps, so a warp is one chunk)
         const float lo[3] = {warpMinF(w.x), warpMinF(w.y), warpMinF(w.z)};
@@ -217,7 +222,7 @@ __global__ void kSiteNeighbors(AtmBuffers A, AtmConfig C) {
         // scans every later site instead of reading the list
         A.nbrCount[a] = count;
         if (count > A.cap) atomicOr(A.flag + 1, 1);
-        // flag[2]: some site needs the wide triple kernel (cleared before each build)
+        // flag[2]: some site needs the wide triple kernel (cleared with each request of a build)
         if (count > kAtmFast || count > A.cap) atomicOr(A.flag + 2, 1);
         if (a == 0) A.flag[3] = 1;
     }
@@ -238,7 +243,6 @@ __global__ void __launch_bounds__(1024) kSiteCellSort(AtmBuffers A, AtmConfig C,
     const SiteCells& G = A.cells;
     const int numCells = G.nc[0] * G.nc[1] * G.nc[2];
     const int t = threadIdx.x, T = blockDim.x;
-    if (t == 0) A.flag[2] = 0;      // set again by the lists that follow
     for (int c = t; c < numCells; c += T) count[c] = 0;
     __syncthreads();
     for (int s = t; s < C.numSites; s += T) {

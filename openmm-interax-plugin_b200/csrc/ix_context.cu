@@ -1104,11 +1104,11 @@ struct EnergyReduction {
     int *pairRebuild, *siteRebuild;      // rebuild flags to clear (null: none): every kernel that reads them has run
 };
 
-// One block (of `numBlocks`) of the energy reduction; 256 threads.
+// One block (of `numBlocks`) of the energy reduction; at least four warps.
 __device__ void reduceEnergiesBlock(const EnergyReduction& R, int block, int numBlocks) {
-    __shared__ double red[4][256];
+    __shared__ double red[32][4];
     __shared__ bool last;
-    const int t = threadIdx.x;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, threads = blockDim.x;
     // each block sums a fixed contiguous share of each array; the last block to finish adds the block sums in order
     auto share = [&](int total, int& lo, int& hi) {
         const int per = (total + numBlocks - 1) / numBlocks;
@@ -1119,37 +1119,37 @@ __device__ void reduceEnergiesBlock(const EnergyReduction& R, int block, int num
     int lo, hi;
     if (R.pairPartials) {
         share(min(*R.numPairPartials, R.pairCap), lo, hi);
-        for (int w = lo + t; w < hi; w += 256)
+        for (int w = lo + t; w < hi; w += threads)
             for (int k = 0; k < 3; k++) s[k] += R.pairPartials[3 * w + k];
     }
     if (R.atmPartials) {
         share(R.numAtmWarps, lo, hi);
-        for (int w = lo + t; w < hi; w += 256) s[3] += R.atmPartials[w];
+        for (int w = lo + t; w < hi; w += threads) s[3] += R.atmPartials[w];
     }
-    for (int k = 0; k < 4; k++) red[k][t] = s[k];
-    __syncthreads();
-    for (int half = 128; half > 0; half >>= 1) {
-        if (t < half)
-            for (int k = 0; k < 4; k++) red[k][t] += red[k][t + half];
-        __syncthreads();
+    for (int k = 0; k < 4; k++) {
+        s[k] = warpSumD(s[k]);
+        if (lane == 0) red[warp][k] = s[k];
     }
-    if (t == 0) {
-        for (int k = 0; k < 4; k++) R.blockSums[4 * block + k] = red[k][0];
-        __threadfence();
-        // wraps to 0 on the last block, ready for the next launch
-        last = atomicInc(R.ticket, numBlocks - 1) == (unsigned)(numBlocks - 1);
-    }
-    __syncthreads();
-    if (!last) return;
-    // the block sums are loaded in parallel, then added in block order
-    __threadfence();
-    for (int k = t; k < 4 * numBlocks; k += 256) red[k & 3][k >> 2] = ((volatile double*)R.blockSums)[k];
     __syncthreads();
     if (t < 4) {
-        double v = 0.0;
-        for (int b = 0; b < numBlocks; b++) v += red[t][b];
+        double v = red[0][t];
+        for (int w = 1; w < threads / 32; w++) v += red[w][t];
+        R.blockSums[4 * block + t] = v;
+        __threadfence();
+    }
+    __syncthreads();
+    // wraps to 0 on the last block, ready for the next launch
+    if (t == 0) last = atomicInc(R.ticket, numBlocks - 1) == (unsigned)(numBlocks - 1);
+    __syncthreads();
+    if (!last || warp >= 4) return;
+    // warp k adds the block sums of component k
+    __threadfence();
+    double v = 0.0;
+    for (int b = lane; b < numBlocks; b += 32) v += ((volatile double*)R.blockSums)[4 * b + warp];
+    v = warpSumD(v);
+    if (lane == 0) {
         if (t == 0) v += R.lrcEnergy;
-        if (R.outEnergy) R.outEnergy[t] = v;
+        if (R.outEnergy) R.outEnergy[warp] = v;
         if (t == 0) {
             if (R.counts) {
                 R.counts[2] = R.counts[0];
@@ -1188,12 +1188,17 @@ struct FinishForces {
     const double* invMass;               // null: no velocity half kick
     double* vel;
     double halfDt;
-    int blocks;                          // blocks of 256 particles; the grid's remaining blocks reduce the energies
+    int blocks;                          // blocks of kFinishThreads particles; the remaining blocks reduce the energies
 };
 
 // The end of an evaluation in one launch: each particle's force (its pair force and its share of the forces on its
 // three-body sites, in 64-bit fixed point, so the sum is the same in any order) to the outputs, and in an MD step
 // the second velocity half kick; the grid's last kReduceBlocks blocks reduce the term energies.
+// What bounds it: latency, of two chains of dependent loads for the forces (taken side by side, stores after them) and
+// of the reduction (shuffles within a warp, the block sums added by a warp per component).  With the chains one after
+// the other, a tree in shared memory over 256 threads and the block sums added by one thread, it took 10.2 us at 24,000
+// atoms, 17 at 96,000 and 5.6 at 648, and takes 6.8, 10 and 5.2.
+constexpr int kFinishThreads = 128;
 __global__ void kFinish(FinishForces F, EnergyReduction R) {
     if ((int)blockIdx.x >= F.blocks) {
         reduceEnergiesBlock(R, (int)blockIdx.x - F.blocks, (int)gridDim.x - F.blocks);
@@ -1201,23 +1206,22 @@ __global__ void kFinish(FinishForces F, EnergyReduction R) {
     }
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= F.n) return;
+    // the loads of both chains (slot and pair force; sites, their sizes and forces) side by side, stores after them
+    const int slot = F.pairForce ? F.slotOf[i] : 0;
+    const int first = F.siteForce ? F.particleSiteStart[i] : 0, end = F.siteForce ? F.particleSiteStart[i + 1] : 0;
     long long f[3] = {0, 0, 0};
-    if (F.pairForce) {
-        const int s = F.slotOf[i];
+    if (F.pairForce)
+        for (int d = 0; d < 3; d++) f[d] = F.pairForce[d * F.np + slot];
+    for (int k = first; k < end; k++) {
+        const int site = F.particleSites[k];
+        const double inv = 1.0 / (double)(F.siteOffsets[site + 1] - F.siteOffsets[site]);
         for (int d = 0; d < 3; d++) {
-            f[d] = F.pairForce[d * F.np + s];
-            F.pairForce[d * F.np + s] = 0;
+            const long long v = F.siteForce[d * F.numSites + site];
+            if (v != 0) f[d] += __double2ll_rn((double)v * inv);
         }
     }
-    if (F.siteForce)
-        for (int k = F.particleSiteStart[i]; k < F.particleSiteStart[i + 1]; k++) {
-            const int site = F.particleSites[k];
-            const double inv = 1.0 / (double)(F.siteOffsets[site + 1] - F.siteOffsets[site]);
-            for (int d = 0; d < 3; d++) {
-                const long long v = F.siteForce[d * F.numSites + site];
-                if (v != 0) f[d] += __double2ll_rn((double)v * inv);
-            }
-        }
+    if (F.pairForce)
+        for (int d = 0; d < 3; d++) F.pairForce[d * F.np + slot] = 0;
     const double inv = 1.0 / kFixedScale;
     const double fx = (double)f[0] * inv, fy = (double)f[1] * inv, fz = (double)f[2] * inv;
     if (F.outForces) {
@@ -1328,10 +1332,6 @@ static void recordTiming(ix_ctx* ctx, int i, cudaStream_t s) {
     else cudaEventRecord(ctx->ev[i], s);
 }
 
-__global__ void kClearFlagIf(int* target, const int* gate) {
-    if (*(volatile const int*)gate != 0) *target = 0;
-}
-
 // The configuration of the three-body kernels at the context's parameters, and the cell grid of the site-list search.
 static AtmConfig atmConfig(ix_ctx* ctx) {
     AtmBuffers& A = ctx->A;
@@ -1424,21 +1424,18 @@ static int launchEvaluation(ix_ctx* ctx, unsigned terms, double* outForces, doub
         const int gS = (C.numSites + 63) / 64;   // 64-thread blocks, so that a few thousand sites reach every SM
         kSiteCentroids<<<gS, 64, 0, sa>>>(A, C, ctx->dPos);
         // site list rebuild when the centroid kernel set the flag: these kernels return at once otherwise.  The
-        // long-list flag is recomputed with the lists (the cell sort clears it)
+        // long-list flag is recomputed with the lists
         if (A.cells.nc[0]) {
             const int sharedSites = C.numSites <= kSiteSortSharedMax;
             kSiteCellSort<<<1, 1024, sharedSites ? C.numSites * sizeof(int) : 0, sa>>>(A, C, sharedSites);
             kSiteNeighborsCells<<<std::min((C.numSites * 32 + tpb - 1) / tpb, ctx->numSMs * 2), tpb, 0, sa>>>(A, C);
         }
-        else {
-            kClearFlagIf<<<1, 1, 0, sa>>>(A.flag + 2, A.flag);
-            kSiteNeighbors<<<(C.numSites * 32 + tpb - 1) / tpb, tpb, 0, sa>>>(A, C);
-        }
+        else kSiteNeighbors<<<(C.numSites * 32 + tpb - 1) / tpb, tpb, 0, sa>>>(A, C);
         recordTiming(ctx, 2, sa);
         // the sites whose lists are too long for the fast kernel go to the wide one, which returns at once when there
         // are none and goes first
         launchTriples<false>(A, C, ctx->atmFastBlocks, ctx->atmGridBlocks, A.flag + 2, sa, fork ? ctx->evFork : nullptr);
-        ctx->launches += 5;
+        ctx->launches += A.cells.nc[0] ? 5 : 4;
         recordTiming(ctx, 3, sa);
         ctx->evAtm = ctx->profiling;
         IX_CUDA(ctx, cudaGetLastError());
@@ -1531,12 +1528,12 @@ static int launchEvaluation(ix_ctx* ctx, unsigned terms, double* outForces, doub
         F.vel = kick->vel;
         F.halfDt = kick->halfDt;
     }
-    F.blocks = (n + 255) / 256;
+    F.blocks = (n + kFinishThreads - 1) / kFinishThreads;
     EnergyReduction R{doPair ? ctx->dPairPartials : nullptr, ctx->L.numTiles, ctx->L.tileCap,
                       doAtm ? ctx->dAtmPartials : nullptr, (int)atmPartialCount(ctx), lrcEnergy, outEnergy,
                       ctx->dEnergyBlocks, ctx->dReduceTicket, ctx->dCounts, doPair ? ctx->L.taskCounter : nullptr,
                       doPair ? ctx->L.flag : nullptr, doAtm ? ctx->A.flag : nullptr};
-    kFinish<<<F.blocks + kReduceBlocks, 256, 0, st>>>(F, R);
+    kFinish<<<F.blocks + kReduceBlocks, kFinishThreads, 0, st>>>(F, R);
     ctx->launches += 1;
     IX_CUDA(ctx, cudaGetLastError());
     return IX_OK;
@@ -2649,10 +2646,10 @@ static int windowSlope(ix_ctx* ctx, bool atm, bool pairs, double* dSlope, double
     F.particleSiteStart = ctx->dParticleSiteStart;
     F.particleSites = ctx->dParticleSites;
     F.outForces = dSlope;
-    F.blocks = (ctx->n + 255) / 256;
+    F.blocks = (ctx->n + kFinishThreads - 1) / kFinishThreads;
     EnergyReduction R{nullptr, nullptr, 0, atm ? ctx->dAtmPartials : nullptr, (int)atmPartialCount(ctx), 0.0, dEnergy,
                       ctx->dEnergyBlocks, ctx->dReduceTicket, atm ? ctx->dCounts : nullptr, nullptr, nullptr, nullptr};
-    kFinish<<<F.blocks + kReduceBlocks, 256, 0, ctx->stream>>>(F, R);
+    kFinish<<<F.blocks + kReduceBlocks, kFinishThreads, 0, ctx->stream>>>(F, R);
     ctx->launches += 1;
     IX_CUDA(ctx, cudaGetLastError());
     return IX_OK;
