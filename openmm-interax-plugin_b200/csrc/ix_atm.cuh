@@ -132,6 +132,7 @@ __device__ __forceinline__ float siteBoxDist2(const AtmConfig& C, float3 p, floa
 }
 
 __global__ void kSiteCentroids(AtmBuffers A, AtmConfig C, const double* pos) {
+    dependentStart(C.numSites <= kEarlySites);
     int s = blockIdx.x * blockDim.x + threadIdx.x;
     for (int k = s; k < C.zeroSlots; k += gridDim.x * blockDim.x) A.energyPartials[C.zeroOffset + k] = 0.0;
     bool moved = false;
@@ -189,6 +190,7 @@ __device__ __forceinline__ void siteDelta(const AtmBuffers& A, const AtmConfig& 
 // One warp per site A scans the sites above it, 32-site chunk by chunk, skipping the chunks whose box is farther
 // than the list cutoff from A (when the centroid kernel wrote the chunk boxes).  The list is in increasing site order.
 __global__ void kSiteNeighbors(AtmBuffers A, AtmConfig C) {
+    dependentStart(C.numSites <= kEarlySites);
     if (*(volatile int*)A.flag == 0) return;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -236,6 +238,7 @@ __global__ void kSiteNeighbors(AtmBuffers A, AtmConfig C) {
 // the launch giving 4 bytes of dynamic shared memory per site) the scatter goes to shared memory and a warp per cell
 // writes each site at its rank among the cell's sites; else each cell is insertion-sorted in place in global memory.
 __global__ void __launch_bounds__(1024) kSiteCellSort(AtmBuffers A, AtmConfig C, int sharedSites) {
+    dependentStart(C.numSites <= kEarlySites);
     if (*(volatile int*)A.flag == 0) return;
     __shared__ int count[kSiteCellMax];
     __shared__ int threadSum[1024];
@@ -321,6 +324,7 @@ __global__ void __launch_bounds__(1024) kSiteCellSort(AtmBuffers A, AtmConfig C,
 // leave out, never the reverse, and the triple kernels test the cutoff itself in double.  The counts and flags are
 // those of kSiteNeighbors.  Launched with 256-thread blocks.
 __global__ void __launch_bounds__(256) kSiteNeighborsCells(AtmBuffers A, AtmConfig C) {
+    dependentStart(C.numSites <= kEarlySites);
     if (*(volatile int*)A.flag == 0) return;
     __shared__ int cellFirst[8][32], cellEnd[8][32];   // per warp: each cell's first site and its end in the sequence
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -630,6 +634,7 @@ __device__ __forceinline__ int stageTripleNeighborsScan(const AtmBuffers& A, con
 
 template <bool DAMP, bool IMAGE, bool ALCH>
 __global__ void __launch_bounds__(32 * kAtmFastWarps, IX_TUNE_ATM_MIN_BLOCKS) kTriplesFast(AtmBuffers A, AtmConfig C) {
+    dependentStart(false);
     __shared__ TripleStorage<DAMP, kAtmFastStaged> storage[kAtmFastWarps];
     auto& S = storage[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
@@ -681,6 +686,7 @@ constexpr int kAtmWideParts = 8;
 template <bool DAMP, bool IMAGE, bool ALCH>
 __global__ void __launch_bounds__(32 * kAtmWarps) kTriplesWide(AtmBuffers A, AtmConfig C, int partialsOffset,
                                                                const int* gate) {
+    dependentStart(C.numSites <= kEarlySites);
     if (gate && *(volatile const int*)gate == 0) return;
     extern __shared__ float4 atmShared[];
     auto& S = reinterpret_cast<TripleStorage<DAMP, kAtmMaxStaged>*>(atmShared)[threadIdx.x >> 5];
@@ -743,22 +749,21 @@ __global__ void __launch_bounds__(32 * kAtmWarps) kTriplesWide(AtmBuffers A, Atm
 // be null) is recorded ahead of the fast kernel.  ALCH: only the triples with an alchemical site.
 template <bool DAMP, bool IMAGE, bool ALCH>
 static void launchTriplesAs(const AtmBuffers& A, const AtmConfig& C, int fastBlocks, int wideBlocks, const int* gate,
-                            cudaStream_t st, cudaEvent_t before) {
+                            cudaStream_t st, cudaEvent_t before, bool early) {
     if (wideBlocks > 0)
-        kTriplesWide<DAMP, IMAGE, ALCH><<<wideBlocks, 32 * kAtmWarps,
-                                    kAtmWarps * sizeof(TripleStorage<DAMP, kAtmMaxStaged>), st>>>(
-            A, C, fastBlocks * kAtmFastWarps, gate);
+        launchNext(early, st, kTriplesWide<DAMP, IMAGE, ALCH>, wideBlocks, 32 * kAtmWarps,
+                   kAtmWarps * sizeof(TripleStorage<DAMP, kAtmMaxStaged>), A, C, fastBlocks * kAtmFastWarps, gate);
     if (before) cudaEventRecord(before, st);
-    kTriplesFast<DAMP, IMAGE, ALCH><<<fastBlocks, 32 * kAtmFastWarps, 0, st>>>(A, C);
+    launchNext(early && C.numSites <= kEarlySites, st, kTriplesFast<DAMP, IMAGE, ALCH>, fastBlocks, 32 * kAtmFastWarps, 0, A, C);
 }
 template <bool ALCH>
 static void launchTriples(const AtmBuffers& A, const AtmConfig& C, int fastBlocks, int wideBlocks, const int* gate,
-                          cudaStream_t st, cudaEvent_t before = nullptr) {
+                          cudaStream_t st, cudaEvent_t before = nullptr, bool early = false) {
     const bool damp = C.useTangToennies || C.invCentroidRadius > 0.0f;
-    if (damp && C.imageBC) launchTriplesAs<true, true, ALCH>(A, C, fastBlocks, wideBlocks, gate, st, before);
-    else if (damp) launchTriplesAs<true, false, ALCH>(A, C, fastBlocks, wideBlocks, gate, st, before);
-    else if (C.imageBC) launchTriplesAs<false, true, ALCH>(A, C, fastBlocks, wideBlocks, gate, st, before);
-    else launchTriplesAs<false, false, ALCH>(A, C, fastBlocks, wideBlocks, gate, st, before);
+    if (damp && C.imageBC) launchTriplesAs<true, true, ALCH>(A, C, fastBlocks, wideBlocks, gate, st, before, early);
+    else if (damp) launchTriplesAs<true, false, ALCH>(A, C, fastBlocks, wideBlocks, gate, st, before, early);
+    else if (C.imageBC) launchTriplesAs<false, true, ALCH>(A, C, fastBlocks, wideBlocks, gate, st, before, early);
+    else launchTriplesAs<false, false, ALCH>(A, C, fastBlocks, wideBlocks, gate, st, before, early);
 }
 
 // Each particle of a site receives the site force divided by the number of particles

@@ -154,4 +154,42 @@ struct NvtxRange {
     NvtxRange& operator=(const NvtxRange&) = delete;
 };
 
+// Kernels in a row, each of a few microseconds or a return at once (the list build of a step that needs none): launched
+// by launchNext, a kernel is set up while the one before it in the stream still runs, and waits in dependentStart, its
+// first statement, until that one has finished and its writes are visible.  With `trigger` the kernel lets its own
+// successor be set up as soon as all of its blocks have started (else when they have ended).
+// Measured without and with it: 100 steps of 648 atoms 3890 and 3660 us, of 24,000 atoms 16930 and 16730; an evaluation
+// of 648 atoms 66.5 and 64.9 us.  Eight evaluations of 96,000 atoms, whose triple kernel is as long as its pair kernel, took
+// 4617 us without and 4635 with it (the two kernels' blocks are placed in another order): more than kEarlyLaunchBlocks
+// blocks of 32 particles are launched the ordinary way.
+__device__ __forceinline__ void dependentStart(bool trigger) {
+    cudaGridDependencySynchronize();
+    if (trigger) cudaTriggerProgrammaticLaunchCompletion();
+}
+
+// A launch behind the kernel before it in the stream.  early: false where something else lies between the two (an event
+// of the kernel times): an ordinary launch.
+template <class... Params, class... Args>
+static cudaError_t launchNext(bool early, cudaStream_t st, void (*kernel)(Params...), unsigned grid, unsigned block,
+                              size_t shared, const Args&... args) {
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(grid);
+    config.blockDim = dim3(block);
+    config.dynamicSmemBytes = shared;
+    config.stream = st;
+    cudaLaunchAttribute serialization{};
+    serialization.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    serialization.val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = &serialization;
+    config.numAttrs = early ? 1 : 0;
+    return cudaLaunchKernelEx(&config, kernel, Params(args)...);
+}
+
+constexpr int kEarlyLaunchBlocks = 1024;
+
+// Systems of at most this many blocks of 32 particles, and of this many sites, trigger: their successors' waiting blocks
+// keep nothing else from the SMs (with it everywhere the dynamics of 24,000 atoms gained nothing: 16950 us), and 648
+// atoms take 3700 us for 3850 without.
+constexpr int kEarlyBlocks = 192, kEarlySites = 2048;
+
 }  // namespace ix

@@ -1200,6 +1200,7 @@ struct FinishForces {
 // atoms, 17 at 96,000 and 5.6 at 648, and takes 6.8, 10 and 5.2.
 constexpr int kFinishThreads = 128;
 __global__ void kFinish(FinishForces F, EnergyReduction R) {
+    dependentStart(F.n <= 32 * kEarlyBlocks);
     if ((int)blockIdx.x >= F.blocks) {
         reduceEnergiesBlock(R, (int)blockIdx.x - F.blocks, (int)gridDim.x - F.blocks);
         return;
@@ -1251,6 +1252,7 @@ __global__ void kFinish(FinishForces F, EnergyReduction R) {
 // position (the rebuild, when it runs, sorts and refreshes again).
 __global__ void kStepStart(ListBuffers L, double* pos, double dt, const double* invMass, const double* force,
                            double* vel, float maxMove2) {
+    dependentStart(L.nb <= kEarlyBlocks);
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     bool moved = false;
     if (s < L.n) {
@@ -1377,11 +1379,11 @@ constexpr int kSmallBlocks = 192;
 
 // The pair kernel's instance for the configuration: lean (no soft core, switching function or order-2 overlap), from
 // the class-pair table, uniform (no gates or scales), and the form for small systems.
-static void launchPairTiles(bool lean, bool table, bool uniform, bool small, int grid, int tiles, size_t dyn,
-                            cudaStream_t st, const ListBuffers& L, const PairBuffers& P, const PairTermConfig& C) {
+static void launchPairTiles(bool early, bool lean, bool table, bool uniform, bool small, int grid, int tiles,
+                            size_t dyn, cudaStream_t st, const ListBuffers& L, const PairBuffers& P, const PairTermConfig& C) {
     auto run = [&](auto* tileKernel, auto* smallKernel, size_t shared) {
-        if (small) smallKernel<<<std::max(tiles, 1), kTileThreads, shared, st>>>(L, P, C);
-        else tileKernel<<<grid, 32 * kPairWarps, shared, st>>>(L, P, C);
+        if (small) launchNext(early, st, smallKernel, std::max(tiles, 1), kTileThreads, shared, L, P, C);
+        else launchNext(early, st, tileKernel, grid, 32 * kPairWarps, shared, L, P, C);
     };
     if (lean && table && uniform) run(kPairTiles<true, true, true>, kPairTilesSmall<true, true, true>, dyn);
     else if (lean && uniform) run(kPairTiles<true, false, true>, kPairTilesSmall<true, false, true>, 0);
@@ -1409,6 +1411,8 @@ static int launchEvaluation(ix_ctx* ctx, unsigned terms, double* outForces, doub
     cudaStream_t st = ctx->stream;
     const bool doPair = (terms & 7u) != 0;
     const bool doAtm = (terms & 8u) != 0;
+    // not with kernel times, whose events lie between the kernels, nor in large systems
+    const bool early = !ctx->profiling && (n + 31) / 32 <= kEarlyLaunchBlocks;
     IX_TRY(stageUploads(ctx, terms));
     // the three-body chain runs on a second stream, concurrently with the pair list and pair kernel
     const bool fork = doPair && doAtm && !ctx->serialize;
@@ -1427,14 +1431,16 @@ static int launchEvaluation(ix_ctx* ctx, unsigned terms, double* outForces, doub
         // long-list flag is recomputed with the lists
         if (A.cells.nc[0]) {
             const int sharedSites = C.numSites <= kSiteSortSharedMax;
-            kSiteCellSort<<<1, 1024, sharedSites ? C.numSites * sizeof(int) : 0, sa>>>(A, C, sharedSites);
-            kSiteNeighborsCells<<<std::min((C.numSites * 32 + tpb - 1) / tpb, ctx->numSMs * 2), tpb, 0, sa>>>(A, C);
+            launchNext(early, sa, kSiteCellSort, 1, 1024, sharedSites ? C.numSites * sizeof(int) : 0, A, C, sharedSites);
+            launchNext(early, sa, kSiteNeighborsCells, std::min((C.numSites * 32 + tpb - 1) / tpb, ctx->numSMs * 2), tpb, 0,
+                       A, C);
         }
-        else kSiteNeighbors<<<(C.numSites * 32 + tpb - 1) / tpb, tpb, 0, sa>>>(A, C);
+        else launchNext(early, sa, kSiteNeighbors, (C.numSites * 32 + tpb - 1) / tpb, tpb, 0, A, C);
         recordTiming(ctx, 2, sa);
         // the sites whose lists are too long for the fast kernel go to the wide one, which returns at once when there
         // are none and goes first
-        launchTriples<false>(A, C, ctx->atmFastBlocks, ctx->atmGridBlocks, A.flag + 2, sa, fork ? ctx->evFork : nullptr);
+        launchTriples<false>(A, C, ctx->atmFastBlocks, ctx->atmGridBlocks, A.flag + 2, sa, fork ? ctx->evFork : nullptr,
+                             early);
         ctx->launches += A.cells.nc[0] ? 5 : 4;
         recordTiming(ctx, 3, sa);
         ctx->evAtm = ctx->profiling;
@@ -1454,16 +1460,17 @@ static int launchEvaluation(ix_ctx* ctx, unsigned terms, double* outForces, doub
         // list rebuild (the displacement check or the host set the flag; else each kernel returns at once)
         const SortedParams S{ctx->dP0o, ctx->dP1o, ctx->dP2o, ctx->dP3o, ctx->dFlagso, ctx->dP0,
                              ctx->dP1,  ctx->dP2,  ctx->dP3,  ctx->dFlagsSorted};
-        if (!ctx->G.periodic) kParticleBounds<<<gN, tpb, 0, st>>>(L);
-        kCellKeys<<<(n + kCellThreads - 1) / kCellThreads, kCellThreads, 0, st>>>(L, ctx->G);
-        kScatterCells<<<gN, tpb, 0, st>>>(L);
-        kSortBlocks<<<gNp, tpb, 0, st>>>(L, ctx->G, S);
+        if (!ctx->G.periodic) launchNext(early, st, kParticleBounds, gN, tpb, 0, L);
+        launchNext(early, st, kCellKeys, (n + kCellThreads - 1) / kCellThreads, kCellThreads, 0, L, ctx->G);
+        launchNext(early, st, kScatterCells, gN, tpb, 0, L);
+        launchNext(early, st, kSortBlocks, gNp, tpb, 0, L, ctx->G, S);
         // at most four blocks per SM: more gain nothing in a rebuild and return later in a step without one
-        kListBlocks<<<std::min(ctx->numSMs * 4, L.nb), kListThreads, 0, st>>>(L, ctx->G);
+        launchNext(early, st, kListBlocks, std::min(ctx->numSMs * 4, L.nb), kListThreads, 0, L, ctx->G);
         // no more warps than tiles, and four blocks per SM at most: with eight the masks of 24,000 atoms take 37 us for
         // 41, but a step without a rebuild waits 4.2 us for the blocks to return for 2.7
-        kTileMasks<<<std::min(ctx->numSMs * 4, std::max(1, (L.tileCap + kListWarps - 1) / kListWarps)),
-                     kListThreads, 0, st>>>(L, ctx->G);
+        launchNext(early, st, kTileMasks,
+                   std::min(ctx->numSMs * 4, std::max(1, (L.tileCap + kListWarps - 1) / kListWarps)), kListThreads, 0,
+                   L, ctx->G);
         ctx->launches += ctx->G.periodic ? 5 : 6;
         // the pair kernel's persistent grid fills the SMs: the triple kernel, ready at the same time and on a stream of
         // higher priority, is placed first (it was left to the end of the pair kernel when its chain came a microsecond
@@ -1494,7 +1501,7 @@ static int launchEvaluation(ix_ctx* ctx, unsigned terms, double* outForces, doub
         const size_t dyn = table && tableBytes <= (size_t)IX_TUNE_PAIR_SHARED_TABLE_BYTES ? tableBytes : 0;
         P.coefShared = dyn > 0;
         C.coefShared = P.coefShared;
-        launchPairTiles(lean, table, uniform, ctx->L.nb <= kSmallBlocks, grid, L.tileCap, dyn, st, L, P, C);
+        launchPairTiles(early && ctx->L.nb <= kSmallBlocks, lean, table, uniform, ctx->L.nb <= kSmallBlocks, grid, L.tileCap, dyn, st, L, P, C);
         ctx->launches += 1;
         recordTiming(ctx, 1, st);
         ctx->evPair = ctx->profiling;
@@ -1533,7 +1540,7 @@ static int launchEvaluation(ix_ctx* ctx, unsigned terms, double* outForces, doub
                       doAtm ? ctx->dAtmPartials : nullptr, (int)atmPartialCount(ctx), lrcEnergy, outEnergy,
                       ctx->dEnergyBlocks, ctx->dReduceTicket, ctx->dCounts, doPair ? ctx->L.taskCounter : nullptr,
                       doPair ? ctx->L.flag : nullptr, doAtm ? ctx->A.flag : nullptr};
-    kFinish<<<F.blocks + kReduceBlocks, kFinishThreads, 0, st>>>(F, R);
+    launchNext(early, st, kFinish, F.blocks + kReduceBlocks, kFinishThreads, 0, F, R);
     ctx->launches += 1;
     IX_CUDA(ctx, cudaGetLastError());
     return IX_OK;
@@ -2496,8 +2503,8 @@ static int enqueueSteps(ix_ctx* ctx, int num_steps, double dt) {
         ctx->launches += 1;
         IX_TRY(launchEvaluation(ctx, terms, ctx->dOutForces, ctx->dOutEnergy, nullptr, 0, &kick));
         if (ctx->numConstraints) {
-            kConstrainVelocities<<<clusterGrid, kClusterBlock, 0, ctx->stream>>>(ctx->K, ctx->dInvMass, ctx->dPos,
-                                                                                ctx->dVel);
+            launchNext(true, ctx->stream, kConstrainVelocities, clusterGrid, kClusterBlock, 0, ctx->K, ctx->dInvMass,
+                       ctx->dPos, ctx->dVel);
             ctx->launches += 1;
         }
         IX_CUDA(ctx, cudaGetLastError());

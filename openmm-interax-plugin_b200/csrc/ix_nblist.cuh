@@ -100,6 +100,7 @@ constexpr int kTileBuckets = 16;
 // which sets the rebuild flag (then, and where it is set already, the build writes the positions itself).  Padding
 // slots copy the last real particle's position, which keeps the blocks' boxes tight; they never interact.
 __global__ void kRefreshPositions(ListBuffers L, float maxMove2) {
+    dependentStart(L.nb <= kEarlyBlocks);
     if (rebuildRequested(L)) return;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     bool moved = false;
@@ -170,6 +171,7 @@ __device__ __forceinline__ void resetBounds(const ListBuffers& L) {
 
 // Bounding box of all particles (non-periodic cell grids span it).
 __global__ void kParticleBounds(ListBuffers L) {
+    dependentStart(L.nb <= kEarlyBlocks);
     if (!rebuildRequested(L)) return;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     float v[6];
@@ -229,6 +231,7 @@ __device__ __forceinline__ int cellOf(const double w[3], const ListGeometry& G, 
 // the counts into the cells' starts, and leaves the counts and the bounds as the next build needs them.
 constexpr int kCellThreads = 512;
 __global__ void __launch_bounds__(kCellThreads) kCellKeys(ListBuffers L, ListGeometry G) {
+    dependentStart(L.nb <= kEarlyBlocks);
     if (!rebuildRequested(L)) return;
     const int t = threadIdx.x, i = blockIdx.x * kCellThreads + t;
     if (i < L.n) {
@@ -267,6 +270,7 @@ __global__ void __launch_bounds__(kCellThreads) kCellKeys(ListBuffers L, ListGeo
 }
 
 __global__ void kScatterCells(ListBuffers L) {
+    dependentStart(L.nb <= kEarlyBlocks);
     if (!rebuildRequested(L)) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < L.n) L.order[L.cellStart[L.cellKey[i]] + L.cellArrival[i]] = i;
@@ -312,6 +316,7 @@ __global__ void kBlockBounds(ListBuffers L, ListGeometry G) {
 // not depend on the atomics (slot k of a cell takes the particle that k others of the cell precede: a cell holds about
 // four), the image shift that places each in the build frame, its positions and parameters, and the block's box.
 __global__ void __launch_bounds__(256) kSortBlocks(ListBuffers L, ListGeometry G, SortedParams P) {
+    dependentStart(L.nb <= kEarlyBlocks);
     if (!rebuildRequested(L)) return;
     const int lane = threadIdx.x & 31;
     const int block = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -407,6 +412,7 @@ constexpr int kListWarps = kListThreads / 32;
 // scans the tile counts.  On overflow no tile is scheduled (nothing is written beyond the buffers); the host grows
 // them and evaluates again.
 __global__ void __launch_bounds__(kListThreads) kListBlocks(ListBuffers L, ListGeometry G) {
+    dependentStart(L.nb <= kEarlyBlocks);
     if (!rebuildRequested(L)) return;
     __shared__ int candJ[kListThreads];
     __shared__ unsigned keep[kListThreads];
@@ -557,6 +563,7 @@ __device__ __forceinline__ unsigned transposeBits(unsigned x, int lane) {
 // minimum image per pair.  Exclusions are looked up only for the pairs whose i lies in j's exclusion range.  Row
 // masks: lane = i slot, bit k = the tile's j lane k; column masks: the transpose.
 __global__ void __launch_bounds__(kListThreads) kTileMasks(ListBuffers L, ListGeometry G) {
+    dependentStart(false);
     if (!rebuildRequested(L)) return;
     __shared__ float4 ipos[kListWarps][32];   // xyz and the original index (as its bits)
     __shared__ int slots[kListWarps][32];

@@ -457,6 +457,7 @@ __device__ __forceinline__ void computeQueuedPair2(PairWarpStorage& S, int entry
 
 template <bool LEAN, bool TABLE, bool UNIFORM = false>
 __global__ void __launch_bounds__(32 * kPairWarps, IX_TUNE_PAIR_MIN_BLOCKS) kPairTiles(ListBuffers L, PairBuffers P, PairTermConfig C) {
+    dependentStart(false);
     __shared__ PairWarpStorage storage[kPairWarps];
     extern __shared__ float4 pairShared[];
     // the candidates are filtered against the cutoff when queued, except on the class-table path without soft core,
@@ -752,6 +753,7 @@ __device__ __forceinline__ void addPairCount(const PairBuffers& P, unsigned pair
 
 template <bool LEAN, bool TABLE, bool UNIFORM = false>
 __global__ void __launch_bounds__(kTileThreads) kPairTilesSmall(ListBuffers L, PairBuffers P, PairTermConfig C) {
+    dependentStart(true);
     __shared__ PairTileStorage S;
     extern __shared__ float4 pairShared[];
     const int tid = threadIdx.x;
