@@ -362,7 +362,7 @@ int buildBatchPairs(ix_batch* b, const std::vector<int>& blockStart, int nb) {
             if (!(flags[k] & (kFlagGateDisp << t))) b->gatesAll &= ~(1u << t);
         b->alchAny |= (unsigned)(flags[k] & 7);
     }
-    // the pair kernel takes the tiles largest first (see kTileOrder), here ordered once on the host
+    // the pair kernel takes the tiles largest first, here ordered once on the host
     std::vector<int> tileOrder(b->numTiles), tilePairs(b->numTiles, 0);
     for (int t = 0; t < b->numTiles; t++) {
         tileOrder[t] = t;

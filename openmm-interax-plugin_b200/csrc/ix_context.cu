@@ -320,7 +320,9 @@ struct ix_ctx {
     // state that a captured launch depends on (parameters, box, buffers, settings) bumps the version
     bool useGraphs = true;
     unsigned long long version = 1;
-    LaunchGraph graphCompute, graphDevice, graphMd, graphPosq;
+    LaunchGraph graphCompute, graphDevice, graphMd, graphMdSeveral, graphPosq;
+    unsigned long long mdGraphVersion = 0;   // version of the captures that mdGraphRun steps have replayed
+    int mdGraphRun = 0;
     std::vector<LaunchGraph> graphWindows;  // evaluations at window values of one parameter, one graph per value
     size_t windowNext = 0;                  // slot replaced next when graphWindows is full
 };
@@ -1403,6 +1405,10 @@ struct StepKick {
     bool started = true;     // the step's first kernel checked the displacement and refreshed the sorted positions
 };
 
+// Whether the kernels of an evaluation are set up behind one another: not with kernel times, whose events lie between
+// them, nor in large systems.
+static bool launchesEarly(const ix_ctx* ctx) { return !ctx->profiling && (ctx->n + 31) / 32 <= kEarlyLaunchBlocks; }
+
 // `kick`: an MD step whose first kernel (kStepStart) has already moved the particles, checked their displacement and
 // refreshed the pair list's sorted positions; the evaluation ends with the second half kick.
 static int launchEvaluation(ix_ctx* ctx, unsigned terms, double* outForces, double* outEnergy, long long* addFixed,
@@ -1411,8 +1417,7 @@ static int launchEvaluation(ix_ctx* ctx, unsigned terms, double* outForces, doub
     cudaStream_t st = ctx->stream;
     const bool doPair = (terms & 7u) != 0;
     const bool doAtm = (terms & 8u) != 0;
-    // not with kernel times, whose events lie between the kernels, nor in large systems
-    const bool early = !ctx->profiling && (n + 31) / 32 <= kEarlyLaunchBlocks;
+    const bool early = launchesEarly(ctx);
     IX_TRY(stageUploads(ctx, terms));
     // the three-body chain runs on a second stream, concurrently with the pair list and pair kernel
     const bool fork = doPair && doAtm && !ctx->serialize;
@@ -1472,10 +1477,11 @@ static int launchEvaluation(ix_ctx* ctx, unsigned terms, double* outForces, doub
                    std::min(ctx->numSMs * 4, std::max(1, (L.tileCap + kListWarps - 1) / kListWarps)), kListThreads, 0,
                    L, ctx->G);
         ctx->launches += ctx->G.periodic ? 5 : 6;
-        // the pair kernel's persistent grid fills the SMs: the triple kernel, ready at the same time and on a stream of
+        const bool small = L.nb <= kSmallBlocks;
+        // the pair kernel's persistent grid fills the SMs (not in a small system): the triple kernel, ready at the same time and on a stream of
         // higher priority, is placed first (it was left to the end of the pair kernel when its chain came a microsecond
         // later: 139 us for the two instead of 112)
-        if (fork) IX_CUDA(ctx, cudaStreamWaitEvent(st, ctx->evFork, 0));
+        if (fork && !small) IX_CUDA(ctx, cudaStreamWaitEvent(st, ctx->evFork, 0));
         PairTermConfig C = pairConfig(ctx, terms);
         // the lean instantiation when no selected term has a soft core, a switching function or the order-2 overlap
         bool lean = true;
@@ -1501,7 +1507,7 @@ static int launchEvaluation(ix_ctx* ctx, unsigned terms, double* outForces, doub
         const size_t dyn = table && tableBytes <= (size_t)IX_TUNE_PAIR_SHARED_TABLE_BYTES ? tableBytes : 0;
         P.coefShared = dyn > 0;
         C.coefShared = P.coefShared;
-        launchPairTiles(early && ctx->L.nb <= kSmallBlocks, lean, table, uniform, ctx->L.nb <= kSmallBlocks, grid, L.tileCap, dyn, st, L, P, C);
+        launchPairTiles(early && small, lean, table, uniform, small, grid, L.tileCap, dyn, st, L, P, C);
         ctx->launches += 1;
         recordTiming(ctx, 1, st);
         ctx->evPair = ctx->profiling;
@@ -1633,7 +1639,6 @@ static int launchGraph(ix_ctx* ctx, LaunchGraph& g, const GraphKey& key, F&& enq
             if (rc != IX_OK) return rc;
             return fail(ctx, IX_ERR_CUDA, "stream capture failed: %s", cudaGetErrorString(e));
         }
-        // a new instantiation (the conditional nodes' handles belong to the captured graph)
         if (g.exec) {
             cudaGraphExecDestroy(g.exec);
             g.exec = nullptr;
@@ -1870,6 +1875,7 @@ void ix_ctx_destroy(ix_ctx* ctx) {
     releaseGraph(ctx->graphCompute);
     releaseGraph(ctx->graphDevice);
     releaseGraph(ctx->graphMd);
+    releaseGraph(ctx->graphMdSeveral);
     releaseGraph(ctx->graphPosq);
     for (auto& g : ctx->graphWindows) releaseGraph(g);
     for (auto& kv : ctx->buffers) arenaFree(ctx->arena, kv.second.p);
@@ -2445,6 +2451,11 @@ int ix_get_kernel_times(ix_ctx* ctx, double* pair_ms, double* three_body_ms) {
 
 }  // extern "C"
 
+// A long run replays a graph of several steps: the next graph's first kernel starts 2 to 3 us after the last one's end
+// (100 steps of 648 atoms in graphs of 1, 5, 8 and 20 steps: 3750, 3520, 3490 and 3450 us).  Capturing eight steps takes
+// about 1.2 ms, for a run's first kMdGraphRun steps more than they would save, so those replay a graph of one.
+constexpr int kMdGraphSteps = 8, kMdGraphRun = 512;
+
 // Enqueue velocity-Verlet steps on the context's stream without synchronizing.
 static int enqueueSteps(ix_ctx* ctx, int num_steps, double dt) {
     unsigned terms = selectedTerms(ctx, -1);
@@ -2468,6 +2479,7 @@ static int enqueueSteps(ix_ctx* ctx, int num_steps, double dt) {
     // one step: the first half kick and drift (fused with the list's displacement check and position refresh when
     // there are pair terms), the evaluation at the new positions, whose finishing kernel applies the second half kick
     const int clusterGrid = (ctx->K.num + kClusterBlock - 1) / kClusterBlock;
+    const bool early = launchesEarly(ctx);
     auto step = [&]() -> int {
         if (!terms) {
             if (ctx->numConstraints)
@@ -2490,27 +2502,40 @@ static int enqueueSteps(ix_ctx* ctx, int num_steps, double dt) {
         if (ctx->numConstraints) {
             // the constrained clusters move together, and refresh the pair list's sorted positions with the
             // displacement check as kStepStart does
-            kConstrainedDrift<<<clusterGrid, kClusterBlock, 0, ctx->stream>>>(
-                ctx->K, dt, ctx->dInvMass, ctx->dOutForces, ctx->dVel, ctx->dPos, ctx->L, (terms & 7u) != 0,
+            launchNext(early, ctx->stream, kConstrainedDrift, clusterGrid, kClusterBlock, 0, ctx->K, dt, ctx->dInvMass, ctx->dOutForces, ctx->dVel, ctx->dPos, ctx->L, (terms & 7u) != 0,
                 0.25f * kPairSkin * kPairSkin);
         }
         else if (terms & 7u)
             // 128-thread blocks: a latency-bound gather by particle, spread over every SM
-            kStepStart<<<(n + 127) / 128, 128, 0, ctx->stream>>>(ctx->L, ctx->dPos, dt, ctx->dInvMass, ctx->dOutForces,
-                                                                ctx->dVel, 0.25f * kPairSkin * kPairSkin);
+            launchNext(early, ctx->stream, kStepStart, (n + 127) / 128, 128, 0, ctx->L, ctx->dPos, dt, ctx->dInvMass,
+                       ctx->dOutForces, ctx->dVel, 0.25f * kPairSkin * kPairSkin);
         else
             kVerletFirstHalf<<<g, 256, 0, ctx->stream>>>(n, dt, ctx->dInvMass, ctx->dOutForces, ctx->dVel, ctx->dPos);
         ctx->launches += 1;
         IX_TRY(launchEvaluation(ctx, terms, ctx->dOutForces, ctx->dOutEnergy, nullptr, 0, &kick));
         if (ctx->numConstraints) {
-            launchNext(true, ctx->stream, kConstrainVelocities, clusterGrid, kClusterBlock, 0, ctx->K, ctx->dInvMass,
+            launchNext(early, ctx->stream, kConstrainVelocities, clusterGrid, kClusterBlock, 0, ctx->K, ctx->dInvMass,
                        ctx->dPos, ctx->dVel);
             ctx->launches += 1;
         }
         IX_CUDA(ctx, cudaGetLastError());
         return IX_OK;
     };
-    for (int s = 0; s < num_steps; s++) IX_TRY(launchGraph(ctx, ctx->graphMd, key, step));
+    auto several = [&]() -> int {
+        for (int k = 0; k < kMdGraphSteps; k++) IX_TRY(step());
+        return IX_OK;
+    };
+    if (ctx->mdGraphVersion != ctx->version) {
+        ctx->mdGraphVersion = ctx->version;
+        ctx->mdGraphRun = 0;
+    }
+    for (int s = 0; s < num_steps;) {
+        const bool long_run = ctx->mdGraphRun >= kMdGraphRun && num_steps - s >= kMdGraphSteps;
+        if (long_run) IX_TRY(launchGraph(ctx, ctx->graphMdSeveral, key, several));
+        else IX_TRY(launchGraph(ctx, ctx->graphMd, key, step));
+        s += long_run ? kMdGraphSteps : 1;
+        if (!long_run) ctx->mdGraphRun = std::min(ctx->mdGraphRun + 1, kMdGraphRun);
+    }
     IX_CUDA(ctx, cudaGetLastError());
     return IX_OK;
 }

@@ -358,7 +358,7 @@ __device__ __forceinline__ void constrainClusterVelocities(ConstraintClusters K,
 // Velocities of each constrained cluster with the components along its bonds removed (no bond stretches), after the
 // second half kick: one linear solve of the cluster's multipliers and at most two refinements of the residual.
 __global__ void kConstrainVelocities(ConstraintClusters K, const double* invMass, const double* pos, double* vel) {
-    dependentStart(false);
+    dependentStart(K.num <= kEarlySites);
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= K.num) return;
     const int c0 = K.constraintStart[c], nc = K.constraintStart[c + 1] - c0;

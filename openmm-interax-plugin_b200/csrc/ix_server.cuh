@@ -363,7 +363,7 @@ void retireContext(ix_server* S, ServerShard* H, ix_ctx* c) {
     }
     {
         std::lock_guard<std::mutex> lock(S->graveM);
-        for (LaunchGraph* g : {&c->graphCompute, &c->graphDevice, &c->graphMd})
+        for (LaunchGraph* g : {&c->graphCompute, &c->graphDevice, &c->graphMd, &c->graphMdSeveral})
             if (g->exec) {
                 S->grave.push_back(g->exec);
                 g->exec = nullptr;
