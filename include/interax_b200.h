@@ -237,6 +237,11 @@ int ix_get_launch_count(ix_ctx* ctx, long long* launches);
  * are identical.  No counterpart in the reference (OpenMM launches kernels one by one). */
 int ix_set_graphs(ix_ctx* ctx, int enable);
 
+/* An evaluation's flags, energies and counts come back through a page-locked slot of the context (default), or, where
+ * the host has no page-locked memory left, through ordinary memory.  enable = 0 takes the second way; the results are
+ * identical.  A test aid with no counterpart in the reference. */
+int ix_set_pinned_status(ix_ctx* ctx, int enable);
+
 /* The context evaluated at several values of one alchemical parameter (lambda windows; the other parameters keep
  * their values, and the parameter's own value is restored).  energies: num_windows x 4 term energies; forces:
  * num_windows x num_particles x 3 (may be NULL).  Host buffers, synchronous.  Every term is linear in the parameter

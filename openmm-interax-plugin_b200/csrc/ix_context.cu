@@ -217,6 +217,7 @@ struct ix_ctx {
     std::vector<double> requestPos, requestVel, requestMass;   // starting state of a server request description
     char* uploadBuf = nullptr;           // pinned host staging of a server's context (null: pageable copies)
     unsigned char* hostStatus = nullptr; // pinned host copy of the status block (flags, energies, counts)
+    bool pinnedStatus = true;            // false: never taken (ix_set_pinned_status)
     size_t uploadCap = 0, uploadUsed = 0;
     cudaStream_t stream = nullptr;
     cudaStream_t stream2 = nullptr;      // the three-body chain, forked from and joined back into `stream`
@@ -2089,6 +2090,13 @@ static int readCounts(ix_ctx* ctx, unsigned terms) {
     return IX_OK;
 }
 
+// The context's page-locked copy of its status block, or null (none left, or ix_set_pinned_status).
+static unsigned char* statusSlot(ix_ctx* ctx) {
+    if (!ctx->pinnedStatus) return nullptr;
+    if (!ctx->hostStatus) ctx->hostStatus = pinnedSlots().take();
+    return ctx->hostStatus;
+}
+
 // One evaluation of the selected terms at the current positions and parameters, left on the device: forces in
 // dOutForces, term energies copied to e.  Grows the neighbor lists and repeats on an overflow.
 static int evaluateResident(ix_ctx* ctx, unsigned terms, double e[4], LaunchGraph* graph = nullptr,
@@ -2096,8 +2104,7 @@ static int evaluateResident(ix_ctx* ctx, unsigned terms, double e[4], LaunchGrap
     for (int t = 0; t < 4; t++) e[t] = 0.0;
     if (!terms) return IX_OK;
     IX_TRY(prepare(ctx, terms));
-    if (!ctx->hostStatus) ctx->hostStatus = pinnedSlots().take();
-    unsigned char* hs = ctx->hostStatus;
+    unsigned char* hs = statusSlot(ctx);
     for (int attempt = 0; attempt < 4; attempt++) {
         IX_TRY(enqueueResident(ctx, terms, graph ? *graph : ctx->graphCompute, param));
         // the status block and the forces come back with the evaluation; one wait for all of it
@@ -2585,6 +2592,12 @@ int ix_set_graphs(ix_ctx* ctx, int enable) {
     return IX_OK;
 }
 
+int ix_set_pinned_status(ix_ctx* ctx, int enable) {
+    if (!ctx) return IX_ERR_INVALID;
+    ctx->pinnedStatus = enable != 0;
+    return IX_OK;
+}
+
 // out[w] = (accumulate ? out[w] : 0) + f0 + lambda_w (f1 - f0): the forces of terms linear in the window parameter at
 // each window, FP64, n x 3 per window.
 __global__ void kWindowForces(size_t n3, int num_windows, const double* __restrict__ lambdas,
@@ -2753,23 +2766,15 @@ static int alchemicalWindows(ix_ctx* ctx, const std::string& name, unsigned depe
         bumpVersion(ctx);
         return IX_OK;
     }
-    // everything at 0: forces in dOutForces, energies and counts in the status block, the lists built for these positions
-    double e0[4] = {0, 0, 0, 0};
-    long long pairs = 0, triples = 0;
+    // everything at 0: forces in dOutForces, the lists built for these positions, and the status block (flags, energies,
+    // counts) as this evaluation left it.  The lists that overflowed grow only after the last kernel here: a site list
+    // that has grown holds nothing before its next build, while those that overflowed are known by their counts.
     ctx->parameters[name] = 0.0;
-    if (!ctx->hostStatus) ctx->hostStatus = pinnedSlots().take();
-    unsigned char* hs = ctx->hostStatus;
-    LaunchGraph& graph = windowGraph(ctx, terms, 0.0);
-    if (hs) {
-        IX_TRY(enqueueResident(ctx, terms, graph, 0.0));
-        IX_CUDA(ctx, cudaMemcpyAsync(hs, ctx->dFlags, kStatusBytes, cudaMemcpyDeviceToHost, st));
-    }
-    else {
-        IX_TRY(evaluateResident(ctx, terms, e0, &graph, 0.0));
-        pairs = ctx->lastPairs;
-        triples = ctx->lastTriples;
-        IX_TRY(windowBuffers(ctx, num_windows, passes, softcore, slope && d_forces, B));   // the tile list may have grown
-    }
+    unsigned char ordinary[kStatusBytes];
+    unsigned char* hs = statusSlot(ctx);
+    if (!hs) hs = ordinary;
+    IX_TRY(enqueueResident(ctx, terms, windowGraph(ctx, terms, 0.0), 0.0));
+    IX_CUDA(ctx, cudaMemcpyAsync(hs, ctx->dFlags, kStatusBytes, cudaMemcpyDeviceToHost, st));
     IX_TRY(stageCopy(ctx, B.lambda, values, num_windows * sizeof(double)));
     ctx->parameters[name] = 1.0;
     // the alchemical triples at 1, beside the pairs
@@ -2842,17 +2847,18 @@ static int alchemicalWindows(ix_ctx* ctx, const std::string& name, unsigned depe
     std::vector<double> report(6 + 3 * (size_t)passes, 0.0);
     IX_CUDA(ctx, cudaMemcpyAsync(report.data(), B.report, report.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
     IX_CUDA(ctx, cudaStreamSynchronize(st));
-    if (hs) {
-        IX_TRY(checkOverflowFlags(ctx, terms, reinterpret_cast<const int*>(hs), redo));
-        if (redo) return IX_OK;
-        unsigned long long c[2];
-        std::memcpy(e0, hs + 32, sizeof(e0));
-        std::memcpy(c, hs + 64 + 2 * sizeof(unsigned long long), sizeof(c));
-        for (int t = 0; t < 4; t++)
-            if (!((terms >> t) & 1u)) e0[t] = 0.0;
-        pairs = (terms & 7u) ? (long long)c[0] : 0;
-        triples = (terms & 8u) ? (long long)c[1] : 0;
-    }
+    int flags[8];
+    std::memcpy(flags, hs, sizeof(flags));
+    IX_TRY(checkOverflowFlags(ctx, terms, flags, redo));
+    if (redo) return IX_OK;
+    double e0[4];
+    unsigned long long counts[2];
+    std::memcpy(e0, hs + 32, sizeof(e0));
+    std::memcpy(counts, hs + 64 + 2 * sizeof(unsigned long long), sizeof(counts));
+    for (int t = 0; t < 4; t++)
+        if (!((terms >> t) & 1u)) e0[t] = 0.0;
+    const long long pairs = (terms & 7u) ? (long long)counts[0] : 0;
+    long long triples = (terms & 8u) ? (long long)counts[1] : 0;
     const PairTerm& D = ctx->term[0];
     const double lrc = (dependent & 1u) && D.lrcAlchCoef != 0 ? D.lrcAlchCoef / (ctx->box[0] * ctx->box[4] * ctx->box[8]) : 0.0;
     for (int w = 0; w < num_windows; w++) {
