@@ -757,20 +757,37 @@ static int uploadPairParams(ix_ctx* ctx) {
     return IX_OK;
 }
 
+// Particles per nm3 of the system, by its box or as a liquid.
+static double particleDensity(const ix_ctx* ctx) {
+    const double volume = ctx->method == IX_CUTOFF_PERIODIC ? ctx->box[0] * ctx->box[4] * ctx->box[8]
+                                                            : std::max(1.0, ctx->n / 100.0);   // extent unknown
+    return ctx->n / volume;
+}
+
+// Volume within c of a cube of edge e.
+static double dilatedCube(double e, double c) {
+    return e * e * e + 6 * e * e * c + 3 * M_PI * e * c * c + 4.0 / 3.0 * M_PI * c * c * c;
+}
+
 // Estimated number of tiles of the list (the build reports overflows, and the host then grows the buffers).
 static long long estimateTiles(const ix_ctx* ctx, int nb) {
     if (ctx->method == IX_NO_CUTOFF) return (long long)nb * (nb + 1) / 2 + nb;
-    double volume;
-    if (ctx->method == IX_CUTOFF_PERIODIC) volume = ctx->box[0] * ctx->box[4] * ctx->box[8];
-    else volume = std::max(1.0, ctx->n / 100.0);   // unknown extent: assume liquid density
-    double rho = ctx->n / volume;
-    double e = std::cbrt(32.0 / rho);
-    double c = ctx->cutoff + kPairSkin;
-    double dil = e * e * e + 6 * e * e * c + 3 * M_PI * e * c * c + 4.0 / 3.0 * M_PI * c * c * c;
+    const double rho = particleDensity(ctx);
+    const double dil = dilatedCube(std::cbrt(32.0 / rho), ctx->cutoff + kPairSkin);
     double perBlock = std::min<double>(rho * dil, ctx->n) / 32.0 / 2.0 + 2.0;
     long long est = (long long)(1.5 * nb * perBlock) + 64;
     long long full = (long long)nb * (nb + 1) / 2 + nb;
     return std::min(est, full);
+}
+
+// Entries the list search keeps per i-block: half as many again as there are blocks within the list cutoff of one, and
+// not under 384 (the elongated blocks of a liquid have up to 250 with a 1 nm cutoff).  A block that has more keeps marks
+// in their place.
+static int listEntries(const ix_ctx* ctx, int nb) {
+    if (ctx->method == IX_NO_CUTOFF) return 1;      // every block is listed
+    const double rho = particleDensity(ctx);
+    const double near = rho / 32.0 * dilatedCube(2.0 * std::cbrt(32.0 / rho), ctx->cutoff + kPairSkin);
+    return (int)std::min<double>(nb, std::max(384.0, 1.5 * near));
 }
 
 static int allocatePair(ix_ctx* ctx, long long tileCap) {
@@ -845,11 +862,11 @@ static int allocatePair(ix_ctx* ctx, long long tileCap) {
     IX_TRY(deviceAlloc(ctx, "bbox", 2 * (size_t)nb, &L.bbox));
     IX_TRY(deviceAlloc(ctx, "blockAtoms", nb, &L.blockAtoms));
     IX_TRY(deviceAlloc(ctx, "blockTiles", nb + 1, &L.blockTiles));
-    // an i-block of a liquid has at most about 250 candidate blocks
-    L.entryCap = G.useCutoff ? std::min(nb, 384) : nb;
+    if (tileCap > (long long)1 << 26) return fail(ctx, IX_ERR_INVALID, "neighbor list too large (%lld tiles)", tileCap);
+    L.entryCap = listEntries(ctx, nb);
+    L.markStride = std::max(1, ((nb + kMarkBlocks - 1) / kMarkBlocks + 4 * L.entryCap - 1) / (4 * L.entryCap));
     IX_TRY(deviceAlloc(ctx, "blockEntries", nb, &L.blockEntries));
     IX_TRY(deviceAlloc(ctx, "entries", (size_t)nb * L.entryCap, &L.entries));
-    if (tileCap > (long long)1 << 26) return fail(ctx, IX_ERR_INVALID, "neighbor list too large (%lld tiles)", tileCap);
     ctx->tileCap = (int)tileCap;
     L.tileCap = (int)tileCap;
     IX_TRY(deviceAlloc(ctx, "tileJ", 32 * (size_t)L.tileCap, &L.tileJ));

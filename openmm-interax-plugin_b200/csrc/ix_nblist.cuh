@@ -71,6 +71,7 @@ struct ListBuffers {
     int* blockEntries;          // nb: candidate blocks of each i-block
     int4* entries;              // nb x entryCap: (block J, mask of its candidate particles, candidates before them)
     int entryCap;
+    int markStride;             // a row of `entries` holds 4 x entryCap marks, one for each kMarkBlocks x markStride blocks
     int* blockTiles;            // nb + 1: exclusive scan of the tile counts, then the total
     int* tileJ;                 // tileCap x 32
     int* tileIBlock;            // tileCap
@@ -386,6 +387,11 @@ __device__ __forceinline__ float pointBoxDist2(float4 p, float4 ci, float4 ei, c
     return boxBoxDist2(ci, ei, p, make_float4(0, 0, 0, 0), G);
 }
 
+// Whether every block pairs with every block after it: without a cutoff, and in a triclinic box, where nothing is pruned.
+__device__ __forceinline__ bool everyBlockListed(const ListGeometry& G) {
+    return !G.useCutoff || (G.periodic && G.box.triclinic);
+}
+
 __device__ __forceinline__ bool isExcluded(const ListBuffers& L, int oi, int oj) {
     int2 range = L.exclRange[oi];
     if (oj < range.x || oj > range.y) return false;
@@ -402,58 +408,82 @@ __device__ __forceinline__ bool isExcluded(const ListBuffers& L, int oi, int oj)
 
 constexpr int kListThreads = 256;
 constexpr int kListWarps = kListThreads / 32;
+constexpr int kMarkBlocks = 32;        // what a warp of kListBlocks tests at a time
 
 // The candidates of each i-block: the particles of the blocks J >= I whose box is within the list cutoff of block I's box
 // and whose own position is within it too, in the order (J, slot).  One thread block per i-block: the blocks are
 // examined 256 at a time, each thread testing one block's box; the candidate blocks are compacted in block order and
 // the warps take them round robin for the particle tests (neighbors along the curve are neighbors in space, so
 // contiguous shares would be uneven: 37 us for 24,000 atoms).  The entries hold what the mask kernel needs to find the
-// candidates of a tile; a second pass over the same candidates to write the tiles had taken 15.6 us.  The last block
+// candidates of a tile; a second pass over the same candidates to write the tiles had taken 15.6 us.  A block with more
+// candidate blocks than its row holds keeps marks there instead: the number of its candidates before every kMarkBlocks *
+// markStride blocks from its own on, from which the mask kernel searches again.  Where every block is listed
+// (everyBlockListed) there is nothing to search.  The last block
 // scans the tile counts.  On overflow no tile is scheduled (nothing is written beyond the buffers); the host grows
 // them and evaluates again.
 __global__ void __launch_bounds__(kListThreads) kListBlocks(ListBuffers L, ListGeometry G) {
     dependentStart(L.nb <= kEarlyBlocks);
     if (!rebuildRequested(L)) return;
-    __shared__ int candJ[kListThreads];
+    __shared__ int candJ[kListThreads], prefix[kListThreads];
     __shared__ unsigned keep[kListThreads];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const float cut2 = G.useCutoff ? G.listCutoff * G.listCutoff : INFINITY;
+    const float cut2 = G.listCutoff * G.listCutoff;
     for (int I = blockIdx.x; I < L.nb; I += gridDim.x) {
+        if (everyBlockListed(G)) {
+            if (tid == 0) L.blockAtoms[I] = L.n - 32 * I;
+            continue;
+        }
         const float4 ci = L.bbox[2 * I], ei = L.bbox[2 * I + 1];
         int atoms = 0, entries = 0;
-        for (int Jc = I; Jc < L.nb; Jc += kListThreads) {
-            // the candidate blocks of this chunk, in block order
-            const int J = Jc + tid;
-            const bool cand = J < L.nb && boxBoxDist2(ci, ei, L.bbox[2 * J], L.bbox[2 * J + 1], G) < cut2;
-            int total;
-            const int at = blockPrefix<kListThreads>(cand, total);
-            if (cand) candJ[at] = J;
-            __syncthreads();
-            // the particle tests of the candidate blocks, four blocks' loads in flight
-            for (int k0 = warp; k0 < total; k0 += 4 * kListWarps) {
-                float4 p[4];
+        // the entries, or, of a block that has more than its row holds, in a second pass the row's marks
+        for (int pass = 0; pass < 2; pass++) {
+            atoms = entries = 0;
+            for (int Jc = I; Jc < L.nb; Jc += kListThreads) {
+                // the candidate blocks of this chunk, in block order
+                const int J = Jc + tid;
+                const bool cand = J < L.nb && boxBoxDist2(ci, ei, L.bbox[2 * J], L.bbox[2 * J + 1], G) < cut2;
+                int total;
+                const int at = blockPrefix<kListThreads>(cand, total);
+                if (cand) candJ[at] = J;
+                __syncthreads();
+                // the particle tests of the candidate blocks, four blocks' loads in flight
+                for (int k0 = warp; k0 < total; k0 += 4 * kListWarps) {
+                    float4 p[4];
 #pragma unroll
-                for (int u = 0; u < 4; u++) p[u] = L.sposf[32 * candJ[min(k0 + u * kListWarps, total - 1)] + lane];
+                    for (int u = 0; u < 4; u++) p[u] = L.sposf[32 * candJ[min(k0 + u * kListWarps, total - 1)] + lane];
 #pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const int k = k0 + u * kListWarps;
-                    const bool in = k < total && 32 * candJ[min(k, total - 1)] + lane < L.n &&
-                                    (!G.useCutoff || pointBoxDist2(p[u], ci, ei, G) < cut2);
-                    const unsigned m = __ballot_sync(0xffffffffu, in);
-                    if (lane == 0 && k < total) keep[k] = m;
+                    for (int u = 0; u < 4; u++) {
+                        const int k = k0 + u * kListWarps;
+                        const bool in = k < total && 32 * candJ[min(k, total - 1)] + lane < L.n &&
+                                        pointBoxDist2(p[u], ci, ei, G) < cut2;
+                        const unsigned m = __ballot_sync(0xffffffffu, in);
+                        if (lane == 0 && k < total) keep[k] = m;
+                    }
                 }
+                __syncthreads();
+                // entries (in the upper bits) and candidates of the chunk before each candidate block
+                const unsigned m = tid < total ? keep[tid] : 0u;
+                int sum;
+                const int before = blockPrefix<kListThreads>(__popc(m) + (m ? 1 << 16 : 0), sum);
+                if (pass == 0) {
+                    const int e = entries + (before >> 16);
+                    if (m && e < L.entryCap)
+                        L.entries[(size_t)I * L.entryCap + e] = make_int4(candJ[tid], (int)m, atoms + (before & 0xffff), 0);
+                }
+                else {
+                    prefix[tid] = before & 0xffff;
+                    __syncthreads();
+                    // each warp the 32 blocks it tested first: `at` is their first place among the candidate blocks
+                    const int group = (J - I) / kMarkBlocks;
+                    if (lane == 0 && J < L.nb && group % L.markStride == 0)
+                        reinterpret_cast<int*>(L.entries + (size_t)I * L.entryCap)[group / L.markStride] =
+                            atoms + (at < total ? prefix[at] : sum & 0xffff);
+                }
+                entries += sum >> 16;
+                atoms += sum & 0xffff;
+                __syncthreads();   // the shared arrays are refilled by the next chunk
             }
-            __syncthreads();
-            // entries (in the upper bits) and candidates of the chunk before each candidate block
-            const unsigned m = tid < total ? keep[tid] : 0u;
-            int sum;
-            const int before = blockPrefix<kListThreads>(__popc(m) + (m ? 1 << 16 : 0), sum);
-            const int e = entries + (before >> 16);
-            if (m && e < L.entryCap)
-                L.entries[(size_t)I * L.entryCap + e] = make_int4(candJ[tid], (int)m, atoms + (before & 0xffff), 0);
-            entries += sum >> 16;
-            atoms += sum & 0xffff;
-            __syncthreads();   // the shared arrays are refilled by the next chunk
+            if (entries <= L.entryCap) break;
         }
         if (tid == 0) {
             L.blockAtoms[I] = atoms;
@@ -480,13 +510,12 @@ __global__ void __launch_bounds__(kListThreads) kListBlocks(ListBuffers L, ListG
     }
 }
 
-// The i-block of tile t: the last whose first tile is at or before t and that has tiles (a 32-way search by a warp).
-__device__ __forceinline__ int tileBlock(const ListBuffers& L, int t, int lane) {
-    int lo = 0, n = L.nb + 1;                        // blockTiles[lo] <= t < blockTiles[lo + n]
+// The last of the n ascending marks that is at most `value` (the first always is), by a warp.
+__device__ __forceinline__ int lastMark(const int* marks, int n, int value, int lane) {
+    int lo = 0;
     while (n > 1) {
         const int step = (n + 31) / 32;
-        const int at = lo + lane * step;
-        const unsigned below = __ballot_sync(0xffffffffu, lane * step < n && L.blockTiles[at] <= t);
+        const unsigned below = __ballot_sync(0xffffffffu, lane * step < n && marks[lo + lane * step] <= value);
         const int k = 31 - __clz(below);             // lane 0 always holds
         lo += k * step;
         n = min(step, n - k * step);
@@ -494,10 +523,28 @@ __device__ __forceinline__ int tileBlock(const ListBuffers& L, int t, int lane) 
     return lo;
 }
 
-// The candidates first .. first + 31 of i-block I to slots[0..31] (-1 after the last), by one warp: from the entries,
-// or by the search again where they did not fit (only in a box of very uneven density).
+// The i-block of tile t: the last whose first tile is at or before t and that has tiles (its first tile differs from the
+// next block's, and the last of equals is taken).
+__device__ __forceinline__ int tileBlock(const ListBuffers& L, int t, int lane) {
+    return lastMark(L.blockTiles, L.nb + 1, t, lane);
+}
+
+// The candidates first .. first + 31 of i-block I to slots[0..31] (-1 after the last), by one warp: where every block is
+// listed, block I + first / 32 as it is; else from the entries, or, where they did not fit, by the search again from the
+// last mark before them.  Without the marks each tile searched from block I on, which is cubic in the number of blocks:
+// an evaluation with a rebuild of 96,000 atoms took 169 ms in a triclinic box (whose blocks are all listed) and takes
+// 10.8, and 15.2 ms with a cutoff of 2.6 nm, of 24,000 atoms 3.2 and 4.0 ms; they take 6.2, 0.83 and 1.7 ms (with rows
+// of 384 entries, and so from the marks, 6.6 and 1.84 ms for the long cutoff).
 __device__ __forceinline__ void tileCandidates(const ListBuffers& L, const ListGeometry& G, int I, int first, int lane,
                                                int* slots) {
+    if (everyBlockListed(G)) {
+        const int J = I + first / 32, j = 32 * J + lane;
+        // (without a cutoff a distance beyond the range of a float leaves the block out)
+        const bool near = boxBoxDist2(L.bbox[2 * I], L.bbox[2 * I + 1], L.bbox[2 * J], L.bbox[2 * J + 1], G) < INFINITY;
+        slots[lane] = near && j < L.n ? j : -1;
+        __syncwarp();
+        return;
+    }
     const unsigned lt = laneMaskLt();
     slots[lane] = -1;
     __syncwarp();
@@ -506,8 +553,8 @@ __device__ __forceinline__ void tileCandidates(const ListBuffers& L, const ListG
         if (((m >> lane) & 1u) && q >= 0 && q < 32) slots[q] = 32 * J + lane;
     };
     const int n = L.blockEntries[I];
+    const int4* E = L.entries + (size_t)I * L.entryCap;
     if (n <= L.entryCap) {
-        const int4* E = L.entries + (size_t)I * L.entryCap;
         for (int e0 = 0; e0 < n; e0 += 32) {
             const int4 v = e0 + lane < n ? E[e0 + lane] : make_int4(0, 0, INT_MAX, 0);
             const bool after = v.z >= first + 32, mine = !after && v.z + __popc((unsigned)v.y) > first;
@@ -521,17 +568,30 @@ __device__ __forceinline__ void tileCandidates(const ListBuffers& L, const ListG
     }
     else {
         const float4 ci = L.bbox[2 * I], ei = L.bbox[2 * I + 1];
-        const float cut2 = G.useCutoff ? G.listCutoff * G.listCutoff : INFINITY;
-        int before = 0;
-        for (int Jc = I; Jc < L.nb && before < first + 32; Jc += 32) {
+        const float cut2 = G.listCutoff * G.listCutoff;
+        const int* marks = reinterpret_cast<const int*>(E);
+        const int between = kMarkBlocks * L.markStride;
+        const int k = lastMark(marks, (L.nb - I + between - 1) / between, first, lane);
+        int before = marks[k];
+        for (int Jc = I + k * between; Jc < L.nb && before < first + 32; Jc += 32) {
             const int J = Jc + lane;
             const bool near = J < L.nb && boxBoxDist2(ci, ei, L.bbox[2 * J], L.bbox[2 * J + 1], G) < cut2;
-            for (unsigned todo = __ballot_sync(0xffffffffu, near); todo; todo &= todo - 1) {
-                const int K = Jc + __ffs(todo) - 1, j = 32 * K + lane;
-                const bool in = j < L.n && (!G.useCutoff || pointBoxDist2(L.sposf[j], ci, ei, G) < cut2);
-                const unsigned m = __ballot_sync(0xffffffffu, in);
-                take(K, m, before - first);
-                before += __popc(m);
+            for (unsigned todo = __ballot_sync(0xffffffffu, near); todo && before < first + 32;) {
+                // four blocks' loads in flight
+                int K[4];
+                float4 p[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    K[u] = todo ? Jc + __ffs(todo) - 1 : L.nb;
+                    todo &= todo - 1;
+                    p[u] = L.sposf[32 * min(K[u], L.nb - 1) + lane];
+                }
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const unsigned m = __ballot_sync(0xffffffffu, 32 * K[u] + lane < L.n && pointBoxDist2(p[u], ci, ei, G) < cut2);
+                    take(K[u], m, before - first);
+                    before += __popc(m);
+                }
             }
         }
     }
