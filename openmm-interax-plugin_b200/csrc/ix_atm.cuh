@@ -466,10 +466,11 @@ __device__ __forceinline__ void storeNeighbor(TripleStorage<DAMP, N>& S, const A
                                               const float4& pa, int slot, int b, float x, float y, float z) {
     const float4 p = A.siteParams[b];
     const float u = fmaf(x, x, fmaf(y, y, z * z));
+    const float sum = pa.y + p.y, inv = rcpApprox(sum), product = p.x * p.y, g = product * inv;
     S.pos[slot] = make_float4(x, y, z, u);
     // C9 = 3/2 aA aB aC wA wB wC (wA + wB + wC)/((wA + wB)(wB + wC)(wC + wA)) (InteraxThreeBodyForceImpl.h:69-72)
     //    = (3/2 aA wA) gB gC (1 + wA/(wB + wC)),  g = a w/(wA + w)
-    S.par[slot] = make_float4(p.y, __fdividef(p.x * p.y, pa.y + p.y), p.w, __int_as_float(A.molecule[b]));
+    S.par[slot] = make_float4(p.y, fmaf(fmaf(-sum, g, product), inv, g), p.w, __int_as_float(A.molecule[b]));
     S.site[slot] = b;
     if (DAMP) {
         SiteDamping d;
@@ -483,12 +484,16 @@ __device__ __forceinline__ void storeNeighbor(TripleStorage<DAMP, N>& S, const A
 // cStep, ... (8 at a time, below cEnd), each against every neighbor B of entries [bBegin, bEnd).  Four lanes take one
 // C; lane s of them takes B = bBegin + s, + 4, ...  A triple is visited from both sides, and each visit adds the
 // force on its own C only: the same number of warp iterations as visiting it once with half of the lanes idle, and
-// a third of the arithmetic of all three forces.  The force on A is minus the sum of the others'.
+// a third of the arithmetic of all three forces.  The force on A is minus the sum of the others', in fixed point.
 //   energy (InteraxThreeBodyTerms.h:97-146), with a = AB, b = AC, c = BC, p = a.b, q = a.c, s = b.c, P = (a b c)^2:
 //     E = C9 (P^-3/2 - 3 p q s P^-5/2)
 //     -force on C = b (R/b^2 + t) + c (R/c^2 + t) + a X s (p + q),
 //     R = C9 (15 p q s P^-5/2 - 3 P^-3/2), X = -3 C9 P^-5/2, t = X p q
 //   C9 with the scale and the alchemical factor (ReferenceInteraxThreeBodyIxn.cpp:116-120).
+// Relative RMS errors of the three-body force against FP64 (means of six): 24,000 atoms 3.00e-7, 96,000 atoms 3.01e-7,
+// 258 sites without a cutoff 2.62e-7.  With the sums of a lane in one row of up to 64, approximate quotients throughout and
+// the force on A summed in float they were 3.16e-7, 3.22e-7 and 3.76e-7, in the same time; an energy is summed in FP64,
+// one C's terms at a time.
 // What bounds it: FP32 issue, about 75 instructions a visit, and for a few thousand sites the latency of the staging
 // (list, position, parameters, three dependent loads).  The earlier form gave each lane a pair (B, C) of a flat
 // triangular index, stored both forces in shared memory and gathered them per neighbor, 425 issue slots per 32 pairs.
@@ -497,7 +502,7 @@ __device__ __forceinline__ void storeNeighbor(TripleStorage<DAMP, N>& S, const A
 template <bool DAMP, bool IMAGE, bool ALCH, int N>
 __device__ __forceinline__ void siteTriples(const TripleStorage<DAMP, N>& S, const AtmBuffers& A, const AtmConfig& C,
                                             const float4& pa, int cFirst, int cStep, int cEnd, int bBegin, int bEnd,
-                                            int lane, float (&fa)[3], float& energy,
+                                            int lane, long long& fa, double& energy,
                                             unsigned long long& visits) {
     unsigned seen = 0;
     const int s = lane & 3;
@@ -509,23 +514,27 @@ __device__ __forceinline__ void siteTriples(const TripleStorage<DAMP, N>& S, con
         const float4 xc = S.pos[have ? k : cFirst], pc = S.par[have ? k : cFirst];
         SiteDamping dc;
         if (DAMP) dc = S.damp[have ? k : cFirst];
-        const float invV = rcpApprox(xc.w);
-        float gx = 0.0f, gy = 0.0f, gz = 0.0f;
-        for (int b = have ? bBegin + s : bEnd; b < bEnd; b += 4) {
+        float invV = rcpApprox(xc.w);
+        invV = fmaf(invV, fmaf(-xc.w, invV, 1.0f), invV);
+        // along: the factor of xc, summed over B
+        float gx = 0.0f, gy = 0.0f, gz = 0.0f, along = 0.0f, eC = 0.0f;
+        auto visit = [&](int b) {
             const float4 xb = S.pos[b], pb = S.par[b];
-            if (__float_as_int(pb.w) == __float_as_int(pc.w)) continue;      // one molecule, B = C among them
+            if (__float_as_int(pb.w) == __float_as_int(pc.w)) return;      // one molecule, B = C among them
             float cx = xc.x - xb.x, cy = xc.y - xb.y, cz = xc.z - xb.z;
             if (IMAGE) minimumImageF(cx, cy, cz, C.boxf);
             const float w = fmaf(cx, cx, fmaf(cy, cy, cz * cz));
-            if (!(w < C.cutoff2)) continue;
+            if (!(w < C.cutoff2)) return;
             float c9 = (pb.y * pc.y) * kA * fmaf(pa.y, rcpApprox(pb.x + pc.x), 1.0f);
             if (pb.z != 0.0f || pc.z != 0.0f) c9 *= lambdaBC;
-            else if (ALCH && pa.w == 0.0f) continue;
-            if (c9 == 0.0f) continue;
+            else if (ALCH && pa.w == 0.0f) return;
+            if (c9 == 0.0f) return;
             const float p = fmaf(xb.x, xc.x, fmaf(xb.y, xc.y, xb.z * xc.z));
             const float q = fmaf(xb.x, cx, fmaf(xb.y, cy, xb.z * cz));
             const float r = fmaf(xc.x, cx, fmaf(xc.y, cy, xc.z * cz));
-            const float y = rsqrtApprox(xb.w * xc.w * w);
+            const float P = xb.w * xc.w * w;
+            float y = rsqrtApprox(P);
+            y = fmaf(fmaf(-P * y, y, 1.0f), 0.5f * y, y);      // its fifth power is taken
             const float invP = y * y;
             const float invP32 = invP * y;
             const float invP52 = invP32 * invP;
@@ -544,14 +553,32 @@ __device__ __forceinline__ void siteTriples(const TripleStorage<DAMP, N>& S, con
                 kb = fmaf(kb, damping, e * fbc * dc.dfr);
                 kc = fmaf(kc, damping, e * db.f * dc.f * dfr);
                 ka *= damping;
-                energy = fmaf(e, damping, energy);
+                eC = fmaf(e, damping, eC);
             }
-            else energy += e;
-            gx = fmaf(xc.x, kb, fmaf(cx, kc, fmaf(xb.x, ka, gx)));
-            gy = fmaf(xc.y, kb, fmaf(cy, kc, fmaf(xb.y, ka, gy)));
-            gz = fmaf(xc.z, kb, fmaf(cz, kc, fmaf(xb.z, ka, gz)));
+            else eC += e;
+            along += kb;
+            gx = fmaf(cx, kc, fmaf(xb.x, ka, gx));
+            gy = fmaf(cy, kc, fmaf(xb.y, ka, gy));
+            gz = fmaf(cz, kc, fmaf(xb.z, ka, gz));
             seen++;
-        }
+        };
+        const int first = have ? bBegin + s : bEnd;
+        if constexpr (N > kAtmFastStaged)
+            // a long list in runs of eight a lane, whose sums are added up
+            for (int b0 = first; b0 < bEnd; b0 += 32) {
+                const float sx = gx, sy = gy, sz = gz, sAlong = along;
+                gx = gy = gz = along = 0.0f;
+                for (int b = b0; b < min(b0 + 32, bEnd); b += 4) visit(b);
+                gx += sx;
+                gy += sy;
+                gz += sz;
+                along += sAlong;
+            }
+        else
+            for (int b = first; b < bEnd; b += 4) visit(b);
+        gx = fmaf(xc.x, along, gx);
+        gy = fmaf(xc.y, along, gy);
+        gz = fmaf(xc.z, along, gz);
         __syncwarp();
 #pragma unroll
         for (int o = 1; o < 4; o <<= 1) {
@@ -559,24 +586,19 @@ __device__ __forceinline__ void siteTriples(const TripleStorage<DAMP, N>& S, con
             gy += __shfl_xor_sync(0xffffffffu, gy, o);
             gz += __shfl_xor_sync(0xffffffffu, gz, o);
         }
-        fa[0] += gx;
-        fa[1] += gy;
-        fa[2] += gz;
+        energy += (double)eC;
         // lane s of the four adds component s
-        const float g = s == 0 ? gx : (s == 1 ? gy : gz);
-        if (have && s < 3 && g != 0.0f) atomicAddFixed(A.siteForce + s * C.numSites + S.site[k], -toFixed(g));
+        const long long g = have && s < 3 ? toFixed(s == 0 ? gx : (s == 1 ? gy : gz)) : 0;
+        fa += g;
+        if (g != 0) atomicAddFixed(A.siteForce + s * C.numSites + S.site[k], -g);
     }
     visits += seen;
 }
 
-// The force on A of a warp's share (the four lanes of a C hold the same sums).
-__device__ __forceinline__ void addSiteForce(const AtmBuffers& A, const AtmConfig& C, int a, int lane,
-                                             const float (&fa)[3]) {
-    float f[3] = {fa[0], fa[1], fa[2]};
-    for (int o = 4; o < 32; o <<= 1)
-        for (int d = 0; d < 3; d++) f[d] += __shfl_xor_sync(0xffffffffu, f[d], o);
-    const float g = lane == 0 ? f[0] : (lane == 1 ? f[1] : f[2]);
-    if (lane < 3 && g != 0.0f) atomicAddFixed(A.siteForce + lane * C.numSites + a, toFixed(g));
+// The force on A of a warp's share (lane s < 3 of every four holds component s).
+__device__ __forceinline__ void addSiteForce(const AtmBuffers& A, const AtmConfig& C, int a, int lane, long long fa) {
+    for (int o = 4; o < 32; o <<= 1) fa += __shfl_xor_sync(0xffffffffu, fa, o);
+    if (lane < 3 && fa != 0) atomicAddFixed(A.siteForce + lane * C.numSites + a, fa);
 }
 
 // Stage the neighbors of site a that are within the cutoff (in list order) with their displacements from a and their
@@ -658,11 +680,9 @@ __global__ void __launch_bounds__(32 * kAtmFastWarps, IX_TUNE_ATM_MIN_BLOCKS) kT
                                                storeNeighbor(S, A, C, pa, slot, b, x, y, z);
                                            });
         __syncwarp();
-        float fa[3] = {0.0f, 0.0f, 0.0f};
-        float eSite = 0.0f;
-        siteTriples<DAMP, IMAGE, ALCH>(S, A, C, pa, 0, 8, m, 0, m, lane, fa, eSite, visits);
+        long long fa = 0;
+        siteTriples<DAMP, IMAGE, ALCH>(S, A, C, pa, 0, 8, m, 0, m, lane, fa, eAcc, visits);
         addSiteForce(A, C, a, lane, fa);
-        eAcc += (double)eSite;
     }
     const double sum = 0.5 * warpSumD(eAcc);           // each triple was visited twice
     if (lane == 0) A.energyPartials[warp] = sum;
@@ -708,14 +728,12 @@ __global__ void __launch_bounds__(32 * kAtmWarps) kTriplesWide(AtmBuffers A, Atm
             return scan ? stageTripleNeighborsScan(A, C, a, lane, first, capacity, store)
                         : stageTripleNeighbors(A, C, a, n, lane, first, capacity, store);
         };
-        float fa[3] = {0.0f, 0.0f, 0.0f};
-        float energy = 0.0f;
+        long long fa = 0;
         __syncwarp();
         const int m = stage(0, 0, kAtmMaxStaged);
         __syncwarp();
         if (m <= kAtmMaxStaged) {
-            siteTriples<DAMP, IMAGE, ALCH>(S, A, C, pa, 8 * part, 8 * kAtmWideParts, m, 0, m, lane, fa, energy, visits);
-            eAcc += (double)energy;
+            siteTriples<DAMP, IMAGE, ALCH>(S, A, C, pa, 8 * part, 8 * kAtmWideParts, m, 0, m, lane, fa, eAcc, visits);
         }
         else {
             const int chunks = (m + kAtmChunk - 1) / kAtmChunk;
@@ -728,10 +746,8 @@ __global__ void __launch_bounds__(32 * kAtmWarps) kTriplesWide(AtmBuffers A, Atm
                     if (J != I) stage(J * kAtmChunk, kAtmChunk, kAtmChunk);
                     __syncwarp();
                     const int b0 = J == I ? 0 : kAtmChunk;
-                    energy = 0.0f;
                     siteTriples<DAMP, IMAGE, ALCH>(S, A, C, pa, 8 * part, 8 * kAtmWideParts, cI, b0, b0 + cJ, lane, fa,
-                                             energy, visits);
-                    eAcc += (double)energy;
+                                                   eAcc, visits);
                 }
             }
         }
