@@ -279,7 +279,8 @@ struct ix_ctx {
     double* dAtmPartials = nullptr;      // per-warp energies of the triple kernel
     int* dParticleSiteStart = nullptr;   // n + 1: the sites of each particle (CSR)
     int* dParticleSites = nullptr;
-    int atmFastBlocks = 0;               // grid of the fast triple kernel
+    int atmFastBlocks = 0;               // grid of the fast triple kernel beside the pair kernel
+    int atmFastBlocksAlone = 0;          // and where nothing as long runs beside it
     int atmGridBlocks = 0;               // grid of the wide triple kernel
     int* dFlagso = nullptr;
     float4 *dP0 = nullptr, *dP1 = nullptr, *dP2 = nullptr;
@@ -333,8 +334,8 @@ static void bumpVersion(ix_ctx* ctx) {
 }
 
 // Energy slots of the triple kernels: one per warp of the fast grid, then one per warp of the wide grid.
-static size_t atmPartialCount(const ix_ctx* ctx) {
-    return (size_t)ctx->atmFastBlocks * kAtmFastWarps + (size_t)ctx->atmGridBlocks * kAtmWarps;
+static size_t atmPartialCount(const ix_ctx* ctx, int fastBlocks) {
+    return (size_t)fastBlocks * kAtmFastWarps + (size_t)ctx->atmGridBlocks * kAtmWarps;
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -952,10 +953,13 @@ static void updateGeometry(ix_ctx* ctx) {
 // three-body setup
 // ---------------------------------------------------------------------------------------------------------------------
 
-// Resident blocks per SM of the fast triple kernel.  It runs beside the pair list and the pair kernel, whose persistent
+// Resident blocks per SM of the fast triple kernel beside the pair kernel.  It runs beside the pair list and the pair kernel, whose persistent
 // grid fills what is left of each SM, so it gets its share of the two kernels' work, at least two blocks.  With as many
 // blocks as fit, the two ran one after the other: 103 + 19 us in an MD step of the 24,000-atom box, together 112 us now;
-// 371 + 159 us and 520 us for 96,000 atoms (0.8 nm; two to four blocks measure the same there).
+// 371 + 159 us and 520 us for 96,000 atoms (0.8 nm; two to four blocks measure the same there).  An evaluation without pair
+// terms, a serialized one and the alchemical triples of the windows have the SMs for themselves and take a warp per site:
+// the three-body term alone 55 us for 66 with the blocks meant for company (24,000 atoms) and 195 for 366 (96,000); 16
+// windows of 96,000 atoms 713 for 751.
 static int tripleBlocksPerSM(const ix_ctx* ctx) {
     const int most = IX_TUNE_ATM_MIN_BLOCKS;
     if (!ctx->pairShared) return most;
@@ -1037,11 +1041,12 @@ static int allocateAtm(ix_ctx* ctx) {
     IX_TRY(deviceAlloc(ctx, "nbr", (size_t)ns * A.cap, &A.nbr));
     A.flag = ctx->dFlags + 4;
     A.numParticles = ctx->n;
-    // fast kernel: at most one warp per site; wide kernel (long lists): one wave of blocks over every (site, part) unit
-    ctx->atmFastBlocks = std::max(1, std::min((ns + kAtmFastWarps - 1) / kAtmFastWarps, tripleBlocksPerSM(ctx) * ctx->numSMs));
+    // fast kernel: one warp per site, fewer beside the pair kernel; wide kernel (long lists): one wave of blocks over every (site, part) unit
+    ctx->atmFastBlocksAlone = std::max(1, (ns + kAtmFastWarps - 1) / kAtmFastWarps);
+    ctx->atmFastBlocks = std::min(ctx->atmFastBlocksAlone, tripleBlocksPerSM(ctx) * ctx->numSMs);
     ctx->atmGridBlocks = std::max(1, (int)std::min<long long>(((long long)ns * kAtmWideParts + kAtmWarps - 1) / kAtmWarps,
                                                               (long long)ctx->numSMs * 4));
-    IX_TRY(deviceAlloc(ctx, "atmPartials", atmPartialCount(ctx), &ctx->dAtmPartials));
+    IX_TRY(deviceAlloc(ctx, "atmPartials", atmPartialCount(ctx, ctx->atmFastBlocksAlone), &ctx->dAtmPartials));
     A.energyPartials = ctx->dAtmPartials;
     A.tripleVisits = ctx->dCounts + 1;
     ctx->atmAllocated = true;
@@ -1354,8 +1359,9 @@ static void recordTiming(ix_ctx* ctx, int i, cudaStream_t s) {
     else cudaEventRecord(ctx->ev[i], s);
 }
 
-// The configuration of the three-body kernels at the context's parameters, and the cell grid of the site-list search.
-static AtmConfig atmConfig(ix_ctx* ctx) {
+// The configuration of the three-body kernels at the context's parameters, for a fast triple kernel of fastBlocks, and the
+// cell grid of the site-list search.
+static AtmConfig atmConfig(ix_ctx* ctx, int fastBlocks) {
     AtmBuffers& A = ctx->A;
     AtmConfig C{};
     C.numSites = (int)ctx->siteParams.size() / 3;
@@ -1374,7 +1380,7 @@ static AtmConfig atmConfig(ix_ctx* ctx) {
     C.imageBC = tripleNeedsImages(C, ctx->atmCutoff);
     // the wide kernel's energy slots start at zero (it runs only while some list is long)
     C.zeroSlots = ctx->atmGridBlocks * kAtmWarps;
-    C.zeroOffset = ctx->atmFastBlocks * kAtmFastWarps;
+    C.zeroOffset = fastBlocks * kAtmFastWarps;
     // the cell grid of the list search in a rectangular periodic box with at least three cells per edge
     A.cells.nc[0] = A.cells.nc[1] = A.cells.nc[2] = 0;
     if (C.periodic && !C.box.triclinic && A.cells.cellStart) {
@@ -1439,6 +1445,7 @@ static int launchEvaluation(ix_ctx* ctx, unsigned terms, double* outForces, doub
     IX_TRY(stageUploads(ctx, terms));
     // the three-body chain runs on a second stream, concurrently with the pair list and pair kernel
     const bool fork = doPair && doAtm && !ctx->serialize;
+    const int tripleBlocks = fork ? ctx->atmFastBlocks : ctx->atmFastBlocksAlone;
     cudaStream_t sa = fork ? ctx->stream2 : st;
     if (fork) {
         IX_CUDA(ctx, cudaEventRecord(ctx->evFork, st));
@@ -1446,7 +1453,7 @@ static int launchEvaluation(ix_ctx* ctx, unsigned terms, double* outForces, doub
     }
     if (doAtm) {
         AtmBuffers& A = ctx->A;
-        const AtmConfig C = atmConfig(ctx);
+        const AtmConfig C = atmConfig(ctx, tripleBlocks);
         const int tpb = 256;
         const int gS = (C.numSites + 63) / 64;   // 64-thread blocks, so that a few thousand sites reach every SM
         kSiteCentroids<<<gS, 64, 0, sa>>>(A, C, ctx->dPos);
@@ -1462,8 +1469,7 @@ static int launchEvaluation(ix_ctx* ctx, unsigned terms, double* outForces, doub
         recordTiming(ctx, 2, sa);
         // the sites whose lists are too long for the fast kernel go to the wide one, which returns at once when there
         // are none and goes first
-        launchTriples<false>(A, C, ctx->atmFastBlocks, ctx->atmGridBlocks, A.flag + 2, sa, fork ? ctx->evFork : nullptr,
-                             early);
+        launchTriples<false>(A, C, tripleBlocks, ctx->atmGridBlocks, A.flag + 2, sa, fork ? ctx->evFork : nullptr, early);
         ctx->launches += A.cells.nc[0] ? 5 : 4;
         recordTiming(ctx, 3, sa);
         ctx->evAtm = ctx->profiling;
@@ -1561,7 +1567,7 @@ static int launchEvaluation(ix_ctx* ctx, unsigned terms, double* outForces, doub
     }
     F.blocks = (n + kFinishThreads - 1) / kFinishThreads;
     EnergyReduction R{doPair ? ctx->dPairPartials : nullptr, ctx->L.numTiles, ctx->L.tileCap,
-                      doAtm ? ctx->dAtmPartials : nullptr, (int)atmPartialCount(ctx), lrcEnergy, outEnergy,
+                      doAtm ? ctx->dAtmPartials : nullptr, (int)atmPartialCount(ctx, tripleBlocks), lrcEnergy, outEnergy,
                       ctx->dEnergyBlocks, ctx->dReduceTicket, ctx->dCounts, doPair ? ctx->L.taskCounter : nullptr,
                       doPair ? ctx->L.flag : nullptr, doAtm ? ctx->A.flag : nullptr};
     launchNext(early, st, kFinish, F.blocks + kReduceBlocks, kFinishThreads, 0, F, R);
@@ -2709,8 +2715,9 @@ static int windowSlope(ix_ctx* ctx, bool atm, bool pairs, double* dSlope, double
     F.particleSites = ctx->dParticleSites;
     F.outForces = dSlope;
     F.blocks = (ctx->n + kFinishThreads - 1) / kFinishThreads;
-    EnergyReduction R{nullptr, nullptr, 0, atm ? ctx->dAtmPartials : nullptr, (int)atmPartialCount(ctx), 0.0, dEnergy,
-                      ctx->dEnergyBlocks, ctx->dReduceTicket, atm ? ctx->dCounts : nullptr, nullptr, nullptr, nullptr};
+    EnergyReduction R{nullptr, nullptr, 0, atm ? ctx->dAtmPartials : nullptr,
+                      (int)atmPartialCount(ctx, ctx->atmFastBlocksAlone), 0.0, dEnergy, ctx->dEnergyBlocks,
+                      ctx->dReduceTicket, atm ? ctx->dCounts : nullptr, nullptr, nullptr, nullptr};
     kFinish<<<F.blocks + kReduceBlocks, kFinishThreads, 0, ctx->stream>>>(F, R);
     ctx->launches += 1;
     IX_CUDA(ctx, cudaGetLastError());
@@ -2756,8 +2763,8 @@ static int windowBuffers(ix_ctx* ctx, int num_windows, int passes, bool softcore
 // exactly one, the triple kernel keeps the triples with an alchemical site.  The long-range correction's alchemical part
 // joins each window's energy. Before, the linear case was two whole
 // evaluations and the other a launch and a finish per window, between evaluations of the pairs at 0 and of the triples
-// at 0 and 1: 16 windows of a 96,000-atom box 1197 us and 748 now, 12 soft-core windows of 12,297 atoms 704 and 211.
-// What is left is the evaluation at 0 (590 and 116 us) and, behind it, the alchemical triples (66 and 28 us, most of it
+// at 0 and 1: 16 windows of a 96,000-atom box 1197 us and 713 now, 12 soft-core windows of 12,297 atoms 704 and 211.
+// What is left is the evaluation at 0 (590 and 116 us) and, behind it, the alchemical triples (32 and 30 us, most of it
 // reading the lists that hold no alchemical site) or the alchemical pairs (19 and 43 us).
 // fits: false when the buffers did not fit (nothing was done).  redo: as for windowsPass.
 static int alchemicalWindows(ix_ctx* ctx, const std::string& name, unsigned dependent, bool softcore, int num_windows,
@@ -2802,9 +2809,9 @@ static int alchemicalWindows(ix_ctx* ctx, const std::string& name, unsigned depe
             IX_CUDA(ctx, cudaEventRecord(ctx->evFork, st));
             IX_CUDA(ctx, cudaStreamWaitEvent(sa, ctx->evFork, 0));
         }
-        const AtmConfig C = atmConfig(ctx);
+        const AtmConfig C = atmConfig(ctx, ctx->atmFastBlocksAlone);
         kSiteCentroids<<<(C.numSites + 63) / 64, 64, 0, sa>>>(ctx->A, C, ctx->dPos);   // clears the site forces
-        launchTriples<true>(ctx->A, C, ctx->atmFastBlocks, ctx->atmGridBlocks, ctx->A.flag + 2, sa);
+        launchTriples<true>(ctx->A, C, ctx->atmFastBlocksAlone, ctx->atmGridBlocks, ctx->A.flag + 2, sa);
         ctx->launches += 3;
         if (fork) IX_CUDA(ctx, cudaEventRecord(ctx->evJoin, sa));
     }
