@@ -383,7 +383,9 @@ int buildBatchPairs(ix_batch* b, const std::vector<int>& blockStart, int nb) {
     IX_TRY(batchUpload(b, "tileJ", tileJ, &L.tileJ));
     IX_TRY(batchUpload(b, "tileIBlock", tileI, &L.tileIBlock));
     IX_TRY(batchUpload(b, "tileMask", masks, &L.tileMask));
-    if (b->numTiles > 0) IX_TRY(batchUpload(b, "tileOrder", tileOrder, &L.tileOrder));
+    if (b->numTiles > 0) IX_TRY(batchUpload(b, "tileOrder", tileOrder, &L.bucketTiles));
+    IX_TRY(batchUpload(b, "bucketEnd", std::vector<int>(32, b->numTiles), &L.bucketEnd));
+    IX_TRY(batchUpload(b, "bucketOffset", std::vector<unsigned>(32, 0u), &L.bucketOffset));
     IX_TRY(batchUpload(b, "numTiles", std::vector<int>{b->numTiles}, &L.numTiles));
     IX_TRY(batchUpload(b, "taskCounter", std::vector<int>{0}, &L.taskCounter));
     IX_TRY(batchUpload(b, "tileStart", tileStart, &b->tileStart));

@@ -873,6 +873,8 @@ static int allocatePair(ix_ctx* ctx, long long tileCap) {
     IX_TRY(deviceAlloc(ctx, "tileJ", 32 * (size_t)L.tileCap, &L.tileJ));
     IX_TRY(deviceAlloc(ctx, "tileIBlock", L.tileCap, &L.tileIBlock));
     IX_TRY(deviceAlloc(ctx, "bucketTiles", (size_t)kTileBuckets * L.tileCap, &L.bucketTiles));
+    IX_TRY(deviceAlloc(ctx, "bucketEnd", 32, &L.bucketEnd));
+    IX_TRY(deviceAlloc(ctx, "bucketOffset", 32, &L.bucketOffset));
     IX_TRY(deviceAlloc(ctx, "bucketCount", kTileBuckets, &L.bucketCount));
     IX_TRY(deviceAlloc(ctx, "tileMask", 64 * (size_t)L.tileCap, &L.tileMask));
     IX_TRY(deviceAlloc(ctx, "numTiles", 1, &L.numTiles));

@@ -75,9 +75,10 @@ struct ListBuffers {
     int* blockTiles;            // nb + 1: exclusive scan of the tile counts, then the total
     int* tileJ;                 // tileCap x 32
     int* tileIBlock;            // tileCap
-    int* bucketCount;           // kTileBuckets: tiles by their number of candidate pairs (null: tileOrder)
-    int* bucketTiles;           // kTileBuckets x tileCap: the tiles of each bucket
-    int* tileOrder;             // numTiles: the tiles by decreasing candidate count (a batch's static list)
+    int* bucketCount;           // kTileBuckets: tiles by their number of candidate pairs, while the masks are made
+    int* bucketTiles;           // kTileBuckets x tileCap: the tiles of each bucket (a batch: all in one, in order)
+    int* bucketEnd;             // 32: the end of each bucket, the fullest tiles' first, in the pair kernel's sequence of tasks
+    unsigned* bucketOffset;     // 32: where a bucket's tasks find their tiles: bucketTiles[bucketOffset + task]
     unsigned* tileMask;         // tileCap x 64: row masks (per i lane, bit = j slot), then column masks (per j lane)
     int* numTiles;              // tiles to evaluate (0 after an overflow)
     int* taskCounter;           // next tile of the pair kernel's dynamic schedule (zeroed before each launch)
@@ -91,11 +92,16 @@ struct ListBuffers {
 
 __device__ __forceinline__ bool rebuildRequested(const ListBuffers& L) { return *(volatile int*)L.flag != 0; }
 
-// The pair kernel takes the tiles by decreasing number of candidate pairs, in steps of 64, so that the last tiles its
-// warps take are short.  The mask kernel appends each tile to its bucket; the order within a bucket follows the
-// atomics and varies from build to build, which changes no result: forces are summed in fixed point and energies go to
-// each tile's own slot.
+// The pair kernel takes the tiles by decreasing number of candidate pairs, so that the last tiles its warps take are
+// short: 32 pairs to a bucket up to 320, where the tiles of a liquid lie (64 to a bucket cost 0.9 us of 105 for 24,000
+// atoms), then 64 and 128.  The mask kernel appends each tile to its bucket and its last block sums the counts up; the
+// order within a bucket follows the atomics and varies from build to build, which changes no result: forces are summed in
+// fixed point and energies go to each tile's own slot.
 constexpr int kTileBuckets = 16;
+__device__ __forceinline__ int tileBucket(unsigned pairs) {
+    if (pairs < 320) return (int)(pairs >> 5);
+    return pairs < 512 ? 5 + (int)(pairs >> 6) : min(9 + (int)(pairs >> 7), kTileBuckets - 1);
+}
 
 // Current positions in the build frame, and whether any particle moved more than half the skin since the last build,
 // which sets the rebuild flag (then, and where it is set already, the build writes the positions itself).  Padding
@@ -621,7 +627,8 @@ __device__ __forceinline__ unsigned transposeBits(unsigned x, int lane) {
 // depend on the distance are masks formed once per tile; where the i-block allows it (rectangular box, block small
 // against the box), j is placed at its image nearest the block's center once, as in the pair kernel, instead of a
 // minimum image per pair.  Exclusions are looked up only for the pairs whose i lies in j's exclusion range.  Row
-// masks: lane = i slot, bit k = the tile's j lane k; column masks: the transpose.
+// masks: lane = i slot, bit k = the tile's j lane k; column masks: the transpose.  The last block lays out the pair
+// kernel's sequence of tasks.
 __global__ void __launch_bounds__(kListThreads) kTileMasks(ListBuffers L, ListGeometry G) {
     dependentStart(false);
     if (!rebuildRequested(L)) return;
@@ -705,10 +712,21 @@ __global__ void __launch_bounds__(kListThreads) kTileMasks(ListBuffers L, ListGe
         L.tileMask[64LL * t + 32 + lane] = column;
         const unsigned pairs = __reduce_add_sync(0xffffffffu, (unsigned)__popc(column));
         if (lane == 0) {
-            const int b = min((int)(pairs >> 6), kTileBuckets - 1);
+            const int b = tileBucket(pairs);
             L.bucketTiles[(size_t)b * L.tileCap + atomicAdd(L.bucketCount + b, 1)] = t;
         }
     }
+    if (!lastBlock(L.ticket) || warp != 0) return;
+    const int b = kTileBuckets - 1 - lane;
+    const int count = b >= 0 ? __ldcg(L.bucketCount + b) : 0;
+    int end = count;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, end, o);
+        if (lane >= o) end += v;
+    }
+    L.bucketEnd[lane] = end;
+    if (b >= 0) L.bucketOffset[lane] = (unsigned)b * (unsigned)L.tileCap - (unsigned)(end - count);
 }
 
 }  // namespace ix
