@@ -237,6 +237,10 @@ int ix_get_launch_count(ix_ctx* ctx, long long* launches);
  * are identical.  No counterpart in the reference (OpenMM launches kernels one by one). */
 int ix_set_graphs(ix_ctx* ctx, int enable);
 
+/* How many graphs the context has captured, and how often it has replayed a graph of several MD steps (a measurement
+ * aid; no counterpart in the reference).  Either pointer may be NULL. */
+int ix_get_graph_counts(ix_ctx* ctx, long long* captures, long long* several_step_replays);
+
 /* An evaluation's flags, energies and counts come back through a page-locked slot of the context (default), or, where
  * the host has no page-locked memory left, through ordinary memory.  enable = 0 takes the second way; the results are
  * identical.  A test aid with no counterpart in the reference. */

@@ -323,8 +323,10 @@ struct ix_ctx {
     bool useGraphs = true;
     unsigned long long version = 1;
     LaunchGraph graphCompute, graphDevice, graphMd, graphMdSeveral, graphPosq;
-    unsigned long long mdGraphVersion = 0;   // version of the captures that mdGraphRun steps have replayed
+    unsigned long long mdGraphVersion = 0;   // version and key of the captures that mdGraphRun steps have replayed
+    GraphKey mdGraphKey;
     int mdGraphRun = 0;
+    long long graphCaptures = 0, mdSeveralReplays = 0;   // ix_get_graph_counts
     std::vector<LaunchGraph> graphWindows;  // evaluations at window values of one parameter, one graph per value
     size_t windowNext = 0;                  // slot replaced next when graphWindows is full
 };
@@ -1679,6 +1681,7 @@ static int launchGraph(ix_ctx* ctx, LaunchGraph& g, const GraphKey& key, F&& enq
             }
         }
         cudaGraphDestroy(graph);
+        ctx->graphCaptures++;
         g.launches = ctx->launches - before;
         ctx->launches = before;
         g.key = key;
@@ -2557,13 +2560,19 @@ static int enqueueSteps(ix_ctx* ctx, int num_steps, double dt) {
         for (int k = 0; k < kMdGraphSteps; k++) IX_TRY(step());
         return IX_OK;
     };
-    if (ctx->mdGraphVersion != ctx->version) {
+    // a run goes on while what its graphs were captured for stays: a program that takes turns with two step sizes would
+    // capture eight steps in each turn
+    if (ctx->mdGraphVersion != ctx->version || !(ctx->mdGraphKey == key)) {
         ctx->mdGraphVersion = ctx->version;
+        ctx->mdGraphKey = key;
         ctx->mdGraphRun = 0;
     }
     for (int s = 0; s < num_steps;) {
         const bool long_run = ctx->mdGraphRun >= kMdGraphRun && num_steps - s >= kMdGraphSteps;
-        if (long_run) IX_TRY(launchGraph(ctx, ctx->graphMdSeveral, key, several));
+        if (long_run) {
+            IX_TRY(launchGraph(ctx, ctx->graphMdSeveral, key, several));
+            ctx->mdSeveralReplays += ctx->useGraphs;
+        }
         else IX_TRY(launchGraph(ctx, ctx->graphMd, key, step));
         s += long_run ? kMdGraphSteps : 1;
         if (!long_run) ctx->mdGraphRun = std::min(ctx->mdGraphRun + 1, kMdGraphRun);
@@ -3063,6 +3072,13 @@ int ix_compute_windows(ix_ctx* ctx, const char* parameter, int num_windows, cons
 int ix_get_launch_count(ix_ctx* ctx, long long* launches) {
     if (!ctx || !launches) return IX_ERR_INVALID;
     *launches = ctx->launches;
+    return IX_OK;
+}
+
+int ix_get_graph_counts(ix_ctx* ctx, long long* captures, long long* several_step_replays) {
+    if (!ctx) return IX_ERR_INVALID;
+    if (captures) *captures = ctx->graphCaptures;
+    if (several_step_replays) *several_step_replays = ctx->mdSeveralReplays;
     return IX_OK;
 }
 

@@ -83,6 +83,7 @@ def lib():
             "ix_get_kernel_times": (ctypes.c_int, [P, P, P]),
             "ix_get_launch_count": (ctypes.c_int, [P, P]),
             "ix_set_graphs": (ctypes.c_int, [P, ctypes.c_int]),
+            "ix_get_graph_counts": (ctypes.c_int, [P, P, P]),
             "ix_set_pinned_status": (ctypes.c_int, [P, ctypes.c_int]),
             "ix_compute_windows": (ctypes.c_int, [P, ctypes.c_char_p, ctypes.c_int, P, P, P]),
             "ix_compute_windows_device": (ctypes.c_int, [P, ctypes.c_char_p, ctypes.c_int, P, P, P]),
