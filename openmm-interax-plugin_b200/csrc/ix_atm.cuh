@@ -654,6 +654,10 @@ __device__ __forceinline__ int stageTripleNeighborsScan(const AtmBuffers& A, con
     return m;
 }
 
+static_assert(kAtmFastWarps * sizeof(TripleStorage<true, kAtmFastStaged>) < 48 * 1024, "static shared memory of a block");
+static_assert((kAtmFastWarps * sizeof(TripleStorage<true, kAtmFastStaged>) + 1024) * IX_TUNE_ATM_MIN_BLOCKS <= 228 * 1024,
+              "shared memory of the blocks an SM is asked to hold");
+
 template <bool DAMP, bool IMAGE, bool ALCH>
 __global__ void __launch_bounds__(32 * kAtmFastWarps, IX_TUNE_ATM_MIN_BLOCKS) kTriplesFast(AtmBuffers A, AtmConfig C) {
     dependentStart(false);
@@ -693,6 +697,8 @@ __global__ void __launch_bounds__(32 * kAtmFastWarps, IX_TUNE_ATM_MIN_BLOCKS) kT
 constexpr int kAtmWarps = 4;
 constexpr int kAtmMaxStaged = 256;
 constexpr int kAtmChunk = kAtmMaxStaged / 2;
+static_assert(kAtmWarps * sizeof(TripleStorage<true, kAtmMaxStaged>) <= 48 * 1024,
+              "dynamic shared memory of a block without asking for more than the default");
 // Each long-list site is taken by this many warps, each evaluating every kAtmWideParts-th group of 8 of its neighbors:
 // a site near the start of a large cluster has tens of thousands of (B, C) pairs, which one warp would take alone.
 constexpr int kAtmWideParts = 8;

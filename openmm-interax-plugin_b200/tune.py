@@ -38,6 +38,7 @@ PKG = Path(__file__).resolve().parent
 sys.path.insert(0, str(PKG))
 import build_lib  # noqa: E402
 
+# (IX_TUNE_ATM_ROUND and IX_TUNE_ATM_ACCUM are named by recorded files and read by no kernel)
 DEFAULTS = {"IX_TUNE_PAIR_WARPS": 4, "IX_TUNE_PAIR_ROUND": 128, "IX_TUNE_PAIR_MIN_BLOCKS": 8,
             "IX_TUNE_PAIR_COLUMN_LISTS": 0, "IX_TUNE_PAIR_COLUMN_TRANSPOSE": 0, "IX_TUNE_PAIR_ILP": 0,
             "IX_TUNE_PAIR_SHARED_TABLE_BYTES": 0,
