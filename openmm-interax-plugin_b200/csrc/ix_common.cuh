@@ -159,9 +159,10 @@ struct NvtxRange {
 // first statement, until that one has finished and its writes are visible.  With `trigger` the kernel lets its own
 // successor be set up as soon as all of its blocks have started (else when they have ended).
 // Measured without and with it: 100 steps of 648 atoms 3890 and 3660 us, of 24,000 atoms 16930 and 16730; an evaluation
-// of 648 atoms 66.5 and 64.9 us.  Eight evaluations of 96,000 atoms, whose triple kernel is as long as its pair kernel, took
-// 4617 us without and 4635 with it (the two kernels' blocks are placed in another order): more than kEarlyLaunchBlocks
-// blocks of 32 particles are launched the ordinary way.
+// of 648 atoms 66.5 and 64.9 us.  In large systems the pair and triple kernels' blocks are then placed in another order and
+// the two overlap less; evaluations back to back, without and with it: 24,000 atoms 153.5 and 153.8 us, 33,000 190.5 and
+// 190.2, 48,000 255.6 and 253.9, 63,000 390 and 412, 96,000 551 and 574: more than kEarlyLaunchBlocks blocks of 32
+// particles are launched the ordinary way.
 __device__ __forceinline__ void dependentStart(bool trigger) {
     cudaGridDependencySynchronize();
     if (trigger) cudaTriggerProgrammaticLaunchCompletion();
@@ -188,8 +189,8 @@ static cudaError_t launchNext(bool early, cudaStream_t st, void (*kernel)(Params
 constexpr int kEarlyLaunchBlocks = 1024;
 
 // Systems of at most this many blocks of 32 particles, and of this many sites, trigger: their successors' waiting blocks
-// keep nothing else from the SMs (with it everywhere the dynamics of 24,000 atoms gained nothing: 16950 us), and 648
-// atoms take 3700 us for 3850 without.
+// keep nothing else from the SMs (with it everywhere the dynamics of 24,000 atoms gained nothing: 16950 us; evaluations of
+// 6,300 atoms 92.6 us for 90.8, of 9,000 93.3 for 91.6), and 648 atoms take 3700 us for 3850 without.
 constexpr int kEarlyBlocks = 192, kEarlySites = 2048;
 
 }  // namespace ix
