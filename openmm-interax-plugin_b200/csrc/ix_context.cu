@@ -760,6 +760,12 @@ static int uploadPairParams(ix_ctx* ctx) {
     return IX_OK;
 }
 
+// Systems of at most this many blocks of 32 particles take a thread block per tile (kPairTilesSmall).  Evaluations of the
+// pair terms back to back, a warp per tile and a block per tile: 24 atoms 37.1 and 36.6 us, 648 atoms 53.6 and 37.0,
+// 1,500 atoms 61.5 and 40.9, 3,000 atoms 74.1 and 56.3, 4,500 atoms 79.9 and 63.6, 7,800 atoms 87.4 and 86.1, 24,000
+// atoms 137 and 186.
+constexpr int kSmallBlocks = 192;
+
 // Particles per nm3 of the system, by its box or as a liquid.
 static double particleDensity(const ix_ctx* ctx) {
     const double volume = ctx->method == IX_CUTOFF_PERIODIC ? ctx->box[0] * ctx->box[4] * ctx->box[8]
@@ -874,10 +880,13 @@ static int allocatePair(ix_ctx* ctx, long long tileCap) {
     L.tileCap = (int)tileCap;
     IX_TRY(deviceAlloc(ctx, "tileJ", 32 * (size_t)L.tileCap, &L.tileJ));
     IX_TRY(deviceAlloc(ctx, "tileIBlock", L.tileCap, &L.tileIBlock));
-    IX_TRY(deviceAlloc(ctx, "bucketTiles", (size_t)kTileBuckets * L.tileCap, &L.bucketTiles));
-    IX_TRY(deviceAlloc(ctx, "bucketEnd", 32, &L.bucketEnd));
-    IX_TRY(deviceAlloc(ctx, "bucketOffset", 32, &L.bucketOffset));
     IX_TRY(deviceAlloc(ctx, "bucketCount", kTileBuckets, &L.bucketCount));
+    L.bucketEnd = nullptr;
+    if (nb > kSmallBlocks) {
+        IX_TRY(deviceAlloc(ctx, "bucketTiles", (size_t)kTileBuckets * L.tileCap, &L.bucketTiles));
+        IX_TRY(deviceAlloc(ctx, "bucketEnd", 32, &L.bucketEnd));
+        IX_TRY(deviceAlloc(ctx, "bucketOffset", 32, &L.bucketOffset));
+    }
     IX_TRY(deviceAlloc(ctx, "tileMask", 64 * (size_t)L.tileCap, &L.tileMask));
     IX_TRY(deviceAlloc(ctx, "numTiles", 1, &L.numTiles));
     IX_TRY(deviceAlloc(ctx, "taskCounter", 1, &L.taskCounter));
@@ -1400,12 +1409,6 @@ static AtmConfig atmConfig(ix_ctx* ctx, int fastBlocks) {
     }
     return C;
 }
-
-// Systems of at most this many blocks of 32 particles take a thread block per tile (kPairTilesSmall).  Evaluations of the
-// pair terms back to back, a warp per tile and a block per tile: 24 atoms 37.1 and 36.6 us, 648 atoms 53.6 and 37.0,
-// 1,500 atoms 61.5 and 40.9, 3,000 atoms 74.1 and 56.3, 4,500 atoms 79.9 and 63.6, 7,800 atoms 87.4 and 86.1, 24,000
-// atoms 137 and 186.
-constexpr int kSmallBlocks = 192;
 
 // The pair kernel's instance for the configuration: lean (no soft core, switching function or order-2 overlap), from
 // the class-pair table, uniform (no gates or scales), and the form for small systems.

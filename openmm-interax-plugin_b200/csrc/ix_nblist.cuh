@@ -78,6 +78,7 @@ struct ListBuffers {
     int* bucketCount;           // kTileBuckets: tiles by their number of candidate pairs, while the masks are made
     int* bucketTiles;           // kTileBuckets x tileCap: the tiles of each bucket (a batch: all in one, in order)
     int* bucketEnd;             // 32: the end of each bucket, the fullest tiles' first, in the pair kernel's sequence of tasks
+                                // (null: no buckets; a small system's kernel takes the tiles as they are)
     unsigned* bucketOffset;     // 32: where a bucket's tasks find their tiles: bucketTiles[bucketOffset + task]
     unsigned* tileMask;         // tileCap x 64: row masks (per i lane, bit = j slot), then column masks (per j lane)
     int* numTiles;              // tiles to evaluate (0 after an overflow)
@@ -711,12 +712,12 @@ __global__ void __launch_bounds__(kListThreads) kTileMasks(ListBuffers L, ListGe
         L.tileMask[64LL * t + lane] = row;
         L.tileMask[64LL * t + 32 + lane] = column;
         const unsigned pairs = __reduce_add_sync(0xffffffffu, (unsigned)__popc(column));
-        if (lane == 0) {
+        if (lane == 0 && L.bucketEnd) {
             const int b = tileBucket(pairs);
             L.bucketTiles[(size_t)b * L.tileCap + atomicAdd(L.bucketCount + b, 1)] = t;
         }
     }
-    if (!lastBlock(L.ticket) || warp != 0) return;
+    if (!L.bucketEnd || !lastBlock(L.ticket) || warp != 0) return;
     const int b = kTileBuckets - 1 - lane;
     const int count = b >= 0 ? __ldcg(L.bucketCount + b) : 0;
     int end = count;
