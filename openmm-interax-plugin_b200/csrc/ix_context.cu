@@ -1469,8 +1469,10 @@ static int launchEvaluation(ix_ctx* ctx, unsigned terms, double* outForces, doub
         if (A.cells.nc[0]) {
             const int sharedSites = C.numSites <= kSiteSortSharedMax;
             launchNext(early, sa, kSiteCellSort, 1, 1024, sharedSites ? C.numSites * sizeof(int) : 0, A, C, sharedSites);
-            launchNext(early, sa, kSiteNeighborsCells, std::min((C.numSites * 32 + tpb - 1) / tpb, ctx->numSMs * 2), tpb, 0,
-                       A, C);
+            // two blocks per SM beside the pair list, whose build takes longer anyway; alone, as many as the sites fill (eight):
+            // with two the three-body term of 24,000 atoms took 129 us with a rebuild for 100, of 96,000 643 for 425
+            launchNext(early, sa, kSiteNeighborsCells,
+                       std::min((C.numSites * 32 + tpb - 1) / tpb, ctx->numSMs * (fork ? 2 : 8)), tpb, 0, A, C);
         }
         else launchNext(early, sa, kSiteNeighbors, (C.numSites * 32 + tpb - 1) / tpb, tpb, 0, A, C);
         recordTiming(ctx, 2, sa);

@@ -1,6 +1,7 @@
 """The three-body term evaluated alone (a force group of its own, as in a multiple-time-step engine) by a context that
 has pair forces too: the same sums and the same time as by a context without them.  The triple kernel takes fewer thread
-blocks beside the pair kernel; with those the term alone took 1.2 times as long for 24,000 atoms, 1.9 times for 96,000.
+blocks beside the pair kernel, and the list search beside the pair list; with those the term alone took 1.2 times as long
+for 24,000 atoms and 1.9 times for 96,000, and a rebuild of its lists twice as long.
 """
 import ctypes
 
@@ -14,8 +15,8 @@ from interaxplugin import workloads as W
 pytestmark = pytest.mark.gpu
 
 
-def _contexts(waters):
-    system, pos, _ = W.water_box(waters, W.box_length_for(waters), 1.0, seed=2, three_body_cutoff=0.8)
+def _contexts(waters, cutoff):
+    system, pos, _ = W.water_box(waters, W.box_length_for(waters), 1.0, seed=2, three_body_cutoff=cutoff)
     alone = System()
     alone.setDefaultPeriodicBoxVectors(*system.getDefaultPeriodicBoxVectors())
     for i in range(system.getNumParticles()):
@@ -27,16 +28,17 @@ def _contexts(waters):
     return contexts, 1 << system.getForce(3).getForceGroup(), np.asarray(pos)
 
 
-def _time(ctx, group, pos):
+def _time(ctx, group, pos, shifts=(0.0,)):
     stream = torch.cuda.ExternalStream(ctx._lib.ix_get_stream(ctx._ctx))
-    x = torch.as_tensor(pos, device="cuda")
+    frames = [torch.as_tensor(pos + shift, device="cuda") for shift in shifts]
     out = torch.zeros(len(pos), 3, dtype=torch.float64, device="cuda")
     torch.cuda.synchronize()
     best = np.inf
     for _ in range(6):
         start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         start.record(stream)
-        for _ in range(20):
+        for k in range(20):
+            x = frames[k % len(frames)]
             ctx._check(ctx._lib.ix_compute_device_f64(ctx._ctx, group, ctypes.c_void_p(x.data_ptr()), None,
                                                       ctypes.c_void_p(out.data_ptr()), None))
         end.record(stream)
@@ -46,7 +48,7 @@ def _time(ctx, group, pos):
 
 
 def test_the_term_alone():
-    (both, alone), group, pos = _contexts(16000)
+    (both, alone), group, pos = _contexts(16000, 0.8)
     states = [both.getState(groups=group), alone.getState()]
     assert np.array_equal(states[0].getForces(), states[1].getForces())
     assert np.allclose(states[0].getTermEnergies(), states[1].getTermEnergies(), rtol=1e-12, atol=0)
@@ -54,3 +56,12 @@ def test_the_term_alone():
     assert np.isclose(both.getState().getTermEnergies()[3], states[1].getTermEnergies()[3], rtol=1e-12, atol=0)
     t_both, t_alone = _time(both, group, pos), _time(alone, group, pos)
     assert t_both <= 1.15 * t_alone, (t_both, t_alone)
+
+
+def test_a_rebuild_of_the_lists():
+    # every evaluation builds the lists: beside their own work it costs less than an evaluation (0.8 of one; 1.4 with the
+    # grid that the search takes beside the pair list)
+    (both, _), group, pos = _contexts(8000, 0.6)
+    alone = _time(both, group, pos)
+    rebuilt = _time(both, group, pos, (0.0, 0.2))
+    assert rebuilt - alone <= 1.1 * alone, (alone, rebuilt)
