@@ -234,10 +234,12 @@ __global__ void kSiteNeighbors(AtmBuffers A, AtmConfig C) {
 
 // The sites binned into the cell grid (rebuild only), in one block: each site's cell from its wrapped position, the
 // cell counts in shared memory, their scan, the scatter, and each cell's sites put in increasing order (so that the
-// lists built from the cells come out the same on every run).  With `sharedSites` (at most kSiteSortSharedMax sites,
-// the launch giving 4 bytes of dynamic shared memory per site) the scatter goes to shared memory and a warp per cell
-// writes each site at its rank among the cell's sites; else each cell is insertion-sorted in place in global memory.
-__global__ void __launch_bounds__(1024) kSiteCellSort(AtmBuffers A, AtmConfig C, int sharedSites) {
+// lists built from the cells come out the same on every run).  SHARED (at most kSiteSortSharedMax sites, the launch
+// giving 4 bytes of dynamic shared memory per site): the scatter goes to shared memory and a warp per cell writes each
+// site at its rank among the cell's sites; else each cell is insertion-sorted in place in global memory, which is why that
+// form leaves the SM its cache (100,000 sites: 225 us, and 335 with all of the memory set aside for shared memory).
+template <bool SHARED>
+__global__ void __launch_bounds__(1024) kSiteCellSort(AtmBuffers A, AtmConfig C) {
     dependentStart(C.numSites <= kEarlySites);
     if (*(volatile int*)A.flag == 0) return;
     __shared__ int count[kSiteCellMax];
@@ -283,10 +285,10 @@ __global__ void __launch_bounds__(1024) kSiteCellSort(AtmBuffers A, AtmConfig C,
     }
     if (t == T - 1) G.cellStart[numCells] = run;
     __syncthreads();
-    int* dst = sharedSites ? scattered : G.cellSites;
+    int* dst = SHARED ? scattered : G.cellSites;
     for (int s = t; s < C.numSites; s += T) dst[atomicAdd(&count[G.siteCell[s]], 1)] = s;
     __syncthreads();
-    if (sharedSites) {
+    if (SHARED) {
         // the sites are distinct, so each one's rank among its cell's sites is its place
         const int warp = t >> 5, lane = t & 31;
         for (int c = warp; c < numCells; c += T >> 5) {

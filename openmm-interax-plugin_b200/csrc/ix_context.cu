@@ -1019,7 +1019,7 @@ static int allocateAtm(ix_ctx* ctx) {
         IX_TRY(deviceAlloc(ctx, "siteWrapped", ns, &A.cells.wrapped));
         IX_TRY(deviceAlloc(ctx, "siteOrder", ns, &A.cells.order));
         // the one-block cell sort scatters up to kSiteSortSharedMax sites in dynamic shared memory (on this device)
-        IX_CUDA(ctx, cudaFuncSetAttribute(kSiteCellSort, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        IX_CUDA(ctx, cudaFuncSetAttribute(kSiteCellSort<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           kSiteSortSharedMax * (int)sizeof(int)));
     }
     {
@@ -1467,8 +1467,9 @@ static int launchEvaluation(ix_ctx* ctx, unsigned terms, double* outForces, doub
         // site list rebuild when the centroid kernel set the flag: these kernels return at once otherwise.  The
         // long-list flag is recomputed with the lists
         if (A.cells.nc[0]) {
-            const int sharedSites = C.numSites <= kSiteSortSharedMax;
-            launchNext(early, sa, kSiteCellSort, 1, 1024, sharedSites ? C.numSites * sizeof(int) : 0, A, C, sharedSites);
+            if (C.numSites <= kSiteSortSharedMax)
+                launchNext(early, sa, kSiteCellSort<true>, 1, 1024, C.numSites * sizeof(int), A, C);
+            else launchNext(early, sa, kSiteCellSort<false>, 1, 1024, 0, A, C);
             // two blocks per SM beside the pair list, whose build takes longer anyway; alone, as many as the sites fill (eight):
             // with two the three-body term of 24,000 atoms took 129 us with a rebuild for 100, of 96,000 643 for 425
             launchNext(early, sa, kSiteNeighborsCells,
@@ -1746,7 +1747,7 @@ static void sharedSplit() {
     most(kSiteCentroids);
     most(kSiteNeighbors);
     most(kSiteNeighborsCells);
-    most(kSiteCellSort);
+    most(kSiteCellSort<true>);
     most(kRefreshPositions);
     most(kCellKeys);
     most(kScatterCells);

@@ -65,3 +65,12 @@ def test_a_rebuild_of_the_lists():
     alone = _time(both, group, pos)
     rebuilt = _time(both, group, pos, (0.0, 0.2))
     assert rebuilt - alone <= 1.1 * alone, (alone, rebuilt)
+
+
+def test_a_rebuild_of_many_sites():
+    # more sites than the sort of the cell grid holds in shared memory: it works in global memory and needs its cache
+    # (a rebuild took 2.9 evaluations of 100,000 sites without the cache, and 2.4 with it)
+    (both, _), group, pos = _contexts(100000, 0.6)
+    alone = _time(both, group, pos)
+    rebuilt = _time(both, group, pos, (0.0, 0.2))
+    assert rebuilt - alone <= 2.7 * alone, (alone, rebuilt)
