@@ -43,11 +43,11 @@ F_PAIR = 612.4
 F_TRIPLE = 151.0
 # DRAM bytes (read + write) of one pair-kernel launch on this workload, from one ncu capture of an MD-step launch
 # (dram__bytes.sum.per_second x gpu__time_duration.sum); the kernel is FP32-issue bound, the traffic is reported beside it
-PAIR_TRAFFIC_BYTES = 10162432
+PAIR_TRAFFIC_BYTES = 10164500
 # The same capture's hardware view: FMA-pipe busy fraction (sm__pipe_fma_cycles_active, pct of peak over active
 # cycles) and issue-slot use (sm__inst_issued), beside the algorithmic fraction
-PAIR_FMA_PIPE_ACTIVE = 0.355
-PAIR_ISSUE_ACTIVE = 0.747
+PAIR_FMA_PIPE_ACTIVE = 0.339
+PAIR_ISSUE_ACTIVE = 0.743
 METRIC = "interactions/s"
 WORKLOAD = "water box 24,000 atoms (8,000 rigid 3-site waters, constrained, 6.208 nm periodic, cutoff 1.0 nm) + ATM " \
            "on 8,000 molecular sites (cutoff 0.6 nm); velocity-Verlet 1 fs with SHAKE/RATTLE"
@@ -61,8 +61,8 @@ def parse():
     p.add_argument("--impl", default="ours", choices=["ours", "reference"])
     p.add_argument("--config", default="24k")
     p.add_argument("--seed", type=int, default=1)
-    # graph: each step replays one CUDA graph (conditional nodes skip the list rebuild); direct: kernel by kernel,
-    # the same kernels and results (profilers cannot see into graphs with conditional nodes)
+    # graph: each step replays a CUDA graph; direct: kernel by kernel, the same kernels and results (for profilers that
+    # count launches)
     p.add_argument("--launch", default="graph", choices=["graph", "direct"])
     # served stream: Poisson arrival rate (requests/s) of its latency phase and the server's running-request limit
     p.add_argument("--rate", type=float, default=100.0)

@@ -499,8 +499,9 @@ __device__ __forceinline__ void storeNeighbor(TripleStorage<DAMP, N>& S, const A
 // What bounds it: FP32 issue, about 75 instructions a visit, and for a few thousand sites the latency of the staging
 // (list, position, parameters, three dependent loads).  The earlier form gave each lane a pair (B, C) of a flat
 // triangular index, stored both forces in shared memory and gathered them per neighbor, 425 issue slots per 32 pairs.
-// Kernel times on one B200, both triple kernels, before and now: 96,000-atom box, 0.8 nm, 13.6 M triples: 421 and
-// 159 us; 24,000 atoms, 0.6 nm, 0.46 M triples: 24 and 19 us; 648 atoms: 15.7 and 10.9 us.
+// Kernel times on one B200, both triple kernels with a warp per site, before and now: 96,000-atom box, 0.8 nm, 13.6 M
+// triples: 410 and 166 us; 24,000 atoms, 0.6 nm, 0.46 M triples: 27 and 25 us.  Beside the pair kernel, on two blocks an
+// SM, the 24,000-atom launch takes 41 us of the pair kernel's 110 and is hidden behind it.
 template <bool DAMP, bool IMAGE, bool ALCH, int N>
 __device__ __forceinline__ void siteTriples(const TripleStorage<DAMP, N>& S, const AtmBuffers& A, const AtmConfig& C,
                                             const float4& pa, int cFirst, int cStep, int cEnd, int bBegin, int bEnd,

@@ -9,8 +9,9 @@
 // without periodic boundaries), each as much as can be done before the next grid-wide dependency, with the scans in
 // the last block of the kernel that feeds them.  As a chain of fifteen kernels in the body of a conditional graph node
 // a step without a rebuild paid 9.5 us for the node (28 us where its other branch held the position refresh), and a
-// step with one waited 49 us for the body's first kernel and 115 us for the build (24,000 atoms); five launches that
-// return at once take 10 us beside the triple kernels, and the build takes 71 us.
+// step with one waited 49 us for the body's first kernel and 115 us for the build (24,000 atoms); the five launches take
+// 10 us when they return at once (4.4 us for 648 atoms, whose kernels let their successors in early) and 71 us when they
+// build.
 //
 // The reference gets its list from OpenMM (NonbondedUtilities, called at platforms/common/src/
 // CommonInteraxKernels.cpp:209) and, on the Reference platform, a voxel hash (ReferenceInteraxPairIxn.h:86-87).
