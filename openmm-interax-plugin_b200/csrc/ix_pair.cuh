@@ -491,8 +491,8 @@ __global__ void __launch_bounds__(32 * kPairWarps, IX_TUNE_PAIR_MIN_BLOCKS) kPai
         task = __shfl_sync(0xffffffffu, task, 0);
         if (task >= numTasks) break;
         // the task's tile, of the first bucket that ends behind it.  The buckets' ends are read for each task: kept in a
-        // register all along they cost 1.8 us of 105 for 24,000 atoms, and 11 of 115 in the general form (12,000 atoms of 64
-        // types with soft core, switch and order-2 overlap).
+        // register all along they cost 1.8 us of 105 for 24,000 atoms, and up to 12 of 116 in the general form (12,000 atoms of
+        // 64 types with soft core, switch and order-2 overlap, whose last wave of tiles varies with the list).
         const int bucket = __ffs(__ballot_sync(0xffffffffu, task < __ldg(L.bucketEnd + lane))) - 1;
         const int t = L.bucketTiles[__ldg(L.bucketOffset + bucket) + (unsigned)task];
         const int I = L.tileIBlock[t];
