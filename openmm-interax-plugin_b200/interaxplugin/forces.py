@@ -349,9 +349,11 @@ class System:
         return self._masses[index]
 
     def _masses_array(self):
-        if self._mass_array is None:
-            self._mass_array = np.array(self._masses, dtype=np.float64)
-        return self._mass_array
+        # (a System kept by an earlier build has no array, and one whose list a copy shares can have grown)
+        kept = self.__dict__.get("_mass_array")
+        if kept is None or len(kept) != len(self._masses):
+            self._mass_array = kept = np.array(self._masses, dtype=np.float64)
+        return kept
 
     def addForce(self, force):
         self._forces.append(force)
