@@ -443,6 +443,18 @@ static BoxF makeBoxF(const Box& b) {
     return f;
 }
 
+// A new box: captured launches hold the old one, and the lists the images and neighbors of the box they were built with,
+// however little the particles have moved.
+static int setBox(ix_ctx* ctx, const double* box) {
+    if (std::memcmp(ctx->box, box, sizeof(ctx->box)) == 0) return IX_OK;
+    std::memcpy(ctx->box, box, sizeof(ctx->box));
+    bumpVersion(ctx);
+    static const int rebuild = 1;
+    IX_CUDA(ctx, cudaSetDevice(ctx->device));
+    for (int list : {0, 4}) IX_TRY(stageCopy(ctx, ctx->dFlags + list, &rebuild, sizeof(rebuild)));
+    return IX_OK;
+}
+
 static double lambdaOf(const ix_ctx* ctx, const std::string& name, bool anyAlch) {
     if (!anyAlch) return 1.0;
     auto it = ctx->parameters.find(name);
@@ -2091,8 +2103,7 @@ int ix_set_positions(ix_ctx* ctx, const double* positions, const double* box) {
     if (box) {
         if (box[0] <= 0 || box[4] <= 0 || box[8] <= 0)
             return fail(ctx, IX_ERR_INVALID, "Illegal periodic box vectors");
-        if (std::memcmp(ctx->box, box, sizeof(ctx->box)) != 0) bumpVersion(ctx);
-        std::memcpy(ctx->box, box, sizeof(ctx->box));
+        IX_TRY(setBox(ctx, box));
     }
     IX_CUDA(ctx, cudaSetDevice(ctx->device));
     IX_TRY(stageCopy(ctx, ctx->dPos, positions, 3 * (size_t)ctx->n * sizeof(double)));
@@ -2308,8 +2319,7 @@ int ix_compute_device_posq(ix_ctx* ctx, int groups, int posq_format, const void*
     IX_TRY(deviceStatusCheck(ctx));
     if (box) {
         if (box[0] <= 0 || box[4] <= 0 || box[8] <= 0) return fail(ctx, IX_ERR_INVALID, "Illegal periodic box vectors");
-        if (std::memcmp(ctx->box, box, sizeof(ctx->box)) != 0) bumpVersion(ctx);
-        std::memcpy(ctx->box, box, sizeof(ctx->box));
+        IX_TRY(setBox(ctx, box));
     }
     ctx->havePositions = true;
     unsigned terms = selectedTerms(ctx, groups);
@@ -2386,8 +2396,7 @@ int ix_compute_device_f64(ix_ctx* ctx, int groups, const double* d_positions, co
     IX_TRY(deviceStatusCheck(ctx));
     if (box) {
         if (box[0] <= 0 || box[4] <= 0 || box[8] <= 0) return fail(ctx, IX_ERR_INVALID, "Illegal periodic box vectors");
-        if (std::memcmp(ctx->box, box, sizeof(ctx->box)) != 0) bumpVersion(ctx);
-        std::memcpy(ctx->box, box, sizeof(ctx->box));
+        IX_TRY(setBox(ctx, box));
     }
     if (d_positions) {
         IX_CUDA(ctx, cudaMemcpyAsync(ctx->dPos, d_positions, 3 * (size_t)ctx->n * sizeof(double),
